@@ -93,7 +93,7 @@ int rebuild(exo_ensemble* e) {
   std::vector<DevView> views;
   std::vector<unsigned> start((size_t)exo::BK_COUNT * (e->capacity + 1), 0);
   unsigned tot[exo::BK_COUNT] = {0, 0, 0, 0, 0, 0};
-  bool any_full = false;  // some member takes the 5x5 correction
+  int implicit_kinds = 0;  // the block sizes of the members' implicit solves
   int max_nc1 = 1;
   // the x1 blocks' threads: the ensemble's columns per block at the deepest
   // member; every member then takes as many columns as fill those threads
@@ -123,8 +123,8 @@ int rebuild(exo_ensemble* e) {
       x1_smem = std::max(x1_smem, exo::x1_smem_bytes(mv));
     }
     max_nc1 = std::max(max_nc1, m->v.nc1);
-    if (m->v.eqn != EXO_EQN_SHALLOW_YZ && (m->v.implicit_flag & 1) && (m->v.implicit_flag & 8))
-      any_full = true;
+    if (m->v.eqn != EXO_EQN_SHALLOW_YZ && (m->v.implicit_flag & 1))
+      implicit_kinds |= exo::implicit_kind(m->v);
     unsigned b[exo::BK_COUNT];
     exo::member_blocks(m->v, mv.tiles, b);
     for (int k = 0; k < exo::BK_COUNT; ++k) {
@@ -154,10 +154,10 @@ int rebuild(exo_ensemble* e) {
   for (int k = 0; k < exo::BK_COUNT; ++k) pl.threads[k] = e->tiles.t[k];
   pl.max_nc1 = max_nc1;
   pl.precision = e->precision;
-  pl.any_full_correction = any_full;
+  pl.implicit_kinds = implicit_kinds;
   // count the kernel nodes of one step
   int64_t per_stage = (tot[exo::BK_X1] ? 1 : 0) + 1 + 1 +
-                      (tot[exo::BK_IMPLICIT] ? (any_full && exo::split_bwd(e->precision) ? 2 : 1) : 0) + 1;
+                      exo::implicit_launches(implicit_kinds, e->precision) + 1;
   e->launches_per_step = 3 * per_stage + (tot[exo::BK_ROUNDTRIP] ? 1 : 0) + 1 + 1;
   cudaGraph_t graph;
   ECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));

@@ -1,0 +1,623 @@
+// exo_implicit_fused.cuh -- the mixed build's 5x5 solve in FP64 blocks with its
+// back substitution in the same kernel (textually part of exo_kernels.cuh).
+//
+// The same algorithm as implicit_column and kb_implicit_bwd, in the form it
+// had before those two were split and their loads moved to warp tiles.  The
+// split form is faster (6x96^2x64: 764 against 867 us a solve alone; with the
+// blocks kept by their structure 617), but compiled with fused
+// multiply-adds it does not round as this one does: the last bits of u it
+// changes reach the FP32 copy of the primitives, and a run differs by 1e-7
+// within some tens of steps.  FP32 blocks, the 3x3 blocks and the FP64 build,
+// whose results the split form leaves to the bit, take the split form.
+
+// Solve with the LU factors of implicit_column's mixed build (rows taken in
+// the order 1, 4, 2, 3, 0, threshold row swaps packed 3 bits per step): y
+// holds the right-hand side with its rows in natural order on entry and the
+// solution, unknowns in order, on exit.
+template <class R>
+__device__ __forceinline__ void lu_solve_swapped(const R (&t)[5][5], const R (&idg)[5],
+                                              unsigned perm, bool swapped, R* y) {
+  constexpr int O[5] = {1, 4, 2, 3, 0};
+  if (swapped) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned pk = (perm >> (3 * k)) & 7u;
+#pragma unroll
+      for (int r = k + 1; r < 5; ++r) {
+        const bool sw = (pk == (unsigned)r);
+        const R a = y[O[k]], b = y[O[r]];
+        y[O[k]] = sw ? b : a;
+        y[O[r]] = sw ? a : b;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 1; r < 5; ++r)
+#pragma unroll
+    for (int k = 0; k < r; ++k) y[O[r]] -= t[O[r]][k] * y[O[k]];
+  R z[5];
+#pragma unroll
+  for (int r = 4; r >= 0; --r) {
+    R acc = y[O[r]];
+#pragma unroll
+    for (int q = r + 1; q < 5; ++q) acc -= t[O[r]][q] * z[q];
+    z[r] = acc * idg[r];
+  }
+#pragma unroll
+  for (int r = 0; r < 5; ++r) y[r] = z[r];
+}
+
+// The back substitution of the stepping kernel's FP64 blocks (mixed build)
+// with the state u moved through shared memory by the warp: the warp's 32
+// columns go down BWD_TL levels at a time; each lane copies four levels of
+// a column for one variable in one 32-byte run (the per-lane accesses of
+// one level are 816 bytes apart, a sector each), the next chunk's copies in
+// flight while a chunk is corrected.  The factors are read per lane, one
+// level ahead, as in implicit_backward_full (they are contiguous across the
+// warp).  io.live: the lanes of the warp with a column.  wtile: 2 x 5 x 32 x
+// (BWD_TL + 1) doubles of shared memory for the warp alone.
+constexpr int BWD_TL = 4;
+// the two u tiles of a warp's back substitution (5 variables x 32 columns x
+// BWD_TL levels, padded)
+constexpr int WARP_TILE_DOUBLES = 2 * 5 * 32 * (BWD_TL + 1);
+// shared doubles per thread: two face matrices, w and du of the next level
+constexpr int IMPL_SM_STRIDE = 61;
+static_assert(32 * IMPL_SM_STRIDE >= WARP_TILE_DOUBLES,
+              "the tiled back substitution's buffers fit in the warp's slices");
+// NB = 5: the full correction (30 factors per level, delta on every
+// variable); NB = 3: the partial one (12 factors per level, delta on rho,
+// m1 and E, the explicit du on m2 and m3, read per lane one level ahead).
+template <int NB, class IO>
+__device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
+                                                        typename IO::Real* dp, double* wtile) {
+  static_assert(BWD_TL == 4, "the lane -> (column, level) split below assumes 4 levels");
+  static_assert(NB == 5 || NB == 3, "5x5 or 3x3 blocks");
+  constexpr int NF = NB * NB + NB;  // factors per level: (A c)_i and delta_i
+  constexpr int TS = BWD_TL + 1;
+  constexpr int TW = 5 * 32 * TS;
+  const unsigned live = io.live;
+  const int lane = (int)(threadIdx.x & 31);
+  __syncwarp(live);
+  // lane copies level (lane & 3) of columns (lane >> 2) + 8 m, m = 0..3
+  // (in a warp with a column in every lane)
+  double* ub[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+    ub[m] = reinterpret_cast<double*>(__shfl_sync(
+        live, reinterpret_cast<unsigned long long>(io.uc), ((lane >> 2) + 8 * m) & 31));
+  const int l = lane & 3;
+  const int nch = (ie - is + BWD_TL) / BWD_TL;
+  auto range = [&](int c, int& lo, int& hi) {
+    hi = ie - c * BWD_TL;
+    lo = max(is, hi - BWD_TL + 1);
+  };
+  // a warp with a column in every lane copies in 32-byte runs; the last warp
+  // of a member may have fewer, and there each lane copies its own column
+  const bool full = live == 0xffffffffu;
+  auto load = [&](int c) {
+    double* t = wtile + (c & 1) * TW;
+    int lo, hi;
+    range(c, lo, hi);
+    if (full) {
+      if (lo + l <= hi) {
+#pragma unroll
+        for (int e = 0; e < 20; ++e) {
+          const int m = e & 3, n = e >> 2;
+          cp_async8(&t[(n * 32 + (lane >> 2) + 8 * m) * TS + l], ub[m] + n * io.vs + lo + l);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 20; ++e) {
+        const int ll = e & 3, n = e >> 2;
+        if (lo + ll <= hi) cp_async8(&t[(n * 32 + lane) * TS + ll], io.uc + n * io.vs + lo + ll);
+      }
+    }
+    cp_async_commit();
+  };
+  load(0);
+  if (nch > 1) load(1);
+  using R = typename IO::Real;
+  // the factors of the next level (cur_s) and, with 1 2, of the
+  // one after (ahd_s): their loads are in flight for two levels (the
+  // registers of the finished forward sweep are free)
+  R cur_s[NF], ahd_s[NF];
+  if (ie > is) {
+#pragma unroll
+    for (int e = 0; e < NF; ++e) cur_s[e] = io.scr(ie - 1 - is, e);
+  }
+  if constexpr (false) {
+    if (ie - 1 > is) {
+#pragma unroll
+      for (int e = 0; e < NF; ++e) ahd_s[e] = io.scr(ie - 2 - is, e);
+    }
+  }
+  // the partial correction's explicit du of m2 and m3, one level ahead
+  double cur_du[2] = {0., 0.};
+  if constexpr (NB == 3) {
+    cur_du[0] = *io.duptr(ie, IVY);
+    cur_du[1] = *io.duptr(ie, IVZ);
+  }
+  for (int c = 0; c < nch; ++c) {
+    if (c + 1 < nch) cp_async_wait_one();
+    else cp_async_wait_all();
+    __syncwarp(live);
+    double* t = wtile + (c & 1) * TW;
+    int lo, hi;
+    range(c, lo, hi);
+    for (int i = hi; i >= lo; --i) {
+      double nxt_du[2] = {0., 0.};
+      if constexpr (NB == 3) {
+        if (i > is) {
+          nxt_du[0] = *io.duptr(i - 1, IVY);
+          nxt_du[1] = *io.duptr(i - 1, IVZ);
+        }
+      }
+      if (i < ie) {
+        R nxt_s[NF];
+        const int ahead = i - 1;  // the level whose factors load now
+        if (ahead >= is) {
+#pragma unroll
+          for (int e = 0; e < NF; ++e) nxt_s[e] = io.scr(ahead - is, e);
+        }
+        R dl[NB];
+#pragma unroll
+        for (int r = 0; r < NB; ++r) {
+          R ad = cur_s[r * NB] * dp[0];
+#pragma unroll
+          for (int k = 1; k < NB; ++k) ad += cur_s[r * NB + k] * dp[k];
+          dl[r] = cur_s[NB * NB + r] - ad;
+        }
+#pragma unroll
+        for (int r = 0; r < NB; ++r) dp[r] = dl[r];
+        if constexpr (false) {
+#pragma unroll
+          for (int e = 0; e < NF; ++e) {
+            cur_s[e] = ahd_s[e];
+            ahd_s[e] = nxt_s[e];
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < NF; ++e) cur_s[e] = nxt_s[e];
+        }
+      }
+      // the corrected update of every variable
+      double d[5];
+      if constexpr (NB == 5) {
+#pragma unroll
+        for (int n = 0; n < 5; ++n) d[n] = dp[n];
+      } else {
+        d[IDN] = dp[0];
+        d[IVX] = dp[1];
+        d[IVY] = cur_du[0];
+        d[IVZ] = cur_du[1];
+        d[IEN] = dp[2];
+        cur_du[0] = nxt_du[0];
+        cur_du[1] = nxt_du[1];
+      }
+      double uu[5];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) uu[n] = t[(n * 32 + lane) * TS + (i - lo)] + 1. * d[n];
+      if (io.stage == 2) airparcel_round_trip(uu, io.Rd, io.gamma);
+#pragma unroll
+      for (int n = 0; n < 5; ++n) t[(n * 32 + lane) * TS + (i - lo)] = uu[n];
+    }
+    __syncwarp(live);
+    if (full) {
+      if (lo + l <= hi) {
+#pragma unroll
+        for (int e = 0; e < 20; ++e) {
+          const int m = e & 3, n = e >> 2;
+          ub[m][n * io.vs + lo + l] = t[(n * 32 + (lane >> 2) + 8 * m) * TS + l];
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 20; ++e) {
+        const int ll = e & 3, n = e >> 2;
+        if (lo + ll <= hi) io.uc[n * io.vs + lo + ll] = t[(n * 32 + lane) * TS + ll];
+      }
+    }
+    __syncwarp(live);
+    if (c + 2 < nch) load(c + 2);
+  }
+}
+
+// BackwardSubstitution of the full correction (forward_backward.hpp:90-126):
+// delta_i -= (A c)_i delta_{i+1} from level ie (delta_ie given in dp) down
+// to is, each corrected update stored through io.  kPipe: software-pipelined,
+// the next level's factors and state in flight while a level finishes (for
+// the few resident columns of the solve kernel); otherwise one level at a
+// time, leaving the latency to the many columns of the back-substitution
+// kernel.
+template <class IO, bool kPipe = true>
+__device__ __forceinline__ void implicit_backward_full(IO& io, int is, int ie,
+                                                       typename IO::Real* dp) {
+  using R = typename IO::Real;
+  auto store = [&](int i, const double* u) {
+    double d[5];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) d[n] = dp[n];
+    io.ustore(i, u, d);
+  };
+  if constexpr (!kPipe) {
+    {
+      double u[5];
+      io.uload(ie, u);
+      store(ie, u);
+    }
+#pragma unroll 1
+    for (int i = ie - 1; i >= is; --i) {
+      R cs[30];
+      double u[5];
+#pragma unroll
+      for (int e = 0; e < 30; ++e) cs[e] = io.scr(i - is, e);
+      io.uload(i, u);
+      R dl[5];
+#pragma unroll
+      for (int r = 0; r < 5; ++r) {
+        R ad = cs[r * 5] * dp[0];
+#pragma unroll
+        for (int k = 1; k < 5; ++k) ad += cs[r * 5 + k] * dp[k];
+        dl[r] = cs[25 + r] - ad;
+      }
+#pragma unroll
+      for (int r = 0; r < 5; ++r) dp[r] = dl[r];
+      store(i, u);
+    }
+    return;
+  }
+  R cur_s[30];
+  double cur_u[5];
+  io.uload(ie, cur_u);
+  store(ie, cur_u);
+  if (ie > is) {
+#pragma unroll
+    for (int e = 0; e < 30; ++e) cur_s[e] = io.scr(ie - 1 - is, e);
+    io.uload(ie - 1, cur_u);
+  }
+#pragma unroll 1
+  for (int i = ie - 1; i >= is; --i) {
+    R nxt_s[30];
+    double nxt_u[5];
+    if (i > is) {
+#pragma unroll
+      for (int e = 0; e < 30; ++e) nxt_s[e] = io.scr(i - 1 - is, e);
+      io.uload(i - 1, nxt_u);
+    }
+    R dl[5];
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+      R ad = cur_s[r * 5] * dp[0];
+#pragma unroll
+      for (int k = 1; k < 5; ++k) ad += cur_s[r * 5 + k] * dp[k];
+      dl[r] = cur_s[25 + r] - ad;
+    }
+#pragma unroll
+    for (int r = 0; r < 5; ++r) dp[r] = dl[r];
+    store(i, cur_u);
+    if (i > is) {
+#pragma unroll
+      for (int e = 0; e < 30; ++e) cur_s[e] = nxt_s[e];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) cur_u[n] = nxt_u[n];
+    }
+  }
+}
+
+template <class IO>
+__device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real* sa, double* sp, int ss,
+                                                double cos_theta, double sin_theta, double d2,
+                                                double d3, const double* x1f, const double* x1v,
+                                                const double* dx1f, int is, int ie, double dt,
+                                                double gamma, double grav,
+                                                double* wt = nullptr) {
+  using R = typename IO::Real;
+  using ColCell = exo::EXO_KNS::ColCell<R>;
+  const double s = sin_theta;
+  // gmm1 of every cell; the face average equals it
+  const R gm1 = R((gamma - 1.) * 1. / 1.);
+  const R gp = (gm1 + R(1)) / gm1;
+  const R gam = R(gamma);
+  const R grv = R(grav);
+  // the reference's Dt = 1/dt, the same value every time
+  const R rdt = R(1. / dt);
+  auto cell = [&](const double* w) {
+    ColCell c;
+    c.rho = R(w[IDN]);
+    c.v1 = R(w[IVX]);
+    c.v2 = R(w[IVY] + w[IVZ] * cos_theta);
+    c.v3 = R(w[IVZ] * sin_theta);
+    c.p = R(w[IPR]);
+    c.s2 = c.v1 * c.v1 + c.v2 * c.v2 + c.v3 * c.v3;
+    if constexpr (sizeof(R) == 4) {
+      c.isq = rsqrt_r(c.rho);
+      c.sq = c.rho * c.isq;
+      c.hr = gp * c.p * (c.isq * c.isq);
+    } else {
+      c.hr = gp * c.p * inv_r(c.rho);
+    }
+    return c;
+  };
+  auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 25 + r * 5 + q) * ss]; };
+
+  // prefetch slots: w(i+1) and du(i) of the next level, copied asynchronously
+  auto pw = [&](int n) -> double& { return sp[n * ss]; };
+  auto pdu = [&](int n) -> double& { return sp[(5 + n) * ss]; };
+  auto prefetch = [&](int iw, int idu) {
+#pragma unroll
+    for (int n = 0; n < 5; ++n) cp_async8(&pw(n), io.wptr(iw, n));
+    if (idu >= 0) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) cp_async8(&pdu(n), io.duptr(idu, n));
+    }
+    cp_async_commit();
+  };
+  double raw[5];
+  io.w(is - 1, raw);
+  ColCell cm = cell(raw);
+  io.w(is, raw);
+  ColCell c0 = cell(raw);
+  prefetch(is + 1, is);
+  {
+    R A[5][5];
+    abs_jacobian(cm, c0, gm1, gam, A);
+#pragma unroll
+    for (int r = 0; r < 5; ++r)
+#pragma unroll
+      for (int q = 0; q < 5; ++q) AMs(0, r, q) = A[r][q];
+  }
+  R Ap[5][5];
+  R dp[5];  // delta_{i-1}
+  int cur = 0;
+  for (int i = is; i <= ie; ++i) {
+    cp_async_wait_all();
+    double rhs[5];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {
+      raw[n] = pw(n);
+      rhs[n] = pdu(n);
+    }
+    ColCell cp = cell(raw);
+    prefetch(i + 2, i < ie ? i + 1 : -1);
+    const int nxt = cur ^ 1;
+    {
+      R A[5][5];
+      abs_jacobian(c0, cp, gm1, gam, A);
+#pragma unroll
+      for (int r = 0; r < 5; ++r)
+#pragma unroll
+        for (int q = 0; q < 5; ++q) AMs(nxt, r, q) = A[r][q];
+    }
+    const double aleft = d2 * d3 * x1f[i] * x1f[i] * s;
+    const double aright = d2 * d3 * x1f[i + 1] * x1f[i + 1] * s;
+    const double vol = dx1f[i] * d2 * d3 * x1v[i] * x1v[i] * s;
+    const double i2v = 0.5 / vol;
+    const R bl = R(aleft * i2v), cr = R(aright * i2v), dd = R((aright - aleft) * i2v);
+    const bool first = (i == is), last = (i == ie);
+    R x[5];
+    // rows of a, b (and c at the top boundary), then of t = a - b (A c)_{i-1},
+    // written over row r of |A|(i-1/2) once that row has been read; and x
+    unroll<5>([&](auto Row) {
+      constexpr int r = decltype(Row)::value;
+      R brow[5], trow[5];
+      unroll<5>([&](auto Q) {
+        constexpr int q = decltype(Q)::value;
+        const R am = AMs(cur, r, q), ap = AMs(nxt, r, q);
+        R a = am * bl + ap * cr;
+        if constexpr (fj_nz(r, q)) a += dd * fj_entry<r, q>(c0, gm1);
+        if constexpr (r == q) a += rdt;
+        if constexpr ((r == IVX && q == IDN) || (r == IEN && q == IVX)) a -= grv;
+        R bm = am;
+        if constexpr (fj_nz(r, q)) bm += fj_entry<r, q>(cm, gm1);
+        R b = -bm * bl;
+        if (first) a += (q == IVX) ? -b : b;
+        if (last) {
+          R cmv = ap;
+          if constexpr (fj_nz(r, q)) cmv -= fj_entry<r, q>(cp, gm1);
+          R c = -cmv * cr;
+          a += (q == IVX) ? -c : c;
+        }
+        brow[q] = b;
+        trow[q] = a;
+      });
+      x[r] = R(rhs[r]) * rdt;
+      if (!first) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+          R ba = brow[0] * Ap[0][q];
+#pragma unroll
+          for (int k = 1; k < 5; ++k) ba += brow[k] * Ap[k][q];
+          trow[q] = trow[q] - ba;
+        }
+        R bd = brow[0] * dp[0];
+#pragma unroll
+        for (int k = 1; k < 5; ++k) bd += brow[k] * dp[k];
+        x[r] = x[r] - bd;
+      }
+#pragma unroll
+      for (int q = 0; q < 5; ++q) AMs(cur, r, q) = trow[q];
+    });
+    R t[5][5];
+#pragma unroll
+    for (int r = 0; r < 5; ++r)
+#pragma unroll
+      for (int q = 0; q < 5; ++q) t[r][q] = AMs(cur, r, q);
+    // c_i column by column, from |A|(i+1/2) in shared memory and the upper cell
+    auto ccol = [&](auto Q, R* c) {
+      constexpr int q = decltype(Q)::value;
+      unroll<5>([&](auto Row) {
+        constexpr int r = decltype(Row)::value;
+        R cmv = AMs(nxt, r, q);
+        if constexpr (fj_nz(r, q)) cmv -= fj_entry<r, q>(cp, gm1);
+        c[r] = -cmv * cr;
+      });
+    };
+    // LU with the rows taken in the order 1, 4, 2, 3, 0 -- the order partial
+    // pivoting ends with for nearly every block of this solve (density last,
+    // energy and x1 momentum first) -- and threshold partial pivoting on top:
+    // a row swap only where the diagonal falls below a tenth of the largest
+    // entry of its column, so the swap code is skipped almost always.
+    constexpr int O[5] = {1, 4, 2, 3, 0};
+    unsigned perm = 0;  // 3 bits per step: the position swapped in
+    bool swapped = false;
+    R idg[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      if (k < 4) {
+        const R dk = abs_r(t[O[k]][k]);
+        R best = dk;
+        int piv = k;
+#pragma unroll
+        for (int r = k + 1; r < 5; ++r) {
+          const R m = abs_r(t[O[r]][k]);
+          if (m > best) { best = m; piv = r; }
+        }
+        if (dk < R(0.1) * best) {
+          swapped = true;
+          perm |= (unsigned)piv << (3 * k);
+#pragma unroll
+          for (int r = k + 1; r < 5; ++r) {
+            const bool sw = (piv == r);
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+              const R a = t[O[k]][q], b = t[O[r]][q];
+              t[O[k]][q] = sw ? b : a;
+              t[O[r]][q] = sw ? a : b;
+            }
+          }
+        } else {
+          perm |= (unsigned)k << (3 * k);
+        }
+      }
+      idg[k] = inv_r(t[O[k]][k]);
+#pragma unroll
+      for (int r = k + 1; r < 5; ++r) {
+        const R l = t[O[r]][k] * idg[k];
+        t[O[r]][k] = l;
+#pragma unroll
+        for (int q = k + 1; q < 5; ++q) t[O[r]][q] -= l * t[O[k]][q];
+      }
+    }
+    auto solve = [&](R* y) { lu_solve_swapped(t, idg, perm, swapped, y); };
+    solve(x);
+    unroll<5>([&](auto Q) {
+      constexpr int q = decltype(Q)::value;
+      R c[5];
+      ccol(Q, c);
+      solve(c);
+#pragma unroll
+      for (int r = 0; r < 5; ++r) Ap[r][q] = c[r];
+    });
+#pragma unroll
+    for (int r = 0; r < 5; ++r) dp[r] = x[r];
+    const int lev = i - is;
+    if (!last) {
+#pragma unroll
+      for (int r = 0; r < 5; ++r)
+#pragma unroll
+        for (int q = 0; q < 5; ++q) io.scr(lev, r * 5 + q) = Ap[r][q];
+#pragma unroll
+      for (int r = 0; r < 5; ++r) io.scr(lev, 25 + r) = dp[r];
+    }
+    cm = c0;
+    c0 = cp;
+    cur = nxt;
+  }
+  // the last level's prefetch (unused) must land before the back substitution
+  // reuses this thread's slots of shared memory
+  cp_async_wait_all();
+  if constexpr (IO::kLoadsU && sizeof(R) == 8) {
+    if (io.stage >= 0) {
+      // the warp's tiles (FP64 blocks: its 32 shared slices, free once every
+      // lane has finished its forward sweep)
+      implicit_backward_tiled<5>(io, is, ie, dp, wt);
+      return;
+    }
+  }
+  implicit_backward_full(io, is, ie, dp);
+}
+
+// this thread's slices of the block's shared memory: each thread's doubles
+// contiguous, IMPL_SM_STRIDE doubles apart (odd, so that a half-warp's 8-byte
+// accesses fall on distinct banks), then the radial tables
+constexpr size_t fused_smem(int threads, int nc1) {
+  return ((size_t)IMPL_SM_STRIDE * threads + 3 * (size_t)(nc1 + 1)) * sizeof(double);
+}
+
+// A column of the stepping context: primitives and update from the state
+// arrays, the corrected update added to u (with the AirParcel round trip on
+// the last stage).
+template <class R>
+struct FusedColumnIO {
+  using Real = R;
+  const double* wc;
+  const double* duc;
+  double* uc;
+  size_t vs;       // stride between variables
+  R* scr0;         // scratch of this column: [level][entry][32 lanes] per warp of columns
+  int stage;            // < 0: write the corrected update into du, leave u alone
+  double Rd, gamma;
+  double* duw;          // du of this column, for stage < 0
+  __device__ __forceinline__ void w(int i, double* out) const {
+#pragma unroll
+    for (int n = 0; n < 5; ++n) out[n] = wc[n * vs + i];
+  }
+  __device__ __forceinline__ const double* wptr(int i, int n) const { return wc + n * vs + i; }
+  __device__ __forceinline__ const double* duptr(int i, int n) const { return duc + n * vs + i; }
+  __device__ __forceinline__ R& scr(int lev, int e) const {
+    return scr0[(lev * 30 + e) * 32];
+  }
+  static constexpr bool kLoadsU = true;
+  unsigned live = 0xffffffffu;  // the lanes of the warp with a column
+  __device__ __forceinline__ void uload(int i, double* u) const {
+    if (stage < 0) return;
+#pragma unroll
+    for (int n = 0; n < 5; ++n) u[n] = uc[n * vs + i];
+  }
+  __device__ __forceinline__ void ustore(int i, const double* u, const double* dl) const {
+    if (stage < 0) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) duw[n * vs + i] = dl[n];
+      return;
+    }
+    double uu[5];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) uu[n] = u[n] + 1. * dl[n];
+    if (stage == 2) airparcel_round_trip(uu, Rd, gamma);
+#pragma unroll
+    for (int n = 0; n < 5; ++n) uc[n * vs + i] = uu[n];
+  }
+};
+
+
+template <class R>
+__device__ __forceinline__ void implicit_fused_block(const DevView& v, unsigned blk, int stage,
+                                               double dt_given = 0.) {
+  extern __shared__ double ism[];
+  const int ncol = 6 * v.N * v.N;
+  const int col = (int)(blk * blockDim.x + threadIdx.x);
+  // the radial geometry, read every level by every column, staged once per
+  // block: kept out of L1, which the columns' strided loads churn each level
+  const double* x1f;
+  const double* x1v;
+  const double* dx1f;
+  stage_radial(ism + blockDim.x * IMPL_SM_STRIDE, v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
+  const unsigned live = __ballot_sync(0xffffffffu, col < ncol);
+  if (col >= ncol) return;
+  const int j = v.js + col % v.N;
+  const int k = v.ks + (col / v.N) % v.N;
+  const int p = col / (v.N * v.N);
+  const double dt = stage < 0 ? dt_given : rk_beta(stage) * v.sc->dt;
+  const size_t base = idx(v, p, 0, k, j, 0);
+  // scratch in blocks of 32 columns: a warp's 32 entries are 128 (FP32) or
+  // 256 (FP64) contiguous bytes
+  R* scr0 = reinterpret_cast<R*>(v.scratch) + (size_t)(col >> 5) * v.L * 30 * 32 + (col & 31);
+  FusedColumnIO<R> io{v.w + base, v.du + base, v.u + base, v.cells, scr0, stage, v.Rd, v.gamma,
+                     v.du + base};
+  io.live = live;
+  double* const sm = ism + threadIdx.x * IMPL_SM_STRIDE;
+  implicit_column_fused(io, sm, sm + 50, 1, geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j),
+                        geo(v, GDX2A, p, k, j), geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is, v.ie,
+                        dt, v.gamma, v.grav, ism + (threadIdx.x & ~31u) * IMPL_SM_STRIDE);
+}

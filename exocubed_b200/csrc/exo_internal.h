@@ -3,6 +3,7 @@
 #ifndef EXO_INTERNAL_H_
 #define EXO_INTERNAL_H_
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <string>
@@ -122,6 +123,31 @@ struct FastDiv {
     return (unsigned)((hi + (lo >> 32)) >> 8);
   }
 };
+// a / b for many numerators of one denominator, the IEEE quotient bit for
+// bit: with r the correctly rounded 1/b, q <- q + r (a - b q), the remainder
+// exact in a fused multiply-add, gives the correctly rounded quotient once q
+// is within an ulp of a/b (Markstein, IBM J. Res. Dev. 34, 1990); the first
+// such step from q = a r brings it there, the second rounds it.  Five
+// operations a division instead of the twenty instructions of a division
+// with its range checks.  Exact where every intermediate is a normal number:
+// |b| in 2^-400..2^400 and |a| in 2^-500..2^500, or a = 0 (whose quotient is
+// +0 for either sign).  Smaller numerators may be off in the last bit, and an
+// infinite one gives NaN: no valid state's terms.
+struct SharedDiv {
+  double b, r;
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  explicit SharedDiv(double b_) : b(b_), r(1.0 / b_) {}
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  double operator()(double a) const {
+    double q = a * r;
+    q = fma(r, fma(-b, q, a), q);
+    return fma(r, fma(-b, q, a), q);
+  }
+};
 inline FastDiv make_fastdiv(unsigned d) {
   FastDiv f;
   f.m = ((1ull << 40) + d - 1) / d;
@@ -177,7 +203,7 @@ struct BatchPlan {
   int threads[BK_COUNT];         // tiles of the other kernels
   int max_nc1;                   // largest nc1 of the members (radial tables in shared memory)
   int precision;                 // EXO_PREC_* of every member
-  bool any_full_correction;      // some member takes the 5x5 solve (kb_implicit_bwd runs)
+  int implicit_kinds;            // IMPL_FULL, IMPL_PARTIAL: the solves its members take
 };
 // Threads per block ("tile") of each batched kernel by BatchKind.  BK_X1
 // takes one radial column per block (its size follows L) and ignores its
@@ -204,14 +230,16 @@ constexpr int X1_SMEM_MAX = 224 * 1024;
 EXO_HD inline bool mixed_build(int precision) {
   return precision == EXO_PREC_MIXED || precision == EXO_PREC_MIXED_F32_SOLVE;
 }
-// The implicit solve with the full (5x5) correction: FP64 blocks solve and
-// back-substitute each column in kb_implicit (a column's back substitution
-// overlaps other columns' forward sweeps); FP32 blocks run the forward sweep
-// in kb_implicit and the back substitution in kb_implicit_bwd (memory-bound,
-// fed by bulk copies).  The partial (3x3) correction does both in kb_implicit.
-EXO_HD inline bool split_bwd(int precision) { return precision == EXO_PREC_MIXED_F32_SOLVE; }
-inline int implicit_launches(int implicit_flag, int precision) {
-  return ((implicit_flag & 8) && split_bwd(precision)) ? 2 : 1;
+// the block sizes of a member's or a batch's implicit solves (one kernel each)
+enum { IMPL_FULL = 1, IMPL_PARTIAL = 2 };
+EXO_HD inline int implicit_kind(const DevView& v) {
+  return (v.implicit_flag & 8) ? IMPL_FULL : IMPL_PARTIAL;
+}
+// its launches: a forward sweep and a back substitution per block size (the
+// mixed build's 5x5 FP64 blocks do both in one)
+inline int implicit_launches(int kinds, int precision) {
+  return ((kinds & IMPL_FULL) ? (precision == EXO_PREC_MIXED ? 1 : 2) : 0) +
+         ((kinds & IMPL_PARTIAL) ? 2 : 0);
 }
 // shared doubles of one x1 column: w [nv][nc1] and psf [nc1+1]; the mixed
 // build adds ln psf and the face densities [2][nc1+1] and the cells' two

@@ -7,7 +7,7 @@
 // implicit solve, the equation of state and the conserved state stay FP64;
 // compiled with FMA).  EXO_KNS names the namespace of the build.
 //
-// One stage of SSPRK(3,3) is five launches, each one kernel over every
+// One stage of SSPRK(3,3) is six launches, each one kernel over every
 // member of a batch (a single atmosphere is a batch of one):
 //   kb_flux_x1    per radial column: hydrostatic decomposition, WENO5 in x1,
 //                 restore, Riemann solve -> x1 face fluxes         (exo3 only)
@@ -17,8 +17,10 @@
 //                 this panel's basis; Riemann solve -> x2/x3 fluxes
 //   kb_update     per cell: RK register average, flux divergence, geometric
 //                 source, gravity / Coriolis -> u (exo2) or du (exo3)
-//   kb_implicit   per radial column: 5x5 block-tridiagonal vertical correction,
-//                 u += du, AirParcel round trip on the last stage (exo3)
+//   kb_implicit   per radial column: forward sweep of the block-tridiagonal
+//                 vertical correction (5x5 or 3x3 blocks); kb_implicit_bwd: its
+//                 back substitution, u += delta, AirParcel round trip on the
+//                 last stage (exo3)
 //   kb_prim_ghost per cell incl. ghosts: ConservedToPrimitive of the interior,
 //                 of the ghost bands interpolated from the neighbour panels and
 //                 of the reflected x1 ghosts; CFL time-step candidate
@@ -61,10 +63,6 @@
 #ifndef EXO_X1_SHARED_BETA
 #define EXO_X1_SHARED_BETA EXO_MIXED
 #endif
-// 1: the implicit solve keeps (A c)_{i-1} in shared memory instead of registers
-#ifndef EXO_IMPL_AP_SMEM
-#define EXO_IMPL_AP_SMEM 0
-#endif
 
 namespace exo {
 namespace EXO_KNS {
@@ -83,8 +81,7 @@ __device__ __forceinline__ double abs_r(double x) { return fabs(x); }
 // rcp.approx.ftz.f64 refined by two Newton-Raphson steps, r <- r + r (1 - x r)
 // (Newton's method for 1/x: the relative error squares each step, so a
 // seed good to 2^-14 or better ends within an ulp or two of 1/x), instead of
-// the IEEE division sequence: 3.6 % less implicit time at 6x192^2x96, on
-// the LU pivots and the divisions of |A|.  The mixed build's primitive and
+// an IEEE division.  The mixed build's primitive and
 // update kernels take their reciprocals (density, sin^2, volume, radius)
 // the same way.  The FP64 build divides.
 #ifndef EXO_IMPL_RCP_NR
@@ -1227,6 +1224,13 @@ __device__ __forceinline__ void cp_async8(double* smem_dst, const double* gsrc) 
   unsigned sa = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
 }
+// one value of the implicit solve's factors (4 or 8 bytes)
+template <class R>
+__device__ __forceinline__ void cp_async_r(R* smem_dst, const R* gsrc) {
+  unsigned sa = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sa), "l"(gsrc), "n"((int)sizeof(R))
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -1654,11 +1658,18 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
 #pragma unroll
     for (int n = 0; n < 4; ++n) uout[n * vs] = un[n];
   } else if (v.implicit_flag & 1) {
+    // the 3x3 correction leaves the tangential momenta's update as it is, so
+    // it is applied here and the solve moves neither
     double* duout = v.du + c0;
+    const bool partial = !(v.implicit_flag & 8);
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      uout[n * vs] = un[n];
-      duout[n * vs] = du[n];
+      if (partial && (n == IVY || n == IVZ)) {
+        uout[n * vs] = un[n] + 1. * du[n];
+      } else {
+        uout[n * vs] = un[n];
+        duout[n * vs] = du[n];
+      }
     }
   } else {
 #pragma unroll
@@ -1668,20 +1679,25 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
 
 // ------------------------------------------------------------- k_implicit -
 // flux_decomposition.hpp:34-120, X1 direction
-__device__ __forceinline__ void roe_average(double* prim, double gm1, const double* wl,
-                                            const double* wr) {
+#if !EXO_MIXED
+struct GasDiv {
+  SharedDiv gm1, gp1;  // divisions by gamma - 1 and by gamma - 1 + 1
+};
+__device__ __forceinline__ void roe_average(double* prim, double gm1, const GasDiv& gd,
+                                            const double* wl, const double* wr) {
   double sqrtdl = sqrt(wl[IDN]), sqrtdr = sqrt(wr[IDN]);
   double isdlpdr = 1.0 / (sqrtdl + sqrtdr);
   prim[IDN] = sqrtdl * sqrtdr;
   prim[IVX] = (sqrtdl * wl[IVX] + sqrtdr * wr[IVX]) * isdlpdr;
   prim[IVY] = (sqrtdl * wl[IVY] + sqrtdr * wr[IVY]) * isdlpdr;
   prim[IVZ] = (sqrtdl * wl[IVZ] + sqrtdr * wr[IVZ]) * isdlpdr;
-  double el = wl[IPR] / gm1 + 0.5 * wl[IDN] * (sqr(wl[IVX]) + sqr(wl[IVY]) + sqr(wl[IVZ]));
-  double er = wr[IPR] / gm1 + 0.5 * wr[IDN] * (sqr(wr[IVX]) + sqr(wr[IVY]) + sqr(wr[IVZ]));
+  double el = gd.gm1(wl[IPR]) + 0.5 * wl[IDN] * (sqr(wl[IVX]) + sqr(wl[IVY]) + sqr(wl[IVZ]));
+  double er = gd.gm1(wr[IPR]) + 0.5 * wr[IDN] * (sqr(wr[IVX]) + sqr(wr[IVY]) + sqr(wr[IVZ]));
   double hbar = ((el + wl[IPR]) / sqrtdl + (er + wr[IPR]) / sqrtdr) * isdlpdr;
-  prim[IPR] = (hbar - 0.5 * (sqr(prim[IVX]) + sqr(prim[IVY]) + sqr(prim[IVZ]))) * gm1 /
-              (gm1 + 1.) * prim[IDN];
+  prim[IPR] = gd.gp1((hbar - 0.5 * (sqr(prim[IVX]) + sqr(prim[IVY]) + sqr(prim[IVZ]))) * gm1) *
+              prim[IDN];
 }
+#endif
 
 // Structural non-zeros of the X1 flux Jacobian dF/dq (flux_decomposition.hpp:
 // 100-120): row 0 = e_1; rows 2 and 3 carry three entries each.
@@ -1743,22 +1759,19 @@ __device__ __forceinline__ void unroll(F&& f) {
   unroll_impl<N>(f, std::make_integer_sequence<int, N>{});
 }
 
+#if EXO_MIXED
 // |A| = R |Lambda| R^-1 at the Roe average of a face (flux_decomposition.hpp:
-// 34-98).  Exact build: the reference's products R*Lambda and (R*Lambda)*R^-1
-// summed in its order, skipping only terms that are structurally zero (the
-// value is the same; at most the sign of an exact zero differs).  Mixed
-// build: the same matrix as |u| I + (|u-c|-|u|) r0 l0^T + (|u+c|-|u|) r2 l2^T
-// (the three |u| eigenvalues coincide), with shared reciprocals.  FP32
-// blocks take sqrt(rho) and 1/sqrt(rho) from the cells and the sound speed
-// and its reciprocal from one rsqrt (one rsqrt and two reciprocals a face;
-// 1.6 % faster); FP64 blocks keep sqrt and division, which measured 3 %
-// faster than the same rewrite in FP64.
+// 34-98) as |u| I + (|u-c|-|u|) r0 l0^T + (|u+c|-|u|) r2 l2^T (the three |u|
+// eigenvalues coincide), with shared reciprocals.  FP32 blocks take sqrt(rho)
+// and 1/sqrt(rho) from the cells and the sound speed and its reciprocal from
+// one rsqrt (one rsqrt and two reciprocals a face; 1.6 % faster); FP64 blocks
+// keep sqrt and division, which measured 3 % faster than the same rewrite in
+// FP64.
 template <class R>
 __device__ __forceinline__ void abs_jacobian(const ColCell<R>& L, const ColCell<R>& R_, R gm1,
                                              R gamma, R A[5][5]) {
   R wl[5] = {L.rho, L.v1, L.v2, L.v3, L.p};
   R wr[5] = {R_.rho, R_.v1, R_.v2, R_.v3, R_.p};
-#if EXO_MIXED
   // FP32 blocks take the cells' sqrt(rho) and 1/sqrt(rho); the same scheme
   // in FP64 (with a Newton-refined rsqrt) measured 0.5 % slower
   constexpr bool f32 = sizeof(R) == 4;
@@ -1823,25 +1836,39 @@ __device__ __forceinline__ void abs_jacobian(const ColCell<R>& L, const ColCell<
   for (int r = 0; r < 5; ++r)
 #pragma unroll
     for (int c = 0; c < 5; ++c) A[r][c] = (r == c ? au : R(0)) + r0[r] * l0[c] + r2[r] * l2[c];
+}
 #else
+// |A| = R |Lambda| R^-1 at the Roe average of a face (flux_decomposition.hpp:
+// 34-98): the reference's products R*Lambda and (R*Lambda)*R^-1 summed in its
+// order, skipping only terms that are structurally zero (the value is the
+// same; at most the sign of an exact zero differs).
+__device__ __forceinline__ void abs_jacobian(const ColCell<double>& L, const ColCell<double>& R_,
+                                             double gm1, double gamma, const GasDiv& gd,
+                                             double A[5][5]) {
+  const double wl[5] = {L.rho, L.v1, L.v2, L.v3, L.p};
+  const double wr[5] = {R_.rho, R_.v1, R_.v2, R_.v3, R_.p};
   double prim[5];
-  roe_average(prim, gm1, wl, wr);
+  roe_average(prim, gm1, gd, wl, wr);
   double fsig = 1., feps = 1.;
-  double cs = sqrt((1. + (gamma - 1) * feps / fsig) * prim[IPR] / prim[IDN]);
   double rr = prim[IDN], u = prim[IVX], v = prim[IVY], w = prim[IVZ], p = prim[IPR];
+  // divisions by a common denominator share its reciprocal (SharedDiv: the
+  // IEEE quotient)
+  const SharedDiv by_rr(rr);
+  double cs = sqrt(by_rr((1. + (gamma - 1) * feps / fsig) * p));
   double ke = 0.5 * (u * u + v * v + w * w);
-  double hp = (gm1 + 1.) / gm1 * p / rr;
+  double hp = by_rr((gm1 + 1.) / gm1 * p);
   double h = hp + ke;
   const double Rm[5][5] = {{1., 1., 1., 0., 0.},
                            {u - cs, u, u + cs, 0., 0.},
                            {v, v, v, 1., 0.},
                            {w, w, w, 0., 1.},
                            {h - u * cs, ke, h + u * cs, v, w}};
-  double mv2 = -v / (2. * hp), mw2 = -w / (2. * hp), i2 = 1. / (2. * hp);
+  const SharedDiv by_hp(hp), by_2hp(2. * hp), by_2cshp(2. * cs * hp);
+  double mv2 = by_2hp(-v), mw2 = by_2hp(-w), i2 = by_2hp.r;
   const double Ri[5][5] = {
-      {(cs * ke + u * hp) / (2. * cs * hp), (-hp - cs * u) / (2. * cs * hp), mv2, mw2, i2},
-      {(hp - ke) / hp, u / hp, v / hp, w / hp, -1. / hp},
-      {(cs * ke - u * hp) / (2. * cs * hp), (hp - cs * u) / (2. * cs * hp), mv2, mw2, i2},
+      {by_2cshp(cs * ke + u * hp), by_2cshp(-hp - cs * u), mv2, mw2, i2},
+      {by_hp(hp - ke), by_hp(u), by_hp(v), by_hp(w), -by_hp.r},
+      {by_2cshp(cs * ke - u * hp), by_2cshp(hp - cs * u), mv2, mw2, i2},
       {-v, 0., 1., 0., 0.},
       {-w, 0., 0., 1., 0.}};
   const double lam[5] = {fabs(u - cs), fabs(u), fabs(u + cs), fabs(u), fabs(u)};
@@ -1860,30 +1887,16 @@ __device__ __forceinline__ void abs_jacobian(const ColCell<R>& L, const ColCell<
         }
       A[r][c] = s;
     }
-#endif
 }
+#endif
 
 // Solve with the LU factors of implicit_column's mixed build (rows taken in
-// the order 1, 4, 2, 3, 0, threshold row swaps packed 3 bits per step): y
-// holds the right-hand side with its rows in natural order on entry and the
-// solution, unknowns in order, on exit.
+// the order 1, 4, 2, 3, 0): y holds the right-hand side, its rows already
+// swapped as the factors' were, on entry and the solution, unknowns in
+// order, on exit.
 template <class R>
-__device__ __forceinline__ void lu_solve_rows(const R (&t)[5][5], const R (&idg)[5],
-                                              unsigned perm, bool swapped, R* y) {
+__device__ __forceinline__ void lu_solve_rows(const R (&t)[5][5], const R (&idg)[5], R* y) {
   constexpr int O[5] = {1, 4, 2, 3, 0};
-  if (swapped) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const unsigned pk = (perm >> (3 * k)) & 7u;
-#pragma unroll
-      for (int r = k + 1; r < 5; ++r) {
-        const bool sw = (pk == (unsigned)r);
-        const R a = y[O[k]], b = y[O[r]];
-        y[O[k]] = sw ? b : a;
-        y[O[r]] = sw ? a : b;
-      }
-    }
-  }
 #pragma unroll
   for (int r = 1; r < 5; ++r)
 #pragma unroll
@@ -1900,271 +1913,68 @@ __device__ __forceinline__ void lu_solve_rows(const R (&t)[5][5], const R (&idg)
   for (int r = 0; r < 5; ++r) y[r] = z[r];
 }
 
-// BackwardSubstitution of the full correction (forward_backward.hpp:90-126):
-// delta_i -= (A c)_i delta_{i+1} from level ie (delta_ie given in dp) down
-// to is, each corrected update stored through io.  kPipe: software-pipelined,
-// the next level's factors and state in flight while a level finishes (for
-// the few resident columns of the solve kernel); otherwise one level at a
-// time, leaving the latency to the many columns of the back-substitution
-// kernel.
-template <class IO, bool kPipe = true>
-__device__ __forceinline__ void implicit_backward_full(IO& io, int is, int ie,
-                                                       typename IO::Real* dp) {
-  using R = typename IO::Real;
-  auto store = [&](int i, const double* u) {
-    double d[5];
-#pragma unroll
-    for (int n = 0; n < 5; ++n) d[n] = dp[n];
-    io.ustore(i, u, d);
-  };
-  if constexpr (!kPipe) {
-    {
-      double u[5];
-      io.uload(ie, u);
-      store(ie, u);
-    }
+// The forward sweep's inputs, w(i+1) and du(i) of level i, brought in by the
+// whole warp four levels at a time (lane -> level lane & 3 of columns
+// (lane >> 2) + 8 m).  What limits these loads is not bytes but the 128-byte
+// lines of L1 they hold while in flight, one per (column, variable) run,
+// whatever the run's length: with copies of one level per lane, and with
+// runs of two, more warps per SM made the solve slower (fewer lines left of
+// L1 beside their shared memory).  A level takes a warp several
+// microseconds among seven others, so the batch is waited for where it is
+// issued: a second buffer would only cost shared memory.  Column c keeps
+// level k at place (k + c/4) & 3, which keeps a warp's reads of one level on
+// distinct banks.
+constexpr int LEVEL_TILE_DOUBLES = 10 * 32 * 4;
+template <class IO, int ND>
+struct LevelTile {
+  double* tile;
+  int is, L;
+  __device__ __forceinline__ static int var(int m) {
+    return ND == 5 ? m : (m == 2 ? IEN : m);
+  }
+  __device__ __forceinline__ LevelTile(const IO&, double* t, int is_, int L_)
+      : tile(t), is(is_), L(L_) {}
+  // level k's values are about to be read
+  __device__ __forceinline__ void ready(const IO& io, int k0) {
+    if (k0 & 3) return;
+    const int lane = (int)(threadIdx.x & 31), k = k0 + (lane & 3);
+    __syncwarp();
+    const unsigned long long wo =
+        reinterpret_cast<unsigned long long>(io.wptr(is + 1 + k0, 0));
+    const unsigned long long uo = reinterpret_cast<unsigned long long>(io.duptr(is + k0, 0));
+    const size_t ws = io.wstride(), ds = io.dstride();
 #pragma unroll 1
-    for (int i = ie - 1; i >= is; --i) {
-      R cs[30];
-      double u[5];
+    for (int m = 0; m < 4; ++m) {
+      const int c = (lane >> 2) + 8 * m;
+      const double* wp = reinterpret_cast<const double*>(__shfl_sync(0xffffffffu, wo, c)) +
+                         (lane & 3);
+      const double* dp = reinterpret_cast<const double*>(__shfl_sync(0xffffffffu, uo, c)) +
+                         (lane & 3);
+      if (k < L) {
+        double* d = tile + c * 4 + ((k + (c >> 2)) & 3);
 #pragma unroll
-      for (int e = 0; e < 30; ++e) cs[e] = io.scr(i - is, e);
-      io.uload(i, u);
-      R dl[5];
+        for (int n = 0; n < 5; ++n) cp_async8(d + n * 128, wp + n * ws);
 #pragma unroll
-      for (int r = 0; r < 5; ++r) {
-        R ad = cs[r * 5] * dp[0];
-#pragma unroll
-        for (int k = 1; k < 5; ++k) ad += cs[r * 5 + k] * dp[k];
-        dl[r] = cs[25 + r] - ad;
-      }
-#pragma unroll
-      for (int r = 0; r < 5; ++r) dp[r] = dl[r];
-      store(i, u);
-    }
-    return;
-  }
-  R cur_s[30];
-  double cur_u[5];
-  io.uload(ie, cur_u);
-  store(ie, cur_u);
-  if (ie > is) {
-#pragma unroll
-    for (int e = 0; e < 30; ++e) cur_s[e] = io.scr(ie - 1 - is, e);
-    io.uload(ie - 1, cur_u);
-  }
-#pragma unroll 1
-  for (int i = ie - 1; i >= is; --i) {
-    R nxt_s[30];
-    double nxt_u[5];
-    if (i > is) {
-#pragma unroll
-      for (int e = 0; e < 30; ++e) nxt_s[e] = io.scr(i - 1 - is, e);
-      io.uload(i - 1, nxt_u);
-    }
-    R dl[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      R ad = cur_s[r * 5] * dp[0];
-#pragma unroll
-      for (int k = 1; k < 5; ++k) ad += cur_s[r * 5 + k] * dp[k];
-      dl[r] = cur_s[25 + r] - ad;
-    }
-#pragma unroll
-    for (int r = 0; r < 5; ++r) dp[r] = dl[r];
-    store(i, cur_u);
-    if (i > is) {
-#pragma unroll
-      for (int e = 0; e < 30; ++e) cur_s[e] = nxt_s[e];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) cur_u[n] = nxt_u[n];
-    }
-  }
-}
-
-// The back substitution of the stepping kernel's FP64 blocks (mixed build)
-// with the state u moved through shared memory by the warp: the warp's 32
-// columns go down BWD_TL levels at a time; each lane copies four levels of
-// a column for one variable in one 32-byte run (the per-lane accesses of
-// one level are 816 bytes apart, a sector each), the next chunk's copies in
-// flight while a chunk is corrected.  The factors are read per lane, one
-// level ahead, as in implicit_backward_full (they are contiguous across the
-// warp).  io.live: the lanes of the warp with a column.  wtile: 2 x 5 x 32 x
-// (BWD_TL + 1) doubles of shared memory for the warp alone.
-constexpr int BWD_TL = 4;
-// the two u tiles of a warp's back substitution (5 variables x 32 columns x
-// BWD_TL levels, padded)
-constexpr int WARP_TILE_DOUBLES = 2 * 5 * 32 * (BWD_TL + 1);
-// levels of look-ahead of the factor loads (1 or 2): two in the FP64 build
-// (implicit 8.63 -> 8.39 ms per 6x192^2x96 launch), one in the mixed build,
-// where two measured 2.6 % slower
-#ifndef EXO_BWD_AHEAD
-#define EXO_BWD_AHEAD (EXO_MIXED ? 1 : 2)
-#endif
-__device__ __forceinline__ void airparcel_round_trip(double* u, double Rd, double gamma);
-// the stepping solve's shared doubles per thread
-constexpr int IMPL_SM_STRIDE = EXO_IMPL_AP_SMEM ? 87 : 61;
-static_assert(32 * IMPL_SM_STRIDE >= WARP_TILE_DOUBLES,
-              "the tiled back substitution's buffers fit in the warp's slices");
-// NB = 5: the full correction (30 factors per level, delta on every
-// variable); NB = 3: the partial one (12 factors per level, delta on rho,
-// m1 and E, the explicit du on m2 and m3, read per lane one level ahead).
-template <int NB, class IO>
-__device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
-                                                        typename IO::Real* dp, double* wtile) {
-  static_assert(BWD_TL == 4, "the lane -> (column, level) split below assumes 4 levels");
-  static_assert(NB == 5 || NB == 3, "5x5 or 3x3 blocks");
-  constexpr int NF = NB * NB + NB;  // factors per level: (A c)_i and delta_i
-  constexpr int TS = BWD_TL + 1;
-  constexpr int TW = 5 * 32 * TS;
-  const unsigned live = io.live;
-  const int lane = (int)(threadIdx.x & 31);
-  __syncwarp(live);
-  // lane copies level (lane & 3) of columns (lane >> 2) + 8 m, m = 0..3
-  // (in a warp with a column in every lane)
-  double* ub[4];
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-    ub[m] = reinterpret_cast<double*>(__shfl_sync(
-        live, reinterpret_cast<unsigned long long>(io.uc), ((lane >> 2) + 8 * m) & 31));
-  const int l = lane & 3;
-  const int nch = (ie - is + BWD_TL) / BWD_TL;
-  auto range = [&](int c, int& lo, int& hi) {
-    hi = ie - c * BWD_TL;
-    lo = max(is, hi - BWD_TL + 1);
-  };
-  // a warp with a column in every lane copies in 32-byte runs; the last warp
-  // of a member may have fewer, and there each lane copies its own column
-  const bool full = live == 0xffffffffu;
-  auto load = [&](int c) {
-    double* t = wtile + (c & 1) * TW;
-    int lo, hi;
-    range(c, lo, hi);
-    if (full) {
-      if (lo + l <= hi) {
-#pragma unroll
-        for (int e = 0; e < 20; ++e) {
-          const int m = e & 3, n = e >> 2;
-          cp_async8(&t[(n * 32 + (lane >> 2) + 8 * m) * TS + l], ub[m] + n * io.vs + lo + l);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 20; ++e) {
-        const int ll = e & 3, n = e >> 2;
-        if (lo + ll <= hi) cp_async8(&t[(n * 32 + lane) * TS + ll], io.uc + n * io.vs + lo + ll);
+        for (int n = 0; n < ND; ++n) cp_async8(d + (5 + n) * 128, dp + var(n) * ds);
       }
     }
     cp_async_commit();
-  };
-  load(0);
-  if (nch > 1) load(1);
-  using R = typename IO::Real;
-  // the factors of the next level (cur_s) and, with EXO_BWD_AHEAD 2, of the
-  // one after (ahd_s): their loads are in flight for two levels (the
-  // registers of the finished forward sweep are free)
-  R cur_s[NF], ahd_s[NF];
-  if (ie > is) {
-#pragma unroll
-    for (int e = 0; e < NF; ++e) cur_s[e] = io.scr(ie - 1 - is, e);
+    cp_async_wait_all();
+    __syncwarp();
   }
-  if constexpr (EXO_BWD_AHEAD == 2) {
-    if (ie - 1 > is) {
-#pragma unroll
-      for (int e = 0; e < NF; ++e) ahd_s[e] = io.scr(ie - 2 - is, e);
-    }
+  __device__ __forceinline__ double get(int n, int k) const {
+    const int lane = (int)(threadIdx.x & 31);
+    return tile[n * 128 + lane * 4 + ((k + (lane >> 2)) & 3)];
   }
-  // the partial correction's explicit du of m2 and m3, one level ahead
-  double cur_du[2] = {0., 0.};
-  if constexpr (NB == 3) {
-    cur_du[0] = *io.duptr(ie, IVY);
-    cur_du[1] = *io.duptr(ie, IVZ);
-  }
-  for (int c = 0; c < nch; ++c) {
-    if (c + 1 < nch) cp_async_wait_one();
-    else cp_async_wait_all();
-    __syncwarp(live);
-    double* t = wtile + (c & 1) * TW;
-    int lo, hi;
-    range(c, lo, hi);
-    for (int i = hi; i >= lo; --i) {
-      double nxt_du[2] = {0., 0.};
-      if constexpr (NB == 3) {
-        if (i > is) {
-          nxt_du[0] = *io.duptr(i - 1, IVY);
-          nxt_du[1] = *io.duptr(i - 1, IVZ);
-        }
-      }
-      if (i < ie) {
-        R nxt_s[NF];
-        const int ahead = i - EXO_BWD_AHEAD;  // the level whose factors load now
-        if (ahead >= is) {
-#pragma unroll
-          for (int e = 0; e < NF; ++e) nxt_s[e] = io.scr(ahead - is, e);
-        }
-        R dl[NB];
-#pragma unroll
-        for (int r = 0; r < NB; ++r) {
-          R ad = cur_s[r * NB] * dp[0];
-#pragma unroll
-          for (int k = 1; k < NB; ++k) ad += cur_s[r * NB + k] * dp[k];
-          dl[r] = cur_s[NB * NB + r] - ad;
-        }
-#pragma unroll
-        for (int r = 0; r < NB; ++r) dp[r] = dl[r];
-        if constexpr (EXO_BWD_AHEAD == 2) {
-#pragma unroll
-          for (int e = 0; e < NF; ++e) {
-            cur_s[e] = ahd_s[e];
-            ahd_s[e] = nxt_s[e];
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < NF; ++e) cur_s[e] = nxt_s[e];
-        }
-      }
-      // the corrected update of every variable
-      double d[5];
-      if constexpr (NB == 5) {
-#pragma unroll
-        for (int n = 0; n < 5; ++n) d[n] = dp[n];
-      } else {
-        d[IDN] = dp[0];
-        d[IVX] = dp[1];
-        d[IVY] = cur_du[0];
-        d[IVZ] = cur_du[1];
-        d[IEN] = dp[2];
-        cur_du[0] = nxt_du[0];
-        cur_du[1] = nxt_du[1];
-      }
-      double uu[5];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) uu[n] = t[(n * 32 + lane) * TS + (i - lo)] + 1. * d[n];
-      if (io.stage == 2) airparcel_round_trip(uu, io.Rd, io.gamma);
-#pragma unroll
-      for (int n = 0; n < 5; ++n) t[(n * 32 + lane) * TS + (i - lo)] = uu[n];
-    }
-    __syncwarp(live);
-    if (full) {
-      if (lo + l <= hi) {
-#pragma unroll
-        for (int e = 0; e < 20; ++e) {
-          const int m = e & 3, n = e >> 2;
-          ub[m][n * io.vs + lo + l] = t[(n * 32 + (lane >> 2) + 8 * m) * TS + l];
-        }
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < 20; ++e) {
-        const int ll = e & 3, n = e >> 2;
-        if (lo + ll <= hi) io.uc[n * io.vs + lo + ll] = t[(n * 32 + lane) * TS + ll];
-      }
-    }
-    __syncwarp(live);
-    if (c + 2 < nch) load(c + 2);
-  }
-}
+};
 
+// shared memory of a warp of the solve: the level tile, then NE values of R
+// per lane, two face matrices (entry e of lane l at [e * 32 + l])
+template <class R, bool full>
+__host__ __device__ constexpr int impl_warp_doubles() {
+  constexpr int ne = full ? 50 : 18;
+  return LEVEL_TILE_DOUBLES + ne * 32 * (int)sizeof(R) / 8;
+}
 // The vertical 5x5 block-tridiagonal correction of one radial column
 // (ImplicitSolver::SolveImplicit3D X1 branch, solve_implicit_3d.cpp:102-179,
 // with FullCorrection, full_correction.cpp:32-165, and ForwardSweep /
@@ -2178,29 +1988,33 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
 //                reference's inverse) and multiplies, every sum in the
 //                reference's order: the result is the CPU restatement's to
 //                the bit;
-//   mixed build: solves t [X | y] = [c_i | x] by LU with partial pivoting.
-// (A c)_i (25) and delta_i (5) go to scratch for the back substitution.  The
-// face Jacobian |A|(i+1/2) waits in this thread's slice of shared memory
-// until it becomes |A|(i-1/2) of the next level.
-//   io.w(i, out[5])  primitives of level i (is-1 .. ie+2), unprojected
-//   io.scr(lev, e)   scratch double e (0..29) of level lev = i - is
-//   io.uload(i, u[5]), io.ustore(i, u[5], d[5])  the corrected update d of
-//                    level i, from ie down to is, with the state u loaded
-//                    for it beforehand (callers that only need d load nothing)
+//   mixed build: solves t [X | y] = [c_i | x] by LU with partial pivoting
+//                (FP32 blocks; FP64 ones run implicit_column_fused).
+// (A c)_i (25) and delta_i (5) go to scratch for the back substitution
+// (kb_implicit_bwd).
+//
+// What bounds it: at 252 registers eight warps share an SM, a warp issues
+// every 5 to 6 cycles (dependent FP64 operations), so time is instructions;
+// and the L1 beside the blocks' shared memory (see LevelTile).  FP64 build,
+// 6x96^2x64: 2863 warp instructions per level and 32 columns against 4481
+// with a division for every quotient, unconditional swaps and the back
+// substitution in the same kernel; forward sweep 964 us and back
+// substitution 246 us a solve against 1913.
+//   io.w(i, out[5])  primitives of level i (is-1, is), unprojected
+//   io.scr_level(lev)[e * io.scr_stride()]  factor e (0..29) of level lev = i - is
 //   io.wptr(i, n), io.duptr(i, n)  addresses of w and of the explicit update
-//                    du of level i (the inputs are prefetched through shared memory)
-//   sa, sp, ss       this thread's shared memory: entry e (0..49) of the two
-//                    face blocks at sa[e * ss], prefetch slot n (0..9) at
-//                    sp[n * ss]
-// kBwd false: the forward sweep only, with delta_ie stored as scratch
-// entries 25..29 of the last level (implicit_backward_full finishes it).
-template <class IO, bool kBwd = true>
-__device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, double* sp, int ss,
+//                    du of level i, io.wstride(), io.dstride() from one
+//                    variable to the next (LevelTile)
+//   sa, ss           this lane's shared memory: entry e of two face matrices
+//                    at sa[e * ss]
+//   wt               the warp's level tile
+template <class IO>
+__device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, int ss,
                                                 double cos_theta, double sin_theta, double d2,
                                                 double d3, const double* x1f, const double* x1v,
                                                 const double* dx1f, int is, int ie, double dt,
                                                 double gamma, double grav,
-                                                double* wt = nullptr) {
+                                                double* wt) {
   using R = typename IO::Real;
   using ColCell = exo::EXO_KNS::ColCell<R>;
   const double s = sin_theta;
@@ -2234,60 +2048,48 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
 #endif
     return c;
   };
-  auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 25 + r * 5 + q) * ss]; };
-
-  // prefetch slots: w(i+1) and du(i) of the next level, copied asynchronously
-  auto pw = [&](int n) -> double& { return sp[n * ss]; };
-  auto pdu = [&](int n) -> double& { return sp[(5 + n) * ss]; };
-  auto prefetch = [&](int iw, int idu) {
-#pragma unroll
-    for (int n = 0; n < 5; ++n) cp_async8(&pw(n), io.wptr(iw, n));
-    if (idu >= 0) {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) cp_async8(&pdu(n), io.duptr(idu, n));
-    }
-    cp_async_commit();
-  };
+  LevelTile<IO, 5> lt(io, wt, is, ie - is + 1);
   double raw[5];
   io.w(is - 1, raw);
   ColCell cm = cell(raw);
   io.w(is, raw);
   ColCell c0 = cell(raw);
-  prefetch(is + 1, is);
+  auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 25 + r * 5 + q) * ss]; };
+#if EXO_MIXED
+  auto face_jacobian = [&](const ColCell& lo, const ColCell& hi, R (&A)[5][5]) {
+    abs_jacobian(lo, hi, gm1, gam, A);
+  };
+#else
+  const GasDiv gd{SharedDiv(gm1), SharedDiv(gm1 + 1.)};
+  const SharedDiv by_dt(dt);
+  auto face_jacobian = [&](const ColCell& lo, const ColCell& hi, R (&A)[5][5]) {
+    abs_jacobian(lo, hi, gm1, gam, gd, A);
+  };
+#endif
   {
     R A[5][5];
-    abs_jacobian(cm, c0, gm1, gam, A);
+    face_jacobian(cm, c0, A);
 #pragma unroll
     for (int r = 0; r < 5; ++r)
 #pragma unroll
       for (int q = 0; q < 5; ++q) AMs(0, r, q) = A[r][q];
   }
-  // (A c)_{i-1} lives in registers, or in this thread's shared memory when
-  // EXO_IMPL_AP_SMEM (fewer registers, more resident warps)
-#if EXO_IMPL_AP_SMEM
-  static_assert(sizeof(R) == 8, "(A c)_{i-1} in shared memory takes the FP64 slice layout");
-  double* const aps = sa + 60;
-#define EXO_AP(r, q) aps[(r) * 5 + (q)]
-#else
-  R Ap[5][5];
-#define EXO_AP(r, q) Ap[r][q]
-#endif
+  R Ap[5][5];  // (A c)_{i-1}
   R dp[5];  // delta_{i-1}
   int cur = 0;
   for (int i = is; i <= ie; ++i) {
-    cp_async_wait_all();
+    lt.ready(io, i - is);
     double rhs[5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      raw[n] = pw(n);
-      rhs[n] = pdu(n);
+      raw[n] = lt.get(n, i - is);
+      rhs[n] = lt.get(5 + n, i - is);
     }
     ColCell cp = cell(raw);
-    prefetch(i + 2, i < ie ? i + 1 : -1);
     const int nxt = cur ^ 1;
     {
       R A[5][5];
-      abs_jacobian(c0, cp, gm1, gam, A);
+      face_jacobian(c0, cp, A);
 #pragma unroll
       for (int r = 0; r < 5; ++r)
 #pragma unroll
@@ -2299,6 +2101,8 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
 #if EXO_MIXED
     const double i2v = 0.5 / vol;
     const R bl = R(aleft * i2v), cr = R(aright * i2v), dd = R((aright - aleft) * i2v);
+#else
+    const SharedDiv by_2vol(2. * vol);
 #endif
     const bool first = (i == is), last = (i == ie);
     R x[5];
@@ -2328,17 +2132,17 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
 #else
         double num = am * aleft + ap * aright;
         if constexpr (fj_nz(r, q)) num = num + (aright - aleft) * fj_entry<r, q>(c0, gm1);
-        double a = num / (2. * vol);
+        double a = by_2vol(num);
         if constexpr (r == q) a = a + rdt;
         if constexpr ((r == IVX && q == IDN) || (r == IEN && q == IVX)) a = a - grav;
         double bm = am;
         if constexpr (fj_nz(r, q)) bm = am + fj_entry<r, q>(cm, gm1);
-        double b = -bm * aleft / (2. * vol);
+        double b = by_2vol(-bm * aleft);
         if (first) a = a + ((q == IVX) ? -b : b);
         if (last) {
           double cmv = ap;
           if constexpr (fj_nz(r, q)) cmv = ap - fj_entry<r, q>(cp, gm1);
-          double c = -cmv * aright / (2. * vol);
+          double c = by_2vol(-cmv * aright);
           a = a + ((q == IVX) ? -c : c);
         }
 #endif
@@ -2348,14 +2152,14 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
 #if EXO_MIXED
       x[r] = R(rhs[r]) * rdt;
 #else
-      x[r] = rhs[r] / dt;
+      x[r] = by_dt(rhs[r]);
 #endif
       if (!first) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
-          R ba = brow[0] * EXO_AP(0, q);
+          R ba = brow[0] * Ap[0][q];
 #pragma unroll
-          for (int k = 1; k < 5; ++k) ba += brow[k] * EXO_AP(k, q);
+          for (int k = 1; k < 5; ++k) ba += brow[k] * Ap[k][q];
           trow[q] = trow[q] - ba;
         }
         R bd = brow[0] * dp[0];
@@ -2382,7 +2186,7 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
         c[r] = -cmv * cr;
 #else
         if constexpr (fj_nz(r, q)) cmv = cmv - fj_entry<r, q>(cp, gm1);
-        c[r] = -cmv * aright / (2. * vol);
+        c[r] = by_2vol(-cmv * aright);
 #endif
       });
     };
@@ -2391,7 +2195,8 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
     // pivoting ends with for nearly every block of this solve (density last,
     // energy and x1 momentum first) -- and threshold partial pivoting on top:
     // a row swap only where the diagonal falls below a tenth of the largest
-    // entry of its column, so the swap code is skipped almost always.
+    // entry of its column.  The search and the swaps stand behind a vote, so
+    // they are skipped almost always.
     constexpr int O[5] = {1, 4, 2, 3, 0};
     unsigned perm = 0;  // 3 bits per step: the position swapped in
     bool swapped = false;
@@ -2401,15 +2206,20 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
       if (k < 4) {
         const R dk = abs_r(t[O[k]][k]);
         R best = dk;
-        int piv = k;
 #pragma unroll
-        for (int r = k + 1; r < 5; ++r) {
-          const R m = abs_r(t[O[r]][k]);
-          if (m > best) { best = m; piv = r; }
-        }
-        if (dk < R(0.1) * best) {
+        for (int r = k + 1; r < 5; ++r) best = fmax(best, abs_r(t[O[r]][k]));
+        const bool small = dk < R(0.1) * best;
+        int piv = k;
+        if (__any_sync(0xffffffffu, small)) {
+          if (small) {
+            best = dk;
+#pragma unroll
+            for (int r = k + 1; r < 5; ++r) {
+              const R m = abs_r(t[O[r]][k]);
+              if (m > best) { best = m; piv = r; }
+            }
+          }
           swapped = true;
-          perm |= (unsigned)piv << (3 * k);
 #pragma unroll
           for (int r = k + 1; r < 5; ++r) {
             const bool sw = (piv == r);
@@ -2420,9 +2230,8 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
               t[O[r]][q] = sw ? a : b;
             }
           }
-        } else {
-          perm |= (unsigned)k << (3 * k);
         }
+        perm |= (unsigned)piv << (3 * k);
       }
       idg[k] = inv_r(t[O[k]][k]);
 #pragma unroll
@@ -2433,16 +2242,34 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
         for (int q = k + 1; q < 5; ++q) t[O[r]][q] -= l * t[O[k]][q];
       }
     }
-    auto solve = [&](R* y) { lu_solve_rows(t, idg, perm, swapped, y); };
-    solve(x);
-    unroll<5>([&](auto Q) {
-      constexpr int q = decltype(Q)::value;
-      R c[5];
-      ccol(Q, c);
-      solve(c);
+    // the right-hand sides' rows follow the swaps
+    auto solve = [&](R* y) {
+      if (swapped) {
 #pragma unroll
-      for (int r = 0; r < 5; ++r) EXO_AP(r, q) = c[r];
-    });
+        for (int k = 0; k < 4; ++k) {
+          const unsigned pk = (perm >> (3 * k)) & 7u;
+#pragma unroll
+          for (int r = k + 1; r < 5; ++r) {
+            const bool sw = (pk == (unsigned)r);
+            const R a = y[O[k]], b = y[O[r]];
+            y[O[k]] = sw ? b : a;
+            y[O[r]] = sw ? a : b;
+          }
+        }
+      }
+      lu_solve_rows(t, idg, y);
+    };
+    solve(x);
+    if (!last) {
+      unroll<5>([&](auto Q) {
+        constexpr int q = decltype(Q)::value;
+        R c[5];
+        ccol(Q, c);
+        solve(c);
+#pragma unroll
+        for (int r = 0; r < 5; ++r) Ap[r][q] = c[r];
+      });
+    }
 #pragma unroll
     for (int r = 0; r < 5; ++r) dp[r] = x[r];
 #else
@@ -2463,6 +2290,7 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
 #pragma unroll
       for (int r = k + 1; r < 5; ++r) {
         bool sw = (piv == r);
+        if (!__any_sync(0xffffffffu, sw)) continue;  // most rows are no lane's pivot
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
           if (q >= k) {
@@ -2509,44 +2337,25 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
         double acc = B[r][0] * c[0];
 #pragma unroll
         for (int k = 1; k < 5; ++k) acc += B[r][k] * c[k];
-        EXO_AP(r, q) = acc;
+        Ap[r][q] = acc;
       }
     });
 #endif
-    const int lev = i - is;
+    R* const scl = io.scr_level(i - is);
+    const size_t scs = io.scr_stride();
     if (!last) {
 #pragma unroll
       for (int r = 0; r < 5; ++r)
 #pragma unroll
-        for (int q = 0; q < 5; ++q) io.scr(lev, r * 5 + q) = EXO_AP(r, q);
-#pragma unroll
-      for (int r = 0; r < 5; ++r) io.scr(lev, 25 + r) = dp[r];
+        for (int q = 0; q < 5; ++q) scl[(r * 5 + q) * scs] = Ap[r][q];
     }
-    if constexpr (!kBwd) {
-      if (last) {
 #pragma unroll
-        for (int r = 0; r < 5; ++r) io.scr(lev, 25 + r) = dp[r];
-      }
-    }
+    for (int r = 0; r < 5; ++r) scl[(25 + r) * scs] = dp[r];
     cm = c0;
     c0 = cp;
     cur = nxt;
   }
-  // the last level's prefetch (unused) must land before the back substitution
-  // reuses this thread's slots of shared memory
-  cp_async_wait_all();
-  if constexpr (!kBwd) return;
-  if constexpr (IO::kLoadsU && sizeof(R) == 8) {
-    if (io.stage >= 0) {
-      // the warp's tiles (FP64 blocks: its 32 shared slices, free once every
-      // lane has finished its forward sweep)
-      implicit_backward_tiled<5>(io, is, ie, dp, wt);
-      return;
-    }
-  }
-  implicit_backward_full(io, is, ie, dp);
 }
-#undef EXO_AP
 
 // ImplicitSolver::PartialCorrection (partial_correction.cpp:26-173) of one
 // radial column, one thread per column: the 3x3 block-tridiagonal system of
@@ -2557,61 +2366,16 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, d
 // correction corr is zero (its computation is commented out there).  Each
 // 3x3 block is inverted as its adjugate over its determinant, the closed form
 // a fixed-size 3x3 inverse takes.  Scratch per level: (A c)_i (9) and
-// delta_i (3).  IO and arguments as for implicit_column; the shared slices
-// hold the two face blocks (18 entries of sa) and the prefetched w (5) and
-// du (3) of a level (sp).
-// BackwardSubstitution of the partial correction: delta_i -= (A c)_i
-// delta_{i+1} for (rho, m1, E) from level ie (delta_ie in dp) down to is;
-// the update of level i takes delta for rho, m1, E and the explicit du for
-// m2, m3.
+// delta_i (3).  IO and arguments as for implicit_column.  A solve at
+// 6x62^2x45 (mixed build) went from 173 to 126 us, at 6x40^3 (FP64 build) from
+// 213 to 100 us.
 template <class IO>
-__device__ __forceinline__ void implicit_backward_partial(IO& io, int is, int ie,
-                                                          typename IO::Real* dp) {
-  using R = typename IO::Real;
-  auto store = [&](int i, const double* u) {
-    double dl[5];
-    dl[IDN] = dp[0];
-    dl[IVX] = dp[1];
-    dl[IVY] = *io.duptr(i, IVY);
-    dl[IVZ] = *io.duptr(i, IVZ);
-    dl[IEN] = dp[2];
-    io.ustore(i, u, dl);
-  };
-  {
-    double u_ie[5];
-    io.uload(ie, u_ie);
-    store(ie, u_ie);
-  }
-#pragma unroll 1
-  for (int i = ie - 1; i >= is; --i) {
-    R cs[12];
-    double u[5];
-#pragma unroll
-    for (int e = 0; e < 12; ++e) cs[e] = io.scr(i - is, e);
-    io.uload(i, u);
-    R dl[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      R ad = cs[r * 3] * dp[0];
-#pragma unroll
-      for (int k = 1; k < 3; ++k) ad += cs[r * 3 + k] * dp[k];
-      dl[r] = cs[9 + r] - ad;
-    }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) dp[r] = dl[r];
-    store(i, u);
-  }
-}
-
-// kBwd false: the forward sweep only, with delta_ie stored as scratch
-// entries 9..11 of the last level (implicit_backward_partial finishes it).
-template <class IO, bool kBwd = true>
-__device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Real* sa, double* sp, int ss,
+__device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Real* sa, int ss,
                                                         double cos_theta, double sin_theta,
                                                         double d2, double d3, const double* x1f,
                                                         const double* x1v, const double* dx1f,
                                                         int is, int ie, double dt, double gamma,
-                                                        double grav, double* wt = nullptr) {
+                                                        double grav, double* wt) {
   using R = typename IO::Real;
   using ColCell = exo::EXO_KNS::ColCell<R>;
   constexpr int P[3] = {IDN, IVX, IEN};
@@ -2644,45 +2408,41 @@ __device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Rea
 #endif
     return c;
   };
-  auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 9 + r * 3 + q) * ss]; };
-  auto face = [&](const ColCell& lo, const ColCell& hi, int slot) {
-    R A[5][5];
-    abs_jacobian(lo, hi, gm1, gam, A);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) AMs(slot, r, q) = A[P[r]][P[q]];
-  };
-  auto pw = [&](int n) -> double& { return sp[n * ss]; };
-  auto pdu = [&](int m) -> double& { return sp[(5 + m) * ss]; };
-  auto prefetch = [&](int iw, int idu) {
-#pragma unroll
-    for (int n = 0; n < 5; ++n) cp_async8(&pw(n), io.wptr(iw, n));
-    if (idu >= 0) {
-#pragma unroll
-      for (int m = 0; m < 3; ++m) cp_async8(&pdu(m), io.duptr(idu, P[m]));
-    }
-    cp_async_commit();
-  };
+  LevelTile<IO, 3> lt(io, wt, is, ie - is + 1);
   double raw[5];
   io.w(is - 1, raw);
   ColCell cm = cell(raw);
   io.w(is, raw);
   ColCell c0 = cell(raw);
-  prefetch(is + 1, is);
+  auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 9 + r * 3 + q) * ss]; };
+#if !EXO_MIXED
+  const GasDiv gd{SharedDiv(gm1), SharedDiv(gm1 + 1.)};
+  const SharedDiv by_dt(dt);
+#endif
+  auto face = [&](const ColCell& lo, const ColCell& hi, int slot) {
+    R A[5][5];
+#if EXO_MIXED
+    abs_jacobian(lo, hi, gm1, gam, A);
+#else
+    abs_jacobian(lo, hi, gm1, gam, gd, A);
+#endif
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) AMs(slot, r, q) = A[P[r]][P[q]];
+  };
   face(cm, c0, 0);
   R Ap[3][3];  // (A c)_{i-1}
   R dp[3];     // delta_{i-1}
   int cur = 0;
   for (int i = is; i <= ie; ++i) {
-    cp_async_wait_all();
+    lt.ready(io, i - is);
     double rhs[3];
 #pragma unroll
-    for (int n = 0; n < 5; ++n) raw[n] = pw(n);
+    for (int n = 0; n < 5; ++n) raw[n] = lt.get(n, i - is);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) rhs[m] = pdu(m);
+    for (int m = 0; m < 3; ++m) rhs[m] = lt.get(5 + m, i - is);
     ColCell cp = cell(raw);
-    prefetch(i + 2, i < ie ? i + 1 : -1);
     const int nxt = cur ^ 1;
     face(c0, cp, nxt);
     const double aleft = d2 * d3 * x1f[i] * x1f[i] * s;
@@ -2691,6 +2451,8 @@ __device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Rea
 #if EXO_MIXED
     const double i2v = 0.5 / vol;
     const R bl = R(aleft * i2v), cr = R(aright * i2v), dd = R((aright - aleft) * i2v);
+#else
+    const SharedDiv by_2vol(2. * vol);
 #endif
     const bool first = (i == is), last = (i == ie);
     R t[3][3], cc[3][3], x[3];
@@ -2720,15 +2482,15 @@ __device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Rea
 #else
         double num = am * aleft + ap * aright;
         if constexpr (fj_nz(pr, pq)) num = num + (aright - aleft) * fj_entry<pr, pq>(c0, gm1);
-        double a = num / (2. * vol);
+        double a = by_2vol(num);
         if constexpr (r == q) a = a + rdt;
         if constexpr (phi) a = a - grav;
         double bm = am;
         if constexpr (fj_nz(pr, pq)) bm = am + fj_entry<pr, pq>(cm, gm1);
-        double b = -bm * aleft / (2. * vol);
+        double b = by_2vol(-bm * aleft);
         double cmv = ap;
         if constexpr (fj_nz(pr, pq)) cmv = ap - fj_entry<pr, pq>(cp, gm1);
-        double c = -cmv * aright / (2. * vol);
+        double c = by_2vol(-cmv * aright);
         if (first) a = a + ((q == 1) ? -b : b);
         if (last) a = a + ((q == 1) ? -c : c);
 #endif
@@ -2739,7 +2501,7 @@ __device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Rea
 #if EXO_MIXED
       x[r] = R(rhs[r]) * rdt;
 #else
-      x[r] = rhs[r] / dt;
+      x[r] = by_dt(rhs[r]);
 #endif
       if (!first) {
 #pragma unroll
@@ -2791,34 +2553,20 @@ __device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Rea
         for (int k = 1; k < 3; ++k) acc += B[r][k] * cc[k][q];
         Ap[r][q] = acc;
       }
+    R* const scl = io.scr_level(i - is);
+    const size_t scs = io.scr_stride();
     if (!last) {
-      const int lev = i - is;
 #pragma unroll
       for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) io.scr(lev, r * 3 + q) = Ap[r][q];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) io.scr(lev, 9 + r) = dp[r];
+        for (int q = 0; q < 3; ++q) scl[(r * 3 + q) * scs] = Ap[r][q];
     }
-    if constexpr (!kBwd) {
-      if (last) {
 #pragma unroll
-        for (int r = 0; r < 3; ++r) io.scr(i - is, 9 + r) = dp[r];
-      }
-    }
+    for (int r = 0; r < 3; ++r) scl[(9 + r) * scs] = dp[r];
     cm = c0;
     c0 = cp;
     cur = nxt;
   }
-  cp_async_wait_all();  // the last level's prefetch (unused) lands before the slice is reused
-  if constexpr (!kBwd) return;
-  if constexpr (IO::kLoadsU && sizeof(R) == 8) {
-    if (io.stage >= 0) {
-      implicit_backward_tiled<3>(io, is, ie, dp, wt);
-      return;
-    }
-  }
-  implicit_backward_partial(io, is, ie, dp);
 }
 
 // UpdateAllConserved on the last stage with NVAPOR = NCLOUD = 0: the
@@ -2865,70 +2613,40 @@ __device__ __forceinline__ void airparcel_round_trip(double* uu, double Rd, doub
   uu[IEN] = e;
 }
 
-// Launch shape of the implicit kernels: one thread per radial column, 64
-// columns per block, 60 doubles of shared memory per thread (the face
-// Jacobians |A|(i-1/2) and |A|(i+1/2), the next level's w and du).
+// Launch shape of the forward sweep: one thread per radial column, 64
+// columns per block.
 constexpr int IMPL_THREADS = 64;      // default; 32 and 128 are the other tiles
 constexpr int IMPL_MAX_THREADS = 128;
-#ifndef EXO_IMPL_MINB
-#define EXO_IMPL_MINB 2  // resident 128-thread blocks per SM the register budget is sized for
-#endif
-// the mixed build's solve is capped at 204 registers (8 bytes of spill),
-// measured 18 % faster at 6x192^2x96 than uncapped; with the per-warp
-// register rounding that still leaves 4 blocks of 64 columns per SM (8 warps).
-// 200 registers fit a fifth block but measured 1-3 % slower, so the forward
-// sweep is bound by its FP64 dependency chains, not by resident warps.  The
-// FP64 build spills below 254 registers and keeps the full register file.
-#if !defined(EXO_IMPL_MAXNREG) && EXO_MIXED
-#define EXO_IMPL_MAXNREG 204
-#endif
-#ifdef EXO_IMPL_MAXNREG
-#define EXO_IMPL_BOUNDS __maxnreg__(EXO_IMPL_MAXNREG)
-#else
-#define EXO_IMPL_BOUNDS __launch_bounds__(IMPL_MAX_THREADS, EXO_IMPL_MINB)
-#endif
-// FP64 solve: each thread's doubles are contiguous (60, or 85 with
-// (A c)_{i-1} kept there), threads IMPL_SM_STRIDE doubles apart (defined
-// with the back substitution): an odd stride keeps a half-warp's 8-byte
-// accesses on distinct banks.
-// FP32 solve: structure of arrays, the 10 prefetch doubles of every thread
-// first, then the 50 FP32 face-block entries, entry e of thread t at
-// [e * threads + t], so a warp's accesses are consecutive words.
-template <class R>
-__host__ __device__ constexpr int impl_slice_doubles() {
-  return sizeof(R) == 4 ? 10 + 50 / 2 : IMPL_SM_STRIDE;
-}
-// per block: the threads' slices, then x1f (nc1+1), x1v (nc1), dx1f (nc1)
-template <class R>
+// Two 128-thread blocks per SM: the full register file.  A smaller budget
+// spills, and a spill goes past the little L1 that the shared memory leaves
+// (FP64 build at 6x96^2x64 capped at 204: 2247 instead of 1905 us).
+#define EXO_IMPL_BOUNDS __launch_bounds__(IMPL_MAX_THREADS, 2)
+// per block: the warps' shared memory, then x1f (nc1+1), x1v (nc1), dx1f (nc1)
+template <class R, bool full>
 __host__ __device__ constexpr size_t impl_smem(int threads, int nc1) {
-  return ((size_t)impl_slice_doubles<R>() * threads + 3 * (size_t)(nc1 + 1)) * sizeof(double);
+  return ((size_t)impl_warp_doubles<R, full>() * (threads / 32) + 3 * (size_t)(nc1 + 1)) *
+         sizeof(double);
 }
-// this thread's slices of the block's shared memory (arguments sa, sp, ss of
-// implicit_column and implicit_column_partial)
+// this lane's shared memory (arguments sa, ss, wt of implicit_column and
+// implicit_column_partial)
 template <class R>
 struct ImplSlices {
   R* sa;
-  double* sp;
   int ss;
-  double* wt;  // FP64 blocks: the warp's back-substitution tiles (WARP_TILE_DOUBLES)
+  double* wt;  // the warp's tiles
 };
-template <class R>
-__device__ __forceinline__ ImplSlices<R> impl_slices(double* ism, bool full) {
-  if constexpr (sizeof(R) == 4) {
-    const int nt = (int)blockDim.x, t = (int)threadIdx.x;
-    return {reinterpret_cast<R*>(ism + 10 * nt) + t, ism + t, nt, nullptr};
-  } else {
-    double* sm = ism + threadIdx.x * IMPL_SM_STRIDE;
-    return {sm, sm + (full ? 50 : 18), 1, ism + (threadIdx.x & ~31u) * IMPL_SM_STRIDE};
-  }
+template <class R, bool full>
+__device__ __forceinline__ ImplSlices<R> impl_slices(double* ism) {
+  double* w = ism + (threadIdx.x >> 5) * impl_warp_doubles<R, full>();
+  return {reinterpret_cast<R*>(w + LEVEL_TILE_DOUBLES) + (threadIdx.x & 31), 32, w};
 }
 // where the block's copy of the radial geometry starts
-template <class R>
+template <class R, bool full>
 __device__ __forceinline__ double* impl_radial(double* ism) {
-  return ism + blockDim.x * impl_slice_doubles<R>();
+  return ism + (blockDim.x >> 5) * impl_warp_doubles<R, full>();
 }
 // the largest dynamic shared memory a launch may ask for
-constexpr int IMPL_SMEM_MAX = 160 * 1024;
+constexpr int IMPL_SMEM_MAX = 160 * 1024;  // 128 threads, 250 levels
 
 // copies the radial geometry of the member into shared memory (all threads
 // of the block take part; returns the shared copies)
@@ -2953,48 +2671,25 @@ __device__ __forceinline__ void stage_radial(double* sg, int nc1, const double* 
 }
 
 // A column of the stepping context: primitives and update from the state
-// arrays, the corrected update added to u (with the AirParcel round trip on
-// the last stage).
+// arrays, factors in the member's scratch.
 template <class R>
 struct StepColumnIO {
   using Real = R;
   const double* wc;
   const double* duc;
-  double* uc;
-  size_t vs;       // stride between variables
-  R* scr0;         // scratch of this column: [level][entry][32 lanes] per warp of columns
-  int stage;            // < 0: write the corrected update into du, leave u alone
-  double Rd, gamma;
-  double* duw;          // du of this column, for stage < 0
+  size_t vs;  // stride between variables
+  R* scr0;    // scratch of this column: [level][entry][32 lanes] per warp of columns
   __device__ __forceinline__ void w(int i, double* out) const {
 #pragma unroll
     for (int n = 0; n < 5; ++n) out[n] = wc[n * vs + i];
   }
+  __device__ __forceinline__ size_t wstride() const { return vs; }
+  __device__ __forceinline__ size_t dstride() const { return vs; }
   __device__ __forceinline__ const double* wptr(int i, int n) const { return wc + n * vs + i; }
   __device__ __forceinline__ const double* duptr(int i, int n) const { return duc + n * vs + i; }
-  __device__ __forceinline__ R& scr(int lev, int e) const {
-    return scr0[(lev * 30 + e) * 32];
-  }
-  static constexpr bool kLoadsU = true;
-  unsigned live = 0xffffffffu;  // the lanes of the warp with a column
-  __device__ __forceinline__ void uload(int i, double* u) const {
-    if (stage < 0) return;
-#pragma unroll
-    for (int n = 0; n < 5; ++n) u[n] = uc[n * vs + i];
-  }
-  __device__ __forceinline__ void ustore(int i, const double* u, const double* dl) const {
-    if (stage < 0) {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) duw[n * vs + i] = dl[n];
-      return;
-    }
-    double uu[5];
-#pragma unroll
-    for (int n = 0; n < 5; ++n) uu[n] = u[n] + 1. * dl[n];
-    if (stage == 2) airparcel_round_trip(uu, Rd, gamma);
-#pragma unroll
-    for (int n = 0; n < 5; ++n) uc[n * vs + i] = uu[n];
-  }
+  // the factors of a level: entry e at scr_level(lev)[e * 32]
+  __device__ __forceinline__ R* scr_level(int lev) const { return scr0 + (size_t)lev * (30 * 32); }
+  __device__ __forceinline__ size_t scr_stride() const { return 32; }
 };
 
 // One radial column of the stepping context: solve, then u += du and, on
@@ -3002,7 +2697,7 @@ struct StepColumnIO {
 // stage 0..2: a stage of the step (dt = beta_stage * the CFL step, u += du);
 // stage -1: ImplicitSolver::SolveImplicit3D alone (dt given, du corrected in
 // place)
-template <class R>
+template <class R, bool full>
 __device__ __forceinline__ void implicit_block(const DevView& v, unsigned blk, int stage,
                                                double dt_given = 0.) {
   extern __shared__ double ism[];
@@ -3013,219 +2708,270 @@ __device__ __forceinline__ void implicit_block(const DevView& v, unsigned blk, i
   const double* x1f;
   const double* x1v;
   const double* dx1f;
-  stage_radial(impl_radial<R>(ism), v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
-  const unsigned live = __ballot_sync(0xffffffffu, col < ncol);
-  if (col >= ncol) return;
-  const int j = v.js + col % v.N;
-  const int k = v.ks + (col / v.N) % v.N;
-  const int p = col / (v.N * v.N);
+  stage_radial(impl_radial<R, full>(ism), v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
+  if ((col & ~31) >= ncol) return;
+  // lanes past the last column repeat it: same values to the same places
+  // (their own scratch; it holds whole groups of 32 columns)
+  const int cc = min(col, ncol - 1);
+  const int j = v.js + cc % v.N;
+  const int k = v.ks + (cc / v.N) % v.N;
+  const int p = cc / (v.N * v.N);
   const double dt = stage < 0 ? dt_given : rk_beta(stage) * v.sc->dt;
   const size_t base = idx(v, p, 0, k, j, 0);
   // scratch in blocks of 32 columns: a warp's 32 entries are 128 (FP32) or
   // 256 (FP64) contiguous bytes
   R* scr0 = reinterpret_cast<R*>(v.scratch) + (size_t)(col >> 5) * v.L * 30 * 32 + (col & 31);
-  StepColumnIO<R> io{v.w + base, v.du + base, v.u + base, v.cells, scr0, stage, v.Rd, v.gamma,
-                     v.du + base};
-  io.live = live;
-  const bool full = (v.implicit_flag & 8) != 0;
-  const ImplSlices<R> sl = impl_slices<R>(ism, full);
-  using IO = StepColumnIO<R>;
-  // FP32 blocks: the back substitution of the full correction is
-  // kb_implicit_bwd's (split_bwd; the lighter partial one stays here: split,
-  // it measured slower)
-  constexpr bool kBwd = sizeof(R) == 8;
-  if (full)
-    implicit_column<IO, kBwd>(io, sl.sa, sl.sp, sl.ss, geo(v, GCOSC, p, k, j),
-                                         geo(v, GSINC, p, k, j), geo(v, GDX2A, p, k, j),
-                                         geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is, v.ie,
-                                         dt, v.gamma, v.grav, sl.wt);
+  StepColumnIO<R> io{v.w + base, v.du + base, v.cells, scr0};
+  const ImplSlices<R> sl = impl_slices<R, full>(ism);
+  if constexpr (full)
+    implicit_column(io, sl.sa, sl.ss, geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j),
+                    geo(v, GDX2A, p, k, j), geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is, v.ie,
+                    dt, v.gamma, v.grav, sl.wt);
   else
-    implicit_column_partial<IO, true>(io, sl.sa, sl.sp, sl.ss,
-                                                 geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j),
-                                                 geo(v, GDX2A, p, k, j), geo(v, GDX3A, p, k, j),
-                                                 x1f, x1v, dx1f, v.is, v.ie, dt, v.gamma, v.grav,
-                                                 sl.wt);
+    implicit_column_partial(io, sl.sa, sl.ss, geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j),
+                            geo(v, GDX2A, p, k, j), geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is,
+                            v.ie, dt, v.gamma, v.grav, sl.wt);
 }
+
+#if EXO_MIXED
+#include "exo_implicit_fused.cuh"
+#endif
 
 // ---------------------------------------------------- kb_implicit_bwd ---
-// The back substitution of the full correction, delta_i -= (A c)_i
-// delta_{i+1} from the top level down, u += delta (with the AirParcel round
-// trip on the last stage), as a kernel of its own after the forward sweep
-// (kb_implicit, which leaves (A c)_i and delta_i of every level in scratch),
-// for FP32 blocks.  It streams 120 bytes of scratch and 80 bytes of u per
-// cell and computes little, so it is built to keep HBM busy: one
-// warp per group of 32 columns, whose scratch is one contiguous run per
-// chunk of BWD_LEV levels ([group][level][entry][32]); the chunk below the
-// one being finished is already on its way into the other shared-memory
-// buffer, by one bulk TMA copy (cp.async.bulk, completion counted by an
-// mbarrier) for the factors and by 8-byte cp.async copies for u (four lanes
-// read one column's four levels: a 32-byte run per column and variable).
-// u is updated in the shared tile and written back the same way.
-constexpr int BWD_LEV = 4;  // levels per chunk
-// the shared memory of one warp: two buffers, each the factor chunk and the
-// u tile [5][32][BWD_LEV + 1] (padded: a warp's column-wise accesses of one
-// level fall on distinct banks), then the two mbarriers
-template <class R>
-__host__ __device__ constexpr size_t bwd_chunk_bytes() {
-  return (size_t)BWD_LEV * 30 * 32 * sizeof(R);
-}
-constexpr int BWD_TILE_DOUBLES = 5 * 32 * (BWD_LEV + 1);
-template <class R>
-__host__ __device__ constexpr size_t bwd_buffer_bytes() {
-  return bwd_chunk_bytes<R>() + BWD_TILE_DOUBLES * sizeof(double);
-}
-template <class R>
-__host__ __device__ constexpr size_t impl_bwd_smem() {
-  return 2 * bwd_buffer_bytes<R>() + 16;
-}
-static_assert(bwd_chunk_bytes<float>() % 16 == 0 && bwd_buffer_bytes<float>() % 16 == 0,
-              "bulk copies move multiples of 16 bytes to 16-byte aligned addresses");
-static_assert(bwd_chunk_bytes<double>() % 16 == 0 && bwd_buffer_bytes<double>() % 16 == 0,
-              "bulk copies move multiples of 16 bytes to 16-byte aligned addresses");
+// The back substitution, delta_i -= (A c)_i delta_{i+1} from the top level
+// down, u += delta (with the AirParcel round trip on the last stage), as a
+// kernel of its own after the forward sweep, which leaves (A c)_i and
+// delta_i of every level in scratch.  It streams 240 bytes of factors (FP64,
+// 5x5) and 80 bytes of u per cell and computes little, so it is built to
+// keep HBM busy: in the forward kernel, whose registers and shared memory
+// leave eight warps per SM, it took 1.6 of 3.95 ms per 6x192^2x96 launch
+// (FP64 factors); FP32 blocks at 6x126^2x70 went from 1255 to 1170 us a solve.
+// A block of three warps takes 32 columns.  The solver warp runs the
+// recursion, one column per lane, on factors that arrive level by level in a
+// ring of FRING levels: one bulk copy a level (32 columns' factors of a
+// level are contiguous), counted on an mbarrier, its wait bounded.  It
+// leaves the corrections of CL levels at a time in shared memory; the other
+// two warps add them to u meanwhile, a column's CL levels side by side.
+template <class R, int NB>
+struct BwdLayout {
+  static constexpr int NM = NB * NB, NFAC = NM + NB;
+  static constexpr int FRING = 4, CL = 4, DS = CL + 1;
+  static constexpr size_t level_bytes = (size_t)NFAC * 32 * sizeof(R);
+  static constexpr size_t fac_bytes = FRING * level_bytes;
+  static constexpr size_t del_bytes = (size_t)2 * NB * 32 * DS * sizeof(double);
+  static constexpr size_t bytes = fac_bytes + del_bytes;
+  static_assert(level_bytes % 16 == 0, "bulk copies move multiples of 16 bytes");
+};
+constexpr int BWD_THREADS = 96;
 
 template <class R>
-__device__ __forceinline__ void implicit_bwd_warp(const DevView& v, int group, int stage) {
+struct BwdGroup {
+  const R* scr;          // factor e of level l of column c: scr[l lstride + e estride + c]
+  size_t lstride, estride;
+  double* x;             // u (stage >= 0) or du (stage < 0): x[off[c] + n vs + l]
+  size_t vs;
+  const long long* off;  // shared memory, 32 entries
+  int ncols, L, stage;
+  double Rd, gamma;
+  int* timeout;          // sticky flag of a wait that gave up
+};
+
+// kBulk: the factors of 32 columns of a level are contiguous and 16-byte
+// aligned (the stepping scratch); otherwise each lane copies its own
+template <class R, int NB, bool kBulk>
+__device__ __forceinline__ void implicit_bwd_group(const BwdGroup<R>& g, unsigned char* sm) {
+  using LY = BwdLayout<R, NB>;
+  constexpr int NM = LY::NM, NFAC = LY::NFAC, FRING = LY::FRING, CL = LY::CL, DS = LY::DS;
+  static_assert((FRING & (FRING - 1)) == 0, "ring slots by mask");
+  __shared__ unsigned long long full[FRING];
+  __shared__ int s_stop;  // the first chunk a wait that gave up left unfinished
+  R* const ring = reinterpret_cast<R*>(sm);
+  double* const del = reinterpret_cast<double*>(sm + LY::fac_bytes);
+  const int lane = (int)(threadIdx.x & 31), L = g.L;
+  const int nch = (L + CL - 1) / CL;
+  auto var = [](int m) { return NB == 5 ? m : (m == 2 ? (int)IEN : m); };
+  if (threadIdx.x < 32) {
+    // the j-th level from the top, into slot j
+    auto issue = [&](int j) {
+      const int l = L - 1 - j;
+      R* dst = ring + (j & (FRING - 1)) * NFAC * 32;
+      if constexpr (kBulk) {
+        if (l >= 0 && lane == 0) {
+          mbar_expect_tx(&full[j & (FRING - 1)], (unsigned)LY::level_bytes);
+          bulk_g2s(dst, g.scr + (size_t)l * g.lstride, (unsigned)LY::level_bytes,
+                   &full[j & (FRING - 1)]);
+        }
+      } else {
+        if (l >= 0 && lane < g.ncols) {
+          const R* src = g.scr + (size_t)l * g.lstride + lane;
+#pragma unroll
+          for (int e = 0; e < NFAC; ++e) cp_async_r(dst + e * 32 + lane, src + e * g.estride);
+        }
+        cp_async_commit();
+      }
+    };
+    if constexpr (kBulk) {
+      if (lane == 0) {
+#pragma unroll
+        for (int s = 0; s < FRING; ++s) mbar_init(&full[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+      }
+      __syncwarp();
+    }
+#pragma unroll 1
+    for (int j = 0; j < FRING; ++j) issue(j);
+    if (lane == 0) s_stop = nch;
+    bool ok = true;
+    R dp[NB];
+#pragma unroll
+    for (int r = 0; r < NB; ++r) dp[r] = R(0);
+#pragma unroll 1
+    for (int c = 0; c <= nch; ++c) {
+      const int hi = L - 1 - c * CL, lo = max(0, hi - CL + 1);
+      double* const d = del + (c & 1) * NB * 32 * DS + lane * DS;
+      if (c < nch && ok) {
+#pragma unroll 1
+        for (int l = hi; l >= lo; --l) {
+          const int j = L - 1 - l;
+          if constexpr (kBulk) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[j & (FRING - 1)], (j / FRING) & 1));
+            if (!ok) break;
+          } else {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(FRING - 1) : "memory");
+            __syncwarp();
+          }
+          const R* f = ring + (j & (FRING - 1)) * NFAC * 32 + lane;
+          // delta of the top level is its own (its (A c) is not formed)
+          R dl[NB];
+#pragma unroll
+          for (int r = 0; r < NB; ++r) {
+            dl[r] = f[(NM + r) * 32];
+            if (j > 0) {
+              R ad = f[(r * NB) * 32] * dp[0];
+#pragma unroll
+              for (int k = 1; k < NB; ++k) ad += f[(r * NB + k) * 32] * dp[k];
+              dl[r] = dl[r] - ad;
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < NB; ++r) {
+            dp[r] = dl[r];
+            d[r * 32 * DS + (l - lo)] = (double)dl[r];
+          }
+          __syncwarp();
+          issue(j + FRING);
+        }
+        if (!ok && lane == 0) s_stop = c;
+      }
+      __syncthreads();
+    }
+    if (!ok) {
+      // a bulk copy did not complete in time: record it, and give every copy
+      // still outstanding a bounded wait before the shared memory is released
+      if (lane == 0) atomicOr(g.timeout, 1);
+      for (int s = 0; s < FRING; ++s) {
+        mbar_wait(&full[s], 0);
+        mbar_wait(&full[s], 1);
+      }
+    }
+    if constexpr (!kBulk) cp_async_wait_all();
+  } else {
+    // cells (column, level) of a chunk: two per thread
+    const int t0 = (int)threadIdx.x - 32;
+    auto place = [&](int c, int m, int& col, int& l) {
+      const int t = t0 + 64 * m, hi = L - 1 - c * CL, lo = max(0, hi - CL + 1);
+      col = t / CL;
+      l = lo + t % CL;
+      return col < g.ncols && l <= hi;
+    };
+    // the 3x3 correction leaves m2 and m3 to the update kernel; the last
+    // stage's round trip takes every variable
+    const bool all = g.stage == 2;
+    auto moved = [&](int n) { return NB == 5 || all || (n != IVY && n != IVZ); };
+    auto load = [&](int c, int m, double* u) {
+      int col, l;
+      if (g.stage < 0 || !place(c, m, col, l)) return;
+      const double* p = g.x + g.off[col] + l;
+#pragma unroll
+      for (int n = 0; n < 5; ++n)
+        if (moved(n)) u[n] = p[n * g.vs];
+    };
+    double cur0[5] = {}, cur1[5] = {}, nxt0[5] = {}, nxt1[5] = {};
+#pragma unroll 1
+    for (int c = 0; c <= nch; ++c) {
+      if (c < nch) {
+        load(c, 0, nxt0);
+        load(c, 1, nxt1);
+      }
+      if (c > 0) {
+        const double* d = del + ((c - 1) & 1) * NB * 32 * DS;
+        const int lo = max(0, L - (c - 1) * CL - CL);
+        // not unrolled: one copy of the round trip's code
+#pragma unroll 1
+        for (int m = 0; m < 2; ++m) {
+          int col, l;
+          if (!place(c - 1, m, col, l) || c - 1 >= s_stop) continue;
+          double* p = g.x + g.off[col] + l;
+          double dv[5];
+#pragma unroll
+          for (int r = 0; r < NB; ++r) dv[var(r)] = d[(r * 32 + col) * DS + (l - lo)];
+          if (g.stage < 0) {
+#pragma unroll
+            for (int r = 0; r < NB; ++r) p[var(r) * g.vs] = dv[var(r)];
+          } else {
+            double uu[5];
+#pragma unroll
+            for (int n = 0; n < 5; ++n) {
+              uu[n] = m ? cur1[n] : cur0[n];
+              if (NB == 5 || (n != IVY && n != IVZ)) uu[n] = uu[n] + 1. * dv[n];
+            }
+            if (all) airparcel_round_trip(uu, g.Rd, g.gamma);
+#pragma unroll
+            for (int n = 0; n < 5; ++n)
+              if (moved(n)) p[n * g.vs] = uu[n];
+          }
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        cur0[n] = nxt0[n];
+        cur1[n] = nxt1[n];
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Columns 32 group .. of a member: a stage of the step (stage 0..2, u), or
+// SolveImplicit3D alone (stage < 0, du).  If a wait gave up, the columns keep
+// the forward sweep's state below the last finished chunk.
+template <class R, bool full>
+__device__ __forceinline__ void implicit_bwd_block(const DevView& v, int group, int stage) {
   extern __shared__ __align__(128) unsigned char bws[];
-  const int lane = (int)(threadIdx.x & 31);
-  const int ncol = 6 * v.N * v.N;
-  const int col0 = group * 32, col = col0 + lane;
-  const bool active = col < ncol;
-  const int ncb = min(32, ncol - col0);
-  const int L = v.L;
-  const size_t vs = v.cells;
-  size_t base = 0;
-  if (active) {
+  __shared__ long long s_off[32];
+  const int ncol = 6 * v.N * v.N, col0 = group * 32;
+  if (threadIdx.x < 32) {
+    const int col = min(col0 + (int)threadIdx.x, ncol - 1);
     const int j = v.js + col % v.N;
     const int k = v.ks + (col / v.N) % v.N;
     const int p = col / (v.N * v.N);
-    base = idx(v, p, 0, k, j, 0);
+    s_off[threadIdx.x] = (long long)idx(v, p, 0, k, j, v.is);
   }
-  // this column's scratch: entry e of level lev at sg[(lev * 30 + e) * 32 + lane]
-  const R* sg = reinterpret_cast<const R*>(v.scratch) + (size_t)group * L * 30 * 32;
-  unsigned long long* mb = reinterpret_cast<unsigned long long*>(bws + 2 * bwd_buffer_bytes<R>());
-  auto chunk_scr = [&](int b) { return reinterpret_cast<R*>(bws + b * bwd_buffer_bytes<R>()); };
-  auto chunk_tile = [&](int b) {
-    return reinterpret_cast<double*>(bws + b * bwd_buffer_bytes<R>() + bwd_chunk_bytes<R>());
-  };
-  if (lane == 0) {
-    mbar_init(&mb[0], 1);
-    mbar_init(&mb[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncwarp();
-  // the column bases of the group, for the tile copies
-  const long long cb_lane = active ? (long long)base : 0;
-  const int nch = (L + BWD_LEV - 1) / BWD_LEV;
-  double* const u = v.u;
-  // chunk c holds levels [c * BWD_LEV, min(L, (c + 1) * BWD_LEV)) (level
-  // index i - is); a tile element e is (variable n, column c, level l)
-  auto issue = [&](int c, int b) {
-    const int lo = c * BWD_LEV, nl = min(L, lo + BWD_LEV) - lo;
-    if (lane == 0) {
-      const unsigned bytes = (unsigned)(nl * 30 * 32 * sizeof(R));
-      mbar_expect_tx(&mb[b], bytes);
-      bulk_g2s(chunk_scr(b), sg + (size_t)lo * 30 * 32, bytes, &mb[b]);
-    }
-    double* tile = chunk_tile(b);
-    for (int e = lane; e < 5 * 32 * BWD_LEV; e += 32) {
-      const int l = e & (BWD_LEV - 1), cc = (e / BWD_LEV) & 31, n = e / (BWD_LEV * 32);
-      const long long cbase = __shfl_sync(0xffffffffu, cb_lane, cc);
-      if (cc < ncb && l < nl)
-        cp_async8(&tile[(n * 32 + cc) * (BWD_LEV + 1) + l], u + cbase + n * vs + v.is + lo + l);
-    }
-    cp_async_commit();
-  };
-  unsigned phases = 0u;   // bit b: the phase buffer b's mbarrier completes next
-  unsigned pending = 0u;  // bit b: buffer b's bulk copy is still outstanding
-  bool ok = true;
-  R dp[5] = {R(0), R(0), R(0), R(0), R(0)};
-  issue(nch - 1, 0);
-  pending |= 1u;
-  int b = 0;
-  for (int c = nch - 1; c >= 0; --c) {
-    if (c > 0) {
-      issue(c - 1, b ^ 1);
-      pending |= 1u << (b ^ 1);
-    }
-    // the factors of chunk c (bounded wait; the whole warp agrees) and its u tile
-    const bool got = mbar_wait(&mb[b], (phases >> b) & 1u);
-    if (!__all_sync(0xffffffffu, got)) {
-      ok = false;
-      break;
-    }
-    phases ^= 1u << b;
-    pending &= ~(1u << b);
-    if (c > 0) cp_async_wait_one();
-    else cp_async_wait_all();
-    __syncwarp();
-    const R* cs = chunk_scr(b);
-    double* tile = chunk_tile(b);
-    const int lo = c * BWD_LEV, nl = min(L, lo + BWD_LEV) - lo;
-    if (active) {
-      for (int l = nl - 1; l >= 0; --l) {
-        const int lev = lo + l;
-        const R* f = cs + (size_t)l * 30 * 32 + lane;
-        if (lev == L - 1) {
-#pragma unroll
-          for (int r = 0; r < 5; ++r) dp[r] = f[(25 + r) * 32];  // delta_ie
-        } else {
-          R dl[5];
-#pragma unroll
-          for (int r = 0; r < 5; ++r) {
-            R ad = f[(r * 5) * 32] * dp[0];
-#pragma unroll
-            for (int k = 1; k < 5; ++k) ad += f[(r * 5 + k) * 32] * dp[k];
-            dl[r] = f[(25 + r) * 32] - ad;
-          }
-#pragma unroll
-          for (int r = 0; r < 5; ++r) dp[r] = dl[r];
-        }
-        // StepColumnIO::ustore with u in the tile
-        double uu[5];
-#pragma unroll
-        for (int n = 0; n < 5; ++n)
-          uu[n] = tile[(n * 32 + lane) * (BWD_LEV + 1) + l] + 1. * (double)dp[n];
-        if (stage == 2) airparcel_round_trip(uu, v.Rd, v.gamma);
-#pragma unroll
-        for (int n = 0; n < 5; ++n) tile[(n * 32 + lane) * (BWD_LEV + 1) + l] = uu[n];
-      }
-    }
-    __syncwarp();
-    for (int e = lane; e < 5 * 32 * BWD_LEV; e += 32) {
-      const int l = e & (BWD_LEV - 1), cc = (e / BWD_LEV) & 31, n = e / (BWD_LEV * 32);
-      const long long cbase = __shfl_sync(0xffffffffu, cb_lane, cc);
-      if (cc < ncb && l < nl)
-        u[cbase + n * vs + v.is + lo + l] = tile[(n * 32 + cc) * (BWD_LEV + 1) + l];
-    }
-    __syncwarp();
-    b ^= 1;
-  }
-  if (!ok) {
-    // a bulk copy did not complete in time: record it, and give every copy
-    // still outstanding a bounded wait before this warp's shared memory is
-    // released (the columns keep the forward sweep's state)
-    if (lane == 0) atomicOr(&v.sc->timeout, 1);
-    for (int bb = 0; bb < 2; ++bb)
-      if ((pending >> bb) & 1u) mbar_wait(&mb[bb], (phases >> bb) & 1u);
-    cp_async_wait_all();
-  }
-}
-
-// SolveImplicit3D alone (stage < 0): du corrected in place, column by column
-template <class R>
-__device__ __forceinline__ void implicit_bwd_du(const DevView& v, int col) {
-  if (col >= 6 * v.N * v.N) return;
-  const int j = v.js + col % v.N;
-  const int k = v.ks + (col / v.N) % v.N;
-  const int p = col / (v.N * v.N);
-  const size_t base = idx(v, p, 0, k, j, 0);
-  R* scr0 = reinterpret_cast<R*>(v.scratch) + (size_t)(col >> 5) * v.L * 30 * 32 + (col & 31);
-  StepColumnIO<R> io{v.w + base, v.du + base, v.u + base, v.cells, scr0, -1, v.Rd, v.gamma,
-                     v.du + base};
-  R dp[5];
-#pragma unroll
-  for (int r = 0; r < 5; ++r) dp[r] = io.scr(v.L - 1, 25 + r);
-  implicit_backward_full<StepColumnIO<R>, false>(io, v.is, v.ie, dp);
+  __syncthreads();
+  BwdGroup<R> g;
+  g.scr = reinterpret_cast<const R*>(v.scratch) + (size_t)group * v.L * 30 * 32;
+  g.lstride = 30 * 32;
+  g.estride = 32;
+  g.x = stage < 0 ? v.du : v.u;
+  g.vs = v.cells;
+  g.off = s_off;
+  g.ncols = min(32, ncol - col0);
+  g.L = v.L;
+  g.stage = stage;
+  g.Rd = v.Rd;
+  g.gamma = v.gamma;
+  g.timeout = &v.sc->timeout;
+  implicit_bwd_group<R, full ? 5 : 3, true>(g, bws);
 }
 
 // last-stage round trip when the implicit solver is off
@@ -3394,39 +3140,49 @@ __global__ void EXO_UPD_BOUNDS kb_update(Batch bt, int stage) {
   update_block<T>(sv, b, stage);
 }
 
-template <class R>
+// One kernel per block size (full: 5x5, else 3x3), each over the blocks of
+// every member; members of the other kind are skipped.
+template <class R, bool full>
 __global__ void EXO_IMPL_BOUNDS kb_implicit(Batch bt, int stage, double dt_given) {
   __shared__ __align__(16) DevView sv;
   unsigned b = batch_enter(bt, sv);
   if (sv.eqn == EXO_EQN_SHALLOW_YZ || !(sv.implicit_flag & 1)) return;
-  implicit_block<R>(sv, b, stage, dt_given);
+  if (((sv.implicit_flag & 8) != 0) != full) return;
+  implicit_block<R, full>(sv, b, stage, dt_given);
 }
 
-// One warp per group of 32 columns: implicit block b of a member (its
-// columns b*T .. b*T+T-1 at T = the implicit tile) is T/32 blocks here.
-template <class R>
-__global__ void __launch_bounds__(32) kb_implicit_bwd(Batch bt, int stage, int warps_per_iblock) {
+#if EXO_MIXED
+__global__ void __maxnreg__(204) kb_implicit_fused(Batch bt, int stage, double dt_given) {
   __shared__ __align__(16) DevView sv;
-  const unsigned ib = blockIdx.x / (unsigned)warps_per_iblock;
+  unsigned b = batch_enter(bt, sv);
+  if (sv.eqn == EXO_EQN_SHALLOW_YZ || !(sv.implicit_flag & 1)) return;
+  if (!(sv.implicit_flag & 8)) return;
+  implicit_fused_block<double>(sv, b, stage, dt_given);
+}
+#endif
+
+// A block per group of 32 columns: implicit block b of a member (its
+// columns b*T .. b*T+T-1 at T = the implicit tile) is T/32 blocks here.
+template <class R, bool full>
+__global__ void __launch_bounds__(BWD_THREADS) kb_implicit_bwd(Batch bt, int stage,
+                                                               int groups_per_iblock) {
+  __shared__ __align__(16) DevView sv;
+  static_assert(sizeof(DevView) % 16 == 0, "DevView is copied in 16-byte words");
+  const unsigned ib = blockIdx.x / (unsigned)groups_per_iblock;
+  const int m = batch_member(bt, ib);
   {
-    static_assert(sizeof(DevView) % 16 == 0, "DevView is copied in 16-byte words");
-    const int m = batch_member(bt, ib);
     const int4* src = reinterpret_cast<const int4*>(bt.views + m);
     int4* dst = reinterpret_cast<int4*>(&sv);
     for (int t = threadIdx.x; t < (int)(sizeof(DevView) / 16); t += blockDim.x) dst[t] = src[t];
-    __syncwarp();
   }
-  const int m = batch_member(bt, ib);
   const unsigned local = ib - bt.start[m];
-  // members with the partial correction finished in kb_implicit
-  if (sv.eqn == EXO_EQN_SHALLOW_YZ || !(sv.implicit_flag & 1) || !(sv.implicit_flag & 8)) return;
-  const int group = (int)(local * (unsigned)warps_per_iblock + blockIdx.x % (unsigned)warps_per_iblock);
+  __syncthreads();
+  if (sv.eqn == EXO_EQN_SHALLOW_YZ || !(sv.implicit_flag & 1)) return;
+  if (((sv.implicit_flag & 8) != 0) != full) return;
+  const int group =
+      (int)(local * (unsigned)groups_per_iblock + blockIdx.x % (unsigned)groups_per_iblock);
   if (group * 32 >= 6 * sv.N * sv.N) return;
-  if (stage < 0) {
-    implicit_bwd_du<R>(sv, group * 32 + (int)threadIdx.x);
-    return;
-  }
-  implicit_bwd_warp<R>(sv, group, stage);
+  implicit_bwd_block<R, full>(sv, group, stage);
 }
 
 __global__ void kb_roundtrip(Batch bt) {
@@ -3462,31 +3218,43 @@ inline int check_launch() {
 
 inline unsigned nblk(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// the implicit kernel of a precision: FP32 blocks for
-// EXO_PREC_MIXED_F32_SOLVE, FP64 for EXO_PREC_MIXED and the FP64 build
-// the forward sweep, then (when some member has the full correction) the
-// back substitution
+// the implicit kernels of a precision: FP32 blocks for
+// EXO_PREC_MIXED_F32_SOLVE, FP64 for EXO_PREC_MIXED and the FP64 build; kinds:
+// the block sizes the members take (IMPL_FULL, IMPL_PARTIAL)
 template <class R>
 inline void launch_kb_implicit(unsigned blocks, int threads, int nc1, cudaStream_t st, Batch b,
-                               int stage, double dt_given, bool any_full) {
-  kb_implicit<R><<<blocks, threads, impl_smem<R>(threads, nc1), st>>>(b, stage, dt_given);
-  if constexpr (sizeof(R) == 4) {
-    if (any_full)
-      kb_implicit_bwd<R><<<blocks * (unsigned)(threads / 32), 32, impl_bwd_smem<R>(), st>>>(
-          b, stage, threads / 32);
+                               int stage, double dt_given, int kinds) {
+  const int per = threads / 32;
+  if (kinds & IMPL_FULL) {
+#if EXO_MIXED
+    if constexpr (sizeof(R) == 8) {
+      kb_implicit_fused<<<blocks, threads, fused_smem(threads, nc1), st>>>(b, stage, dt_given);
+    } else
+#endif
+    {
+      kb_implicit<R, true><<<blocks, threads, impl_smem<R, true>(threads, nc1), st>>>(b, stage,
+                                                                                     dt_given);
+      kb_implicit_bwd<R, true>
+          <<<blocks * (unsigned)per, BWD_THREADS, BwdLayout<R, 5>::bytes, st>>>(b, stage, per);
+    }
+  }
+  if (kinds & IMPL_PARTIAL) {
+    kb_implicit<R, false><<<blocks, threads, impl_smem<R, false>(threads, nc1), st>>>(b, stage,
+                                                                                     dt_given);
+    kb_implicit_bwd<R, false><<<blocks * (unsigned)per, BWD_THREADS, BwdLayout<R, 3>::bytes, st>>>(
+        b, stage, per);
   }
 }
 inline void launch_kb_implicit(int precision, unsigned blocks, int threads, int nc1,
-                               cudaStream_t st, Batch b, int stage, double dt_given,
-                               bool any_full) {
+                               cudaStream_t st, Batch b, int stage, double dt_given, int kinds) {
 #if EXO_MIXED
   if (precision == EXO_PREC_MIXED_F32_SOLVE) {
-    launch_kb_implicit<float>(blocks, threads, nc1, st, b, stage, dt_given, any_full);
+    launch_kb_implicit<float>(blocks, threads, nc1, st, b, stage, dt_given, kinds);
     return;
   }
 #endif
   (void)precision;
-  launch_kb_implicit<double>(blocks, threads, nc1, st, b, stage, dt_given, any_full);
+  launch_kb_implicit<double>(blocks, threads, nc1, st, b, stage, dt_given, kinds);
 }
 
 }  // namespace
@@ -3526,17 +3294,24 @@ unsigned x23_blocks(const DevView& v, int tile) {
 }
 
 int prepare_kernels() {
-  cudaError_t e = cudaFuncSetAttribute(kb_implicit<double>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, IMPL_SMEM_MAX);
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](const void* f, int bytes) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
 #if EXO_MIXED
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kb_implicit<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit_fused, IMPL_SMEM_MAX);
+#else
+  allow((const void*)kb_implicit<double, true>, IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit_bwd<double, true>, (int)BwdLayout<double, 5>::bytes);
 #endif
+  allow((const void*)kb_implicit<double, false>, IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit_bwd<double, false>, (int)BwdLayout<double, 3>::bytes);
 #if EXO_MIXED
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kb_implicit_bwd<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)impl_bwd_smem<float>());
+  allow((const void*)kb_implicit<float, true>, IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit<float, false>, IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit_bwd<float, true>, (int)BwdLayout<float, 5>::bytes);
+  allow((const void*)kb_implicit_bwd<float, false>, (int)BwdLayout<float, 3>::bytes);
 #endif
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(kb_flux_x1<EXO_FLUX_T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3585,7 +3360,7 @@ int launch_implicit(const DevView& v, int stage, void* stream) {
   if (v.eqn == EXO_EQN_SHALLOW_YZ || !(v.implicit_flag & 1)) return 0;
   launch_kb_implicit(v.precision, member_block_count(v, BK_IMPLICIT), v.tiles[BK_IMPLICIT], v.nc1,
                      (cudaStream_t)stream, one(v, BK_IMPLICIT), stage, 0.,
-                     (v.implicit_flag & 8) != 0);
+                     implicit_kind(v));
   return check_launch();
 }
 
@@ -3593,7 +3368,7 @@ int launch_implicit_du(const DevView& v, double dt, void* stream) {
   if (v.eqn == EXO_EQN_SHALLOW_YZ || !(v.implicit_flag & 1)) return 0;
   launch_kb_implicit(v.precision, member_block_count(v, BK_IMPLICIT), v.tiles[BK_IMPLICIT], v.nc1,
                      (cudaStream_t)stream, one(v, BK_IMPLICIT), -1, dt,
-                     (v.implicit_flag & 8) != 0);
+                     implicit_kind(v));
   return check_launch();
 }
 
@@ -3642,7 +3417,7 @@ int launch_batched_step(const BatchPlan& pl, void* stream) {
     }
     if (pl.total[BK_IMPLICIT]) {
       launch_kb_implicit(pl.precision, pl.total[BK_IMPLICIT], pl.threads[BK_IMPLICIT],
-                         pl.max_nc1, st, B(BK_IMPLICIT), s, 0., pl.any_full_correction);
+                         pl.max_nc1, st, B(BK_IMPLICIT), s, 0., pl.implicit_kinds);
       if ((rc = check_launch())) return rc;
     }
     if (s == 2) {

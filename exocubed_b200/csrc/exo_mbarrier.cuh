@@ -40,7 +40,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 __device__ __forceinline__ bool mbar_wait(unsigned long long* mb, unsigned parity) {
   const unsigned a = smem_u32(mb);
-  const unsigned long long t0 = global_ns();
+  unsigned long long t0 = 0;
   for (;;) {
     unsigned done;
     asm volatile(
@@ -50,7 +50,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* mb, unsigned parit
         : "r"(a), "r"(parity)
         : "memory");
     if (done) return true;
-    if (global_ns() - t0 > MBAR_WAIT_NS) return false;
+    // (the clock is not read where the first try succeeds)
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    else if (t - t0 > MBAR_WAIT_NS) return false;
   }
 }
 

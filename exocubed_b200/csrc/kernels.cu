@@ -23,7 +23,7 @@ namespace {
 struct HookColumnIO {
   using Real = double;
   const double* wc;
-  double* duc;
+  const double* duc;
   int nc1, L;
   double* scr0;
   size_t nslot;
@@ -31,41 +31,67 @@ struct HookColumnIO {
 #pragma unroll
     for (int n = 0; n < 5; ++n) out[n] = wc[n * nc1 + i];
   }
+  __device__ __forceinline__ size_t wstride() const { return nc1; }
+  __device__ __forceinline__ size_t dstride() const { return L; }
   __device__ __forceinline__ const double* wptr(int i, int n) const { return wc + n * nc1 + i; }
   __device__ __forceinline__ const double* duptr(int i, int n) const {
     return duc + n * L + (i - G);
   }
-  __device__ __forceinline__ double& scr(int lev, int e) const {
-    return scr0[((size_t)lev * 30 + e) * nslot];
+  __device__ __forceinline__ double* scr_level(int lev) const {
+    return scr0 + (size_t)lev * 30 * nslot;
   }
-  static constexpr bool kLoadsU = false;
-  __device__ __forceinline__ void uload(int, double*) const {}
-  __device__ __forceinline__ void ustore(int i, const double*, const double* dl) const {
-#pragma unroll
-    for (int n = 0; n < 5; ++n) duc[n * L + (i - G)] = dl[n];
-  }
+  __device__ __forceinline__ size_t scr_stride() const { return nslot; }
 };
 
+template <bool full>
 __global__ void EXO_IMPL_BOUNDS k_implicit_columns(
     int ncol, int L, const double* w, double* du, const double* colgeo, const double* x1f,
     const double* x1v, const double* dx1f, double dt, double gamma, double grav,
-    double* scratch, int full) {
+    double* scratch) {
   extern __shared__ double ism[];
-  const int col = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  int col = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int nc1 = L + 2 * G;
   const double *sx1f, *sx1v, *sdx1f;
-  stage_radial(impl_radial<double>(ism), nc1, x1f, x1v, dx1f, sx1f, sx1v, sdx1f);
-  if (col >= ncol) return;
+  stage_radial(impl_radial<double, full>(ism), nc1, x1f, x1v, dx1f, sx1f, sx1v, sdx1f);
+  if ((col & ~31) >= ncol) return;
+  // lanes past the last column repeat it: same values to the same places
+  col = min(col, ncol - 1);
   HookColumnIO io{w + (size_t)col * 5 * nc1, du + (size_t)col * 5 * L, nc1, L, scratch + col,
                   (size_t)ncol};
   const double* g4 = colgeo + (size_t)col * 4;
-  const ImplSlices<double> sl = impl_slices<double>(ism, full != 0);
-  if (full)
-    implicit_column(io, sl.sa, sl.sp, sl.ss, g4[0], g4[1], g4[2], g4[3], sx1f, sx1v, sdx1f, G,
-                    G + L - 1, dt, gamma, grav);
+  const ImplSlices<double> sl = impl_slices<double, full>(ism);
+  if constexpr (full)
+    implicit_column(io, sl.sa, sl.ss, g4[0], g4[1], g4[2], g4[3], sx1f, sx1v, sdx1f, G,
+                    G + L - 1, dt, gamma, grav, sl.wt);
   else
-    implicit_column_partial(io, sl.sa, sl.sp, sl.ss, g4[0], g4[1], g4[2], g4[3], sx1f, sx1v,
-                            sdx1f, G, G + L - 1, dt, gamma, grav);
+    implicit_column_partial(io, sl.sa, sl.ss, g4[0], g4[1], g4[2], g4[3], sx1f, sx1v,
+                            sdx1f, G, G + L - 1, dt, gamma, grav, sl.wt);
+}
+
+// the back substitution of 32 columns, the corrected update into du
+template <bool full>
+__global__ void __launch_bounds__(BWD_THREADS) k_implicit_columns_bwd(int ncol, int L, double* du,
+                                                                      const double* scratch,
+                                                                      int* timeout) {
+  extern __shared__ __align__(128) unsigned char bws[];
+  __shared__ long long s_off[32];
+  const int col0 = (int)blockIdx.x * 32;
+  if (threadIdx.x < 32)
+    s_off[threadIdx.x] = (long long)min(col0 + (int)threadIdx.x, ncol - 1) * 5 * L;
+  __syncthreads();
+  BwdGroup<double> g;
+  g.scr = scratch + col0;
+  g.lstride = (size_t)30 * ncol;
+  g.estride = ncol;
+  g.x = du;
+  g.vs = L;
+  g.off = s_off;
+  g.ncols = min(32, ncol - col0);
+  g.L = L;
+  g.stage = -1;
+  g.Rd = g.gamma = 0.;
+  g.timeout = timeout;
+  implicit_bwd_group<double, full ? 5 : 3, false>(g, bws);
 }
 
 __global__ void k_riemann_rows(int rsolver, int eqn, int ivx, int n, double gamma,
@@ -203,21 +229,40 @@ size_t decomposition_refs_doubles(const DevView& v) {
 
 // the column kernel's shared memory grows with L (the radial tables); the
 // attribute lets a launch go past the 48 KB default
-static cudaError_t allow_column_smem() {
-  return cudaFuncSetAttribute(fp64::k_implicit_columns,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, fp64::IMPL_SMEM_MAX);
+template <bool full>
+static cudaError_t column_kernel(int ncol, int L, const double* w, double* du,
+                                 const double* colgeo, const double* x1f, const double* x1v,
+                                 const double* dx1f, double dt, double gamma, double grav,
+                                 double* scratch, void* stream) {
+  cudaError_t e = cudaFuncSetAttribute(fp64::k_implicit_columns<full>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       fp64::IMPL_SMEM_MAX);
+  if (e != cudaSuccess) return e;
+  fp64::k_implicit_columns<full><<<fp64::nblk(ncol, fp64::IMPL_THREADS), fp64::IMPL_THREADS,
+                                   fp64::impl_smem<double, full>(fp64::IMPL_THREADS, L + 2 * G),
+                                   (cudaStream_t)stream>>>(ncol, L, w, du, colgeo, x1f, x1v, dx1f,
+                                                           dt, gamma, grav, scratch);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  constexpr size_t smem = fp64::BwdLayout<double, full ? 5 : 3>::bytes;
+  e = cudaFuncSetAttribute(fp64::k_implicit_columns_bwd<full>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // (its waits are on plain asynchronous copies: no flag needed)
+  fp64::k_implicit_columns_bwd<full><<<fp64::nblk(ncol, 32), fp64::BWD_THREADS, smem,
+                                       (cudaStream_t)stream>>>(ncol, L, du, scratch, nullptr);
+  return cudaGetLastError();
 }
 
 int launch_implicit_columns(int ncol, int L, const double* w, double* du, const double* colgeo,
                             const double* x1f, const double* x1v, const double* dx1f, double dt,
                             double gamma, double grav, double* scratch, void* stream, int full) {
   if (ncol <= 0) return 0;
-  if (allow_column_smem() != cudaSuccess) return EXO_ERR_CUDA;
-  fp64::k_implicit_columns<<<fp64::nblk(ncol, fp64::IMPL_THREADS), fp64::IMPL_THREADS,
-                              fp64::impl_smem<double>(fp64::IMPL_THREADS, L + 2 * G),
-                              (cudaStream_t)stream>>>(
-      ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt, gamma, grav, scratch, full);
-  return fp64::check_launch();
+  const cudaError_t e = full ? column_kernel<true>(ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt,
+                                                   gamma, grav, scratch, stream)
+                             : column_kernel<false>(ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt,
+                                                    gamma, grav, scratch, stream);
+  return e == cudaSuccess ? 0 : EXO_ERR_CUDA;
 }
 
 // ---------------------------------------------------------------------------
@@ -270,16 +315,7 @@ int launch_implicit_columns_noalloc(int ncol, int L, const double* w, double* du
     scratch = g_noalloc_addr[dev];
   }
   if (ncol <= 0) return 0;
-  e = allow_column_smem();
-  if (e != cudaSuccess) {
-    *err = std::string("cudaFuncSetAttribute(k_implicit_columns): ") + cudaGetErrorString(e);
-    return EXO_ERR_CUDA;
-  }
-  fp64::k_implicit_columns<<<fp64::nblk(ncol, fp64::IMPL_THREADS), fp64::IMPL_THREADS,
-                              fp64::impl_smem<double>(fp64::IMPL_THREADS, L + 2 * G),
-                              (cudaStream_t)stream>>>(
-      ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt, gamma, grav, scratch, 1);
-  e = cudaGetLastError();
+  e = column_kernel<true>(ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt, gamma, grav, scratch, stream);
   if (e != cudaSuccess) {
     *err = std::string("k_implicit_columns: ") + cudaGetErrorString(e);
     return EXO_ERR_CUDA;

@@ -46,3 +46,8 @@ def test_oracle_under_sanitizers(tmp_path):
 def test_fastdiv_exact_under_sanitizers(tmp_path):
     out = _build_and_run(tmp_path, "fastdiv", ["tests/sanitize/fastdiv_driver.cpp"])
     assert "fastdiv: ok" in out
+
+
+def test_shared_division_is_ieee_under_sanitizers(tmp_path):
+    out = _build_and_run(tmp_path, "shareddiv", ["tests/sanitize/shareddiv_driver.cpp"])
+    assert "shareddiv: ok" in out
