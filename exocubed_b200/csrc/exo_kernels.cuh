@@ -117,10 +117,13 @@ __device__ __forceinline__ double rk_beta(int stage) {
 }
 
 __device__ __forceinline__ size_t idx(const DevView& v, int p, int n, int k, int j, int i) {
-  return ((((size_t)p * v.nv + n) * v.nc3 + k) * v.nc2 + j) * v.nc1 + i;
+  return (size_t)(unsigned)(((p * v.nv + n) * v.nc3 + k) * v.nc2 + j) * (unsigned)v.nc1 +
+         (unsigned)i;
 }
 __device__ __forceinline__ double geo(const DevView& v, int f, int p, int k, int j) {
-  return v.geo[(((size_t)f * 6 + p) * v.nc3 + k) * v.nc2 + j];
+  // (fits 32 bits: NGEO2D * 6 * nc3 * nc2 passes 2^32 beyond nc2 = 4800,
+  // whose state does not fit a GPU)
+  return v.geo[(unsigned)(((f * 6 + p) * v.nc3 + k) * v.nc2 + j)];
 }
 
 // face-flux and primitive arrays in the type the flux kernels work in
@@ -554,19 +557,19 @@ __device__ __forceinline__ void riemann(int rsolver, double gamma, int ivx, cons
 // src is the source panel's (nv, nc3, nc2, nc1) array.
 __device__ __forceinline__ void ghost_interp(const DevView& v, const GhostEntry& e,
                                              const double* src, int i, double* c) {
-  auto S = [&](int n, int k, int j) {
-    return src[(((size_t)n * v.nc3 + k) * v.nc2 + j) * v.nc1 + i];
-  };
+  const size_t vs = v.cells;
+  const double* s0 = src + (size_t)(unsigned)(e.k0 * v.nc2 + e.j0) * (unsigned)v.nc1 + i;
+  const double* s1 = src + (size_t)(unsigned)(e.k1 * v.nc2 + e.j1) * (unsigned)v.nc1 + i;
   #pragma unroll
   for (int n = 0; n < 5; ++n) {
     if (n >= v.nv) break;
     if (n == IVY || n == IVZ) continue;
-    double v1 = S(n, e.k0, e.j0);
-    double v2 = S(n, e.k1, e.j1);
+    double v1 = s0[n * vs];
+    double v2 = s1[n * vs];
     c[n] = (e.A * v1 + e.B * v2) / e.C;
   }
-  double v1y = S(IVY, e.k0, e.j0), v1z = S(IVZ, e.k0, e.j0);
-  double v2y = S(IVY, e.k1, e.j1), v2z = S(IVZ, e.k1, e.j1);
+  double v1y = s0[IVY * vs], v1z = s0[IVZ * vs];
+  double v2y = s1[IVY * vs], v2z = s1[IVZ * vs];
   double vy = (e.A * v1y + e.B * v2y) / e.C;
   double vz = (e.A * v1z + e.B * v2z) / e.C;
   double sth = e.ss, cth = e.cs;
@@ -588,10 +591,12 @@ __device__ __forceinline__ void ghost_interp(const DevView& v, const GhostEntry&
 __device__ __forceinline__ void load_cons(const DevView& v, int p, int k, int j, int i,
                                           bool interior, double* c) {
   if (interior) {
+    const double* u = v.u + idx(v, p, 0, k, j, i);
+    const size_t vs = v.cells;
     #pragma unroll
     for (int n = 0; n < 5; ++n) {
       if (n >= v.nv) break;
-      c[n] = v.u[idx(v, p, n, k, j, i)];
+      c[n] = u[n * vs];
     }
     return;
   }
@@ -675,16 +680,19 @@ __device__ __forceinline__ unsigned long long prim_ghost_cell(const DevView& v, 
   double cth = geo(v, GCOSC, p, k, j);
   int bad = cons_to_prim(v, c, w, cth);
   if (mirror) w[IVX] = -w[IVX];
+  const size_t at = idx(v, p, 0, k, j, i), vs = v.cells;
+  double* const wo = v.w + at;
   #pragma unroll
   for (int n = 0; n < 5; ++n) {
     if (n >= v.nv) break;
-    v.w[idx(v, p, n, k, j, i)] = w[n];
+    wo[n * vs] = w[n];
   }
 #if EXO_MIXED
+  float* const fo = v.w32 + at;
   #pragma unroll
   for (int n = 0; n < 5; ++n) {
     if (n >= v.nv) break;
-    v.w32[idx(v, p, n, k, j, i)] = (float)w[n];
+    fo[n * vs] = (float)w[n];
   }
 #endif
   if (!(kin && jin) || mirror) return none;
@@ -1296,20 +1304,29 @@ __device__ __forceinline__ void cp_async_zfill(void* smem_dst, const void* gsrc,
 
 // The x2/x3 faces of one line (32 radial indices of one row of one panel
 // and direction) chunk by chunk, with the same phases, values and
-// operations per face as the per-face form.  Cell c of the line sits in ring
-// slot (c - c0 + 3) mod XR; the copies of chunk q + 1's new cells are in
-// flight while chunk q is finished.  Slots written for chunk q + 1 held
-// cells at least XR = 2 CF + 5 below them, which chunk q no longer reads;
-// the copies for chunk q + 2 start after the barrier that ends chunk q's
-// reconstruction.
+// operations per face as the per-face form.  Cell m of the line (m = 0 three
+// cells below the first face) sits in ring slot m mod XR; the copies of chunk
+// q + 1's new cells are in flight while chunk q is finished.  Slots written
+// for chunk q + 1 held cells at least XR = 2 CF + 5 below them, which chunk q
+// no longer reads; the copies for chunk q + 2 start after the barrier that
+// ends chunk q's reconstruction.  The ring's position, the line's pointers
+// and strides are carried along: recomputed per row of copies and per face,
+// with divisions by the chunk's runtime length, they were 38 % of the mixed
+// build's instructions.
 template <class T>
-__device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk) {
-  constexpr int CF = x23_chunk<T>();
-  constexpr int NC = CF + 1;
-  constexpr int XR = 2 * CF + 5;
-  __shared__ __align__(16) T ring[5][XR][32];
-  __shared__ T srec[2][5][NC][32];
-  const int N = v.N, L = v.L, nv = v.nv;
+struct X23Shared {
+  static constexpr int CF = x23_chunk<T>(), NC = CF + 1, XR = 2 * CF + 5;
+  T ring[5][XR][32];
+  T srec[2][5][NC][32];
+};
+template <class T, int NV>
+__device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X23Shared<T>& sm) {
+  constexpr int CF = X23Shared<T>::CF;
+  constexpr int NC = X23Shared<T>::NC;
+  constexpr int XR = X23Shared<T>::XR;
+  auto& ring = sm.ring;
+  auto& srec = sm.srec;
+  const int N = v.N, L = v.L;
   const unsigned nit = (unsigned)((L + 31) / 32);
   unsigned r = blk;
   const int itile = (int)(r % nit);
@@ -1322,93 +1339,107 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk) {
   constexpr int NW = X23_THREADS / 32;
   const int il = itile * 32 + lane;
   const bool active = il < L;
-  const int i = v.is + il;
+  const int i = v.is + (active ? il : 0);
   const size_t vs = v.cells;
-  const long s = dir == 1 ? (long)v.nc1 : (long)v.nc1 * v.nc2;
-  const size_t base = dir == 1 ? idx(v, p, 0, v.ks + a, 0, active ? i : v.is)
-                               : idx(v, p, 0, 0, v.js + a, active ? i : v.is);
-  const T* __restrict__ W = prim_array<T>(v) + base;
-  const int c0 = dir == 1 ? v.js : v.ks, c1 = dir == 1 ? v.je : v.ke;
+  const size_t s = dir == 1 ? (size_t)v.nc1 : (size_t)v.nc1 * v.nc2;
+  // the first face's place in the state and flux arrays
+  const size_t base = dir == 1 ? idx(v, p, 0, v.ks + a, v.js, i) : idx(v, p, 0, v.ks, v.js + a, i);
+  const T* const W = prim_array<T>(v) + base - 3 * s;  // cell 0
+  T* const F = flux_array<T>(v, dir) + base;           // face 0
   const int nch = (N + 1 + CF - 1) / CF;
-  // copies of cells [from, to] (line indices), rows (variable, cell) over the warps
-  auto issue = [&](int from, int to) {
-    const int nc = to - from + 1;
-    for (int row = warp; row < nc * nv; row += NW) {
-      const int n = row / nc, c = from + row % nc;
-      int slot = c - c0 + 3;
-      slot -= (slot >= XR) ? XR * (slot / XR) : 0;
-      const bool ok = active && c <= c1 + 3;
-      cp_async_zfill<sizeof(T)>(&ring[n][slot][lane], W + n * vs + (long)(ok ? c : c0) * s,
-                                ok ? (int)sizeof(T) : 0);
+  const int rsolver = v.rsolver;
+  const double gamma = v.gamma;
+  // copies of the cells [m0, m0 + n), the first of them in slot slot0
+  auto issue = [&](int m0, int n, int slot0) {
+#pragma unroll 1
+    for (int c = warp; c < n; c += NW) {
+      const int m = m0 + c;
+      int slot = slot0 + c;
+      slot -= (slot >= XR) ? XR : 0;
+      const bool ok = active && m < N + 6;
+      const T* src = W + (size_t)(ok ? m : 3) * s;
+      T* dst = &ring[0][slot][lane];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        cp_async_zfill<sizeof(T)>(dst + q * (XR * 32), src, ok ? (int)sizeof(T) : 0);
+        src += vs;
+      }
     }
     cp_async_commit();
   };
-  issue(c0 - 3, c0 + CF + 1);
-  T* F = flux_array<T>(v, dir);
+  issue(0, CF + 5, 0);
+  int islot = CF + 5, rslot = 0;  // slots of the next cell to copy and of cell q CF
   for (int q = 0; q < nch; ++q) {
-    const int cb = c0 + q * CF;
     if (q + 1 < nch) {
-      issue(cb + CF + 2, cb + 2 * CF + 1);
+      issue(q * CF + CF + 5, CF, islot);
+      islot += CF;
+      islot -= (islot >= XR) ? XR : 0;
       cp_async_wait_one();
     } else {
       cp_async_wait_all();
     }
     __syncthreads();
-    // 1. both face values of the cells cb-1 .. cb+CF-1
+    // 1. both face values of the cells below and above the chunk's faces
+#pragma unroll 1
     for (int mc = warp; mc < NC; mc += NW) {
-      int s0 = cb - 1 - c0 + 3 + mc - 2;  // slot of cell cb-1+mc-2
-      s0 -= (s0 >= XR) ? XR * (s0 / XR) : 0;
-      int sl[5];
+      const T* st[5];  // the cell's stencil
 #pragma unroll
-      for (int m = 0; m < 5; ++m) sl[m] = (s0 + m >= XR) ? s0 + m - XR : s0 + m;
+      for (int m = 0; m < 5; ++m) {
+        int sl = rslot + mc + m;
+        sl -= (sl >= XR) ? XR : 0;
+        st[m] = &ring[0][sl][lane];
+      }
+      T* const rec = &srec[0][0][mc][lane];
 #pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        if (n >= nv) break;
-        const T q0 = ring[n][sl[0]][lane], q1 = ring[n][sl[1]][lane], q2 = ring[n][sl[2]][lane];
-        const T q3 = ring[n][sl[3]][lane], q4 = ring[n][sl[4]][lane];
+      for (int n = 0; n < NV; ++n) {
+        const T q0 = st[0][n * (XR * 32)], q1 = st[1][n * (XR * 32)], q2 = st[2][n * (XR * 32)];
+        const T q3 = st[3][n * (XR * 32)], q4 = st[4][n * (XR * 32)];
 #if EXO_X23_SHARED_BETA
         const WenoCell<T> wc = weno_cell<T>(q0, q1, q2, q3, q4);
-        srec[0][n][mc][lane] = weno_right<T>(wc, q0, q1, q2, q3, q4);
-        srec[1][n][mc][lane] = weno_left<T>(wc, q0, q1, q2, q3, q4);
+        rec[n * (NC * 32)] = weno_right<T>(wc, q0, q1, q2, q3, q4);
+        rec[(5 + n) * (NC * 32)] = weno_left<T>(wc, q0, q1, q2, q3, q4);
 #else
-        srec[0][n][mc][lane] = weno5<T>(q4, q3, q2, q1, q0);
-        srec[1][n][mc][lane] = weno5<T>(q0, q1, q2, q3, q4);
+        rec[n * (NC * 32)] = weno5<T>(q4, q3, q2, q1, q0);
+        rec[(5 + n) * (NC * 32)] = weno5<T>(q0, q1, q2, q3, q4);
 #endif
       }
     }
+    rslot += CF;
+    rslot -= (rslot >= XR) ? XR : 0;
     __syncthreads();
     if (!active) continue;
-    // 2. the faces cb .. cb+CF-1 (up to c1+1)
+    // 2. the faces q CF .. q CF + CF - 1 (up to N)
+#pragma unroll 1
     for (int mf = warp; mf < CF; mf += NW) {
-      const int c = cb + mf;
-      if (c > c1 + 1) break;
+      const int f = q * CF + mf;
+      if (f > N) break;
       T wl[5], wr[5], fx[5] = {T(0.), T(0.), T(0.), T(0.), T(0.)};
+      const T* const rec = &srec[0][0][mf][lane];
 #pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        if (n >= nv) break;
-        wl[n] = srec[0][n][mf][lane];
-        wr[n] = srec[1][n][mf + 1][lane];
+      for (int n = 0; n < NV; ++n) {
+        wl[n] = rec[n * (NC * 32)];
+        wr[n] = rec[(5 + n) * (NC * 32) + 32];
       }
-      const int k = dir == 1 ? v.ks + a : c;
-      const int j = dir == 1 ? c : v.js + a;
       if (dir == 1) {
-        if (c == c0) edge_outer_state<T>(v, p, UP, a, i, wl);
-        else if (c == c1 + 1) edge_outer_state<T>(v, p, DOWN, a, i, wr);
+        if (f == 0) edge_outer_state<T>(v, p, UP, a, i, wl);
+        else if (f == N) edge_outer_state<T>(v, p, DOWN, a, i, wr);
+        const int k = v.ks + a, j = v.js + f;
         FaceGeo<T> fg{T(geo(v, GCOSF2, p, k, j)), T(geo(v, GSINF2, p, k, j)),
                       T(geo(v, GCTHP2, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-        riemann<T>(v.rsolver, v.gamma, IVY, fg, wl, wr, fx);
+        riemann<T>(rsolver, gamma, IVY, fg, wl, wr, fx);
       } else {
-        if (c == c0) edge_outer_state<T>(v, p, LEFT, a, i, wl);
-        else if (c == c1 + 1) edge_outer_state<T>(v, p, RIGHT, a, i, wr);
+        if (f == 0) edge_outer_state<T>(v, p, LEFT, a, i, wl);
+        else if (f == N) edge_outer_state<T>(v, p, RIGHT, a, i, wr);
+        const int k = v.ks + f, j = v.js + a;
         FaceGeo<T> fg{T(geo(v, GCOSF3, p, k, j)), T(geo(v, GSINF3, p, k, j)),
                       T(geo(v, GCTHP3, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-        riemann<T>(v.rsolver, v.gamma, IVZ, fg, wl, wr, fx);
+        riemann<T>(rsolver, gamma, IVZ, fg, wl, wr, fx);
       }
-      const size_t f0 = idx(v, p, 0, k, j, i);
+      T* out = F + (size_t)f * s;
 #pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        if (n >= nv) break;
-        F[f0 + n * vs] = fx[n];
+      for (int n = 0; n < NV; ++n) {
+        *out = fx[n];
+        out += vs;
       }
     }
   }
@@ -1417,8 +1448,10 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk) {
 template <class T>
 __device__ __forceinline__ void flux_x23_block(const DevView& v, unsigned blk) {
   if constexpr (EXO_X23_TILES) {
-    if (x23_uses_lines(v.L)) flux_x23_pipe<T>(v, blk);
-    else flux_x23_faces<T>(v, blk);
+    __shared__ __align__(16) X23Shared<T> sm;
+    if (!x23_uses_lines(v.L)) flux_x23_faces<T>(v, blk);
+    else if (v.nv == 5) flux_x23_pipe<T, 5>(v, blk, sm);
+    else flux_x23_pipe<T, 4>(v, blk, sm);
   } else if constexpr (EXO_X23_LINES) {
     flux_x23_lines<T>(v, blk);
   } else {
