@@ -145,10 +145,57 @@ template <> __device__ __forceinline__ const float* prim_array<float>(const DevV
   return v.w32;
 }
 
+#if !EXO_MIXED
+// a / b without a division's range checks, for b normal in 2^-400..2^400 and
+// a quotient that is normal or zero: 1/b by two Newton steps from PTX's
+// approximation, q = a r, and one remainder step (Markstein, IBM J. Res. Dev.
+// 34, 1990).  The sum it rounds is within 2^-52 of an ulp of a/b, so the
+// result is the IEEE quotient unless a/b lies that close to the middle of two
+// doubles.
+__device__ __forceinline__ double div_nr(double a, double b) {
+  const double r = rcp_nr(b);
+  const double q = a * r;
+  return fma(fma(-b, q, a), r, q);
+}
+// WENO5's constants as operands from the constant bank (64-bit immediates
+// take two instructions each)
+__constant__ double kWeno[12] = {1.0 / 3.0, 7.0 / 6.0, 11.0 / 6.0, -1.0 / 6.0, 5.0 / 6.0,
+                                 1.0 / 6.0, 13. / 12., 0.25, 1.0e-7, 0.1, 0.6, 0.3};
+#endif
 // interp_weno5(phip2, phip1, phi, phim1, phim2): the face value between the
 // 2nd and 3rd argument (Jiang & Shu 1996; orientation of tests/test_weno.cpp)
 template <class T>
 __device__ __forceinline__ T weno5(T phip2, T phip1, T phi, T phim1, T phim2) {
+#if !EXO_MIXED
+  if constexpr (sizeof(T) == 8) {
+    const double eps = kWeno[8];
+    const double p0 = kWeno[0] * phim2 - kWeno[1] * phim1 + kWeno[2] * phi;
+    const double p1 = kWeno[3] * phim1 + kWeno[4] * phi + kWeno[0] * phip1;
+    const double p2 = kWeno[0] * phi + kWeno[4] * phip1 - kWeno[5] * phip2;
+    const double b0 = kWeno[6] * sqr(phim2 - 2. * phim1 + phi) +
+                      kWeno[7] * sqr(phim2 - 4. * phim1 + 3. * phi);
+    const double b1 = kWeno[6] * sqr(phim1 - 2. * phi + phip1) + kWeno[7] * sqr(phim1 - phip1);
+    const double b2 = kWeno[6] * sqr(phi - 2. * phip1 + phip2) +
+                      kWeno[7] * sqr(3. * phi - 4. * phip1 + phip2);
+    const double d0 = (b0 + eps) * (b0 + eps), d1 = (b1 + eps) * (b1 + eps),
+                 d2 = (b2 + eps) * (b2 + eps);
+    // every weight's denominator below 2^400 (they are above eps^2): the
+    // divisions need no further checks.  NaN and infinity fail this.
+    const unsigned top = max(max((unsigned)__double2hiint(d0), (unsigned)__double2hiint(d1)),
+                             (unsigned)__double2hiint(d2));
+    double a0, a1, a2;
+    if (top < ((1023u + 400u) << 20)) {
+      a0 = div_nr(kWeno[9], d0);
+      a1 = div_nr(kWeno[10], d1);
+      a2 = div_nr(kWeno[11], d2);
+      return div_nr(a0 * p0 + a1 * p1 + a2 * p2, a0 + a1 + a2);
+    }
+    a0 = kWeno[9] / d0;
+    a1 = kWeno[10] / d1;
+    a2 = kWeno[11] / d2;
+    return (a0 * p0 + a1 * p1 + a2 * p2) / (a0 + a1 + a2);
+  }
+#endif
   const T eps = T(WENO_EPS);
   T p0 = T(1.0 / 3.0) * phim2 - T(7.0 / 6.0) * phim1 + T(11.0 / 6.0) * phi;
   T p1 = T(-1.0 / 6.0) * phim1 + T(5.0 / 6.0) * phi + T(1.0 / 3.0) * phip1;
