@@ -25,7 +25,7 @@ from . import _native as nat
 # without the implicit solver) is timed inside EXO_K_UPDATE and follows it
 CANDIDATES = {
     nat.EXO_K_FLUX_X1: (1, 2, 3, 4),     # radial columns per block
-    nat.EXO_K_FLUX_X23: (128,),          # both x2/x3 forms run 128 threads a block
+    nat.EXO_K_FLUX_X23: (128,),          # the x2/x3 kernel runs 128 threads a block
     nat.EXO_K_UPDATE: (32, 64, 128, 256),
     nat.EXO_K_IMPLICIT: (32, 64, 128),
     nat.EXO_K_PRIM_GHOST: (64, 128, 256, 512),

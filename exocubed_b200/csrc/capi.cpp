@@ -311,6 +311,7 @@ int view_allocate(const exo_config& cfg, const HostTables& t, DevView& v,
   v.implicit_flag = shallow ? 0 : cfg.implicit_flag;
   v.coriolis = cfg.coriolis;
   v.precision = cfg.precision;
+  v.x23 = mixed_build(v.precision) ? mixed::x23_split(v.N, v.L) : fp64::x23_split(v.N, v.L);
   v.forcing = shallow ? EXO_FORCING_NONE : cfg.forcing;
   if (v.forcing == EXO_FORCING_HS94) {
     // Mesh::InitUserMeshData (hs94.cpp:212-243): cp from gamma, rates per day
@@ -455,9 +456,7 @@ void member_blocks(const DevView& v, const int* t, unsigned b[BK_COUNT]) {
   bool implicit = !shallow && (v.implicit_flag & 1);
   auto nb = [](size_t n, int th) { return (unsigned)((n + th - 1) / th); };
   b[BK_X1] = shallow ? 0u : nb((size_t)6 * v.N * v.N, t[BK_X1]);  // t[BK_X1] columns per block
-  // tiles of faces, or one thread per line of faces or per face, as the build chose
-  b[BK_X23] = mixed_build(v.precision) ? mixed::x23_blocks(v, t[BK_X23])
-                                        : fp64::x23_blocks(v, t[BK_X23]);
+  b[BK_X23] = 12u * v.x23.groups * v.x23.segments;
   b[BK_UPDATE] = nb((size_t)6 * v.N * v.N * v.L, t[BK_UPDATE]);
   b[BK_IMPLICIT] = implicit ? nb((size_t)6 * v.N * v.N, t[BK_IMPLICIT]) : 0u;  // thread per column
   b[BK_PRIM] = nb((size_t)6 * v.cells, t[BK_PRIM]);

@@ -154,11 +154,18 @@ inline FastDiv make_fastdiv(unsigned d) {
   return f;
 }
 
+// How the x2/x3 fluxes are cut: groups of 32 lines per panel and direction,
+// chunks of faces per segment of a line, segments.
+struct X23Split {
+  unsigned groups, chunks, segments;
+};
+
 // Sizes, parameters and device pointers of one atmosphere; passed by value
 // to every kernel.
 struct alignas(16) DevView {
   int N, L, nv, nc1, nc2, nc3;
   FastDiv div_L, div_N, div_nc1, div_nc2, div_nc3;  // divisions by L, N, nc1, nc2, nc3
+  X23Split x23;
   int is, ie, js, je, ks, ke;
   int eqn, rsolver, implicit_flag, coriolis;
   int precision, forcing;
@@ -290,7 +297,7 @@ int view_refresh_self(DevView& v, void* stream, std::string* err);
   int launch_batched_step(const BatchPlan& plan, void* stream);                     \
   int prepare_kernels();                                                            \
   int launch_reciprocal(int n, const double* x, double* out, void* stream);         \
-  unsigned x23_blocks(const DevView& v, int tile);
+  X23Split x23_split(int N, int L);
 namespace fp64 { EXO_DECLARE_STEP_LAUNCHERS }
 namespace mixed { EXO_DECLARE_STEP_LAUNCHERS }
 #undef EXO_DECLARE_STEP_LAUNCHERS

@@ -35,16 +35,6 @@
 #include "exo_internal.h"
 #include "exo_mbarrier.cuh"
 
-// x2/x3 fluxes: EXO_X23_TILES 1 = a block per line of faces, cells staged
-// through shared memory (flux_x23_pipe), and one thread per face for grids
-// of few levels; otherwise EXO_X23_LINES 1 = one thread per line of faces
-// (sliding stencil window), 0 = one thread per face
-#ifndef EXO_X23_TILES
-#define EXO_X23_TILES 1
-#endif
-#ifndef EXO_X23_LINES
-#define EXO_X23_LINES EXO_MIXED
-#endif
 // 1: the x1 (radial) Riemann flux, its storage and its divergence stay FP64
 // in the mixed build (the reconstruction of the perturbations stays FP32):
 // the radial momentum flux carries the full hydrostatic pressure, whose
@@ -53,13 +43,9 @@
 #ifndef EXO_X1_FLUX64
 #define EXO_X1_FLUX64 EXO_MIXED
 #endif
-// 1: the sliding window computes each cell's WENO smoothness indicators once
-// for both of its faces (mixed build; the FP64 build keeps weno5's order)
-#ifndef EXO_X23_SHARED_BETA
-#define EXO_X23_SHARED_BETA EXO_MIXED
-#endif
-// 1: the same in the x1 kernel, whose cells' face values go through shared
-// memory (mixed build)
+// 1: the x1 kernel, whose cells' face values go through shared memory,
+// computes each cell's WENO smoothness indicators once for both of its faces
+// (mixed build; the FP64 build keeps weno5's order)
 #ifndef EXO_X1_SHARED_BETA
 #define EXO_X1_SHARED_BETA EXO_MIXED
 #endif
@@ -1115,165 +1101,6 @@ __device__ __forceinline__ void edge_outer_state(const DevView& v, int p, int si
   st[IVZ] = T(e.q[2]) * U + T(e.q[3]) * V;
 }
 
-// One thread per face: grids whose level count leaves too many of a line's
-// lanes idle (x23_uses_lines).
-template <class T>
-__device__ __forceinline__ void flux_x23_faces(const DevView& v, unsigned blk) {
-  unsigned tid = blk * blockDim.x + threadIdx.x;
-  unsigned nface = 6u * v.N * (v.N + 1) * v.L;  // per direction
-  if (tid >= 2 * nface) return;
-  int dir = tid < nface ? 1 : 2;
-  unsigned r = dir == 1 ? tid : tid - nface;
-  unsigned L = v.L, N = v.N;
-  int i = v.is + (int)(r % L);
-  r /= L;
-  int k, j;
-  int p;
-  if (dir == 1) {  // x2 faces: j in [js, je+1], k in [ks, ke]
-    j = v.js + (int)(r % (N + 1));
-    r /= (N + 1);
-    k = v.ks + (int)(r % N);
-    p = (int)(r / N);
-  } else {  // x3 faces: j in [js, je], k in [ks, ke+1]
-    j = v.js + (int)(r % N);
-    r /= N;
-    k = v.ks + (int)(r % (N + 1));
-    p = (int)(r / (N + 1));
-  }
-  T wl[5], wr[5], fx[5] = {T(0.), T(0.), T(0.), T(0.), T(0.)};
-  long s2 = v.nc1, s3 = (long)v.nc1 * v.nc2;
-  const T* W = prim_array<T>(v);
-  FaceGeo<T> fg;
-  int ivx;
-  if (dir == 1) {
-    #pragma unroll
-    for (int n = 0; n < 5; ++n) {
-      if (n >= v.nv) break;
-      const T* q = W + idx(v, p, n, k, 0, i);
-      wl[n] = weno_r<T>(q, s2, j - 1);
-      wr[n] = weno_l<T>(q, s2, j);
-    }
-    if (j == v.js) edge_outer_state<T>(v, p, UP, k - v.ks, i, wl);
-    else if (j == v.je + 1) edge_outer_state<T>(v, p, DOWN, k - v.ks, i, wr);
-    fg = FaceGeo<T>{T(geo(v, GCOSF2, p, k, j)), T(geo(v, GSINF2, p, k, j)),
-                    T(geo(v, GCTHP2, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-    ivx = IVY;
-  } else {
-    #pragma unroll
-    for (int n = 0; n < 5; ++n) {
-      if (n >= v.nv) break;
-      const T* q = W + idx(v, p, n, 0, j, i);
-      wl[n] = weno_r<T>(q, s3, k - 1);
-      wr[n] = weno_l<T>(q, s3, k);
-    }
-    if (k == v.ks) edge_outer_state<T>(v, p, LEFT, j - v.js, i, wl);
-    else if (k == v.ke + 1) edge_outer_state<T>(v, p, RIGHT, j - v.js, i, wr);
-    fg = FaceGeo<T>{T(geo(v, GCOSF3, p, k, j)), T(geo(v, GSINF3, p, k, j)),
-                    T(geo(v, GCTHP3, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-    ivx = IVZ;
-  }
-  // the velocity index as a literal, so the solvers index registers only
-  if (ivx == IVY) riemann<T>(v.rsolver, v.gamma, IVY, fg, wl, wr, fx);
-  else riemann<T>(v.rsolver, v.gamma, IVZ, fg, wl, wr, fx);
-  T* F = flux_array<T>(v, dir);
-  #pragma unroll
-  for (int n = 0; n < 5; ++n) {
-    if (n >= v.nv) break;
-    F[idx(v, p, n, k, j, i)] = fx[n];
-  }
-}
-
-
-// One thread per line of faces (the mixed build): for x2 faces the line (p, k, i) runs over
-// j = js .. je+1, for x3 faces the line (p, j, i) over k = ks .. ke+1.  The
-// six cells of the face's WENO5 stencils slide along the line in
-// registers, so every cell is read once per line instead of six times; each
-// face's reconstruction, edge replacement and Riemann solve are those of a
-// face on its own (same values, same operations).
-template <class T>
-__device__ __forceinline__ void flux_x23_lines(const DevView& v, unsigned blk) {
-  const unsigned tid = blk * blockDim.x + threadIdx.x;
-  const unsigned L = v.L, N = v.N;
-  const unsigned nline = 6u * N * L;  // per direction
-  if (tid >= 2 * nline) return;
-  const int dir = tid < nline ? 1 : 2;
-  unsigned r = dir == 1 ? tid : tid - nline;
-  const unsigned rl = v.div_L(r);
-  const int i = v.is + (int)(r - rl * L);
-  const unsigned rn = v.div_N(rl);
-  const int a = (int)(rl - rn * N);  // position across the line: k - ks (x2) or j - js (x3)
-  const int p = (int)rn;
-  const int nv = v.nv;
-  const size_t vs = v.cells;
-  const long s = dir == 1 ? (long)v.nc1 : (long)v.nc1 * v.nc2;  // stride along the line
-  const size_t base = dir == 1 ? idx(v, p, 0, v.ks + a, 0, i) : idx(v, p, 0, 0, v.js + a, i);
-  const T* __restrict__ W = prim_array<T>(v) + base;
-  const int c0 = dir == 1 ? v.js : v.ks, c1 = dir == 1 ? v.je : v.ke;
-  T* F = flux_array<T>(v, dir);
-  // window q[n][m] = cell (c - 3 + m) of the line for face c (cells c-1 | c)
-  T q[5][6];
-#pragma unroll
-  for (int n = 0; n < 5; ++n) {
-    if (n >= nv) break;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) q[n][m] = T(__ldg(W + n * vs + (long)(c0 - 3 + m) * s));
-  }
-#if EXO_X23_SHARED_BETA
-  WenoCell<T> wprev[5];  // indicators of cell c - 1
-#pragma unroll
-  for (int n = 0; n < 5; ++n) {
-    if (n >= nv) break;
-    wprev[n] = weno_cell<T>(q[n][0], q[n][1], q[n][2], q[n][3], q[n][4]);
-  }
-#endif
-  for (int c = c0; c <= c1 + 1; ++c) {
-    T wl[5], wr[5], fx[5] = {T(0.), T(0.), T(0.), T(0.), T(0.)};
-#pragma unroll
-    for (int n = 0; n < 5; ++n) {
-      if (n >= nv) break;
-#if EXO_X23_SHARED_BETA
-      const WenoCell<T> wcur = weno_cell<T>(q[n][1], q[n][2], q[n][3], q[n][4], q[n][5]);
-      wl[n] = weno_right<T>(wprev[n], q[n][0], q[n][1], q[n][2], q[n][3], q[n][4]);
-      wr[n] = weno_left<T>(wcur, q[n][1], q[n][2], q[n][3], q[n][4], q[n][5]);
-      wprev[n] = wcur;
-#else
-      wl[n] = weno5<T>(q[n][4], q[n][3], q[n][2], q[n][1], q[n][0]);  // weno_r of cell c-1
-      wr[n] = weno5<T>(q[n][1], q[n][2], q[n][3], q[n][4], q[n][5]);  // weno_l of cell c
-#endif
-    }
-    const int k = dir == 1 ? v.ks + a : c;
-    const int j = dir == 1 ? c : v.js + a;
-    if (dir == 1) {
-      if (c == c0) edge_outer_state<T>(v, p, UP, a, i, wl);
-      else if (c == c1 + 1) edge_outer_state<T>(v, p, DOWN, a, i, wr);
-      FaceGeo<T> fg{T(geo(v, GCOSF2, p, k, j)), T(geo(v, GSINF2, p, k, j)),
-                    T(geo(v, GCTHP2, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-      riemann<T>(v.rsolver, v.gamma, IVY, fg, wl, wr, fx);
-    } else {
-      if (c == c0) edge_outer_state<T>(v, p, LEFT, a, i, wl);
-      else if (c == c1 + 1) edge_outer_state<T>(v, p, RIGHT, a, i, wr);
-      FaceGeo<T> fg{T(geo(v, GCOSF3, p, k, j)), T(geo(v, GSINF3, p, k, j)),
-                    T(geo(v, GCTHP3, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-      riemann<T>(v.rsolver, v.gamma, IVZ, fg, wl, wr, fx);
-    }
-    const size_t f0 = idx(v, p, 0, k, j, i);
-#pragma unroll
-    for (int n = 0; n < 5; ++n) {
-      if (n >= nv) break;
-      F[f0 + n * vs] = fx[n];
-    }
-    if (c <= c1) {  // slide: the next face needs cell c + 3
-#pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        if (n >= nv) break;
-#pragma unroll
-        for (int m = 0; m < 5; ++m) q[n][m] = q[n][m + 1];
-        q[n][5] = T(__ldg(W + n * vs + (long)(c + 3) * s));
-      }
-    }
-  }
-}
-
 // asynchronous 8-byte global -> shared copies (the next level's inputs)
 __device__ __forceinline__ void cp_async8(double* smem_dst, const double* gsrc) {
   unsigned sa = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -1296,49 +1123,44 @@ __device__ __forceinline__ void cp_async_wait_one() {
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
 }
 
-// Faces staged through shared memory: a block of X23_THREADS threads takes
-// 32 consecutive radial indices i (one per lane, so every global access of a
-// warp is a coalesced row) of one line of one panel and direction, and walks
-// the line in chunks of x23_chunk<T>() faces:
-//   0. the chunk's cells (with the three-cell halos of its stencils) are in
-//      shared memory, each cell copied once;
-//   1. one thread per cell computes both face values of the cell's WENO5
-//      reconstruction (the right-face value for the face above it, the
-//      left-face value for the face below; the mixed build shares the
-//      cell's smoothness indicators between the two, the FP64 build calls
-//      weno5 for each as the reference does);
-//   2. one thread per face takes the right-face value of the cell below
-//      and the left-face value of the cell above -- the neighbour panel's
-//      rotated state at a panel edge -- and solves the Riemann problem.
-// Each face gets the values and operations it gets in the per-face and
-// per-line kernels; phases 1 and 2 each keep few registers, so many warps
-// are resident.
+// Faces staged through shared memory: a block of X23_THREADS threads takes 32
+// lines of faces of one panel and direction, one per lane -- consecutive
+// (line, radial index) pairs, so that a row of 32 lanes reads runs along i and
+// no lane idles whatever the number of levels (with 32 radial indices of one
+// line per block, 40 levels kept 62 % of the lanes busy, 45 levels 70 %) --
+// and walks a segment of the lines in chunks of x23_chunk<T>() faces:
+// the chunk's cells, with the three-cell halos of its stencils, are copied to
+// shared memory while the chunk before is finished; one thread per face then
+// reconstructs both of the face's states (WENO5) -- at a panel edge the outer
+// one is the neighbour panel's rotated state -- and solves the Riemann problem.
+// Where x23_shares_beta says so, the mixed build reconstructs per cell first
+// (one thread per cell, both of its face values from one set of smoothness
+// indicators, through shared memory) and solves per face after a barrier.
+// What bounds it: instruction issue (mixed build, IPC 0.66 a scheduler) and
+// the FP64 pipe (FP64 build, 62 % busy), not memory (16 % and 11 % of DRAM).
+// Per launch, before (32 radial indices of one line per block, or one thread
+// per face where those left lanes idle; FP64 also through shared memory) and
+// now: FP64 48^2x3 33.1 -> 23.1 us, 40^2x40 145 -> 116, 96^2x64 695 -> 616;
+// mixed 24^2x32 26 -> 19, 62^2x45 143 -> 96, 126^2x70 595 -> 447, 192^2x96
+// 1115 -> 1104.
 #ifndef EXO_X23_THREADS
 #define EXO_X23_THREADS 128
 #endif
 constexpr int X23_THREADS = EXO_X23_THREADS;
-// A line's 32 lanes are its radial indices, so the line form keeps
-// L / (32 ceil(L / 32)) of its lanes busy: 3 of 32 at the exo2
-// shallow-water grid's 3 levels, 62.5 % at HS94's 40.  Below a busy
-// fraction the per-face form (X23_THREADS threads a block) is faster:
-// measured at 40 and 64 levels, the FP64 build's crossover lies near 85 %
-// (its line form is 16 % faster at 100 %, 2x slower at 62.5 %), the mixed
-// build's near 65 % (line form 1.7x faster at 100 %).
-#ifndef EXO_X23_LINE_BUSY_PCT
-#define EXO_X23_LINE_BUSY_PCT (EXO_MIXED ? 65 : 85)
-#endif
-__host__ __device__ constexpr bool x23_uses_lines(int L) {
-  return L * 100 >= EXO_X23_LINE_BUSY_PCT * 32 * ((L + 31) / 32);
+// Whether the mixed build shares a cell's smoothness indicators between its
+// two faces: a rule on the levels alone, since the two ways round
+// differently and a run's results have to depend on nothing but its
+// configuration.  (The line is where a block of 32 levels of one line used to
+// give way to one thread per face, which did not share them.)
+__host__ __device__ constexpr bool x23_shares_beta(int L) {
+  return EXO_MIXED && L * 100 >= 65 * 32 * ((L + 31) / 32);
 }
-template <class T>
+template <class T, bool kShareBeta>
 __host__ __device__ constexpr int x23_chunk() {
-  return sizeof(T) == 4 ? 15 : 7;
+  return kShareBeta ? 15 : sizeof(T) == 4 ? 16 : 8;
 }
-// blocks of the tiled x2/x3 kernel for one atmosphere: one per line of 32
-// radial indices of one row of one panel and direction
-__host__ __device__ constexpr unsigned x23_tile_blocks(int N, int L) {
-  return 2u * 6u * (unsigned)N * (unsigned)((L + 31) / 32);
-}
+// resident blocks per SM (launch bounds, or the registers it keeps)
+constexpr unsigned X23_RESIDENT = EXO_MIXED ? 4 : 3;
 
 // cp.async of 4 or 8 bytes, zero-filled when src_bytes is 0
 template <int B>
@@ -1349,51 +1171,54 @@ __device__ __forceinline__ void cp_async_zfill(void* smem_dst, const void* gsrc,
                : "memory");
 }
 
-// The x2/x3 faces of one line (32 radial indices of one row of one panel
-// and direction) chunk by chunk, with the same phases, values and
-// operations per face as the per-face form.  Cell m of the line (m = 0 three
-// cells below the first face) sits in ring slot m mod XR; the copies of chunk
-// q + 1's new cells are in flight while chunk q is finished.  Slots written
-// for chunk q + 1 held cells at least XR = 2 CF + 5 below them, which chunk q
-// no longer reads; the copies for chunk q + 2 start after the barrier that
-// ends chunk q's reconstruction.  The ring's position, the line's pointers
-// and strides are carried along: recomputed per row of copies and per face,
-// with divisions by the chunk's runtime length, they were 38 % of the mixed
-// build's instructions.
-template <class T>
+// The faces of a segment chunk by chunk.  Cell m of a line (m = 0 three cells
+// below the first face) sits in ring slot (m - the segment's first) mod XR;
+// the copies of chunk q + 1's new cells are in flight while chunk q is
+// finished.  Slots written for chunk q + 1 held cells at least XR = 2 CF + 5
+// below them, which chunk q no longer reads; the copies for chunk q + 2 start
+// after the barrier that ends chunk q's reconstruction.  The ring's position,
+// the lines' pointers and strides are carried along: recomputed per row of
+// copies and per face, with divisions by the chunk's runtime length, they
+// were 38 % of the mixed build's instructions.
+template <class T, bool kShareBeta>
 struct X23Shared {
-  static constexpr int CF = x23_chunk<T>(), NC = CF + 1, XR = 2 * CF + 5;
+  static constexpr int CF = x23_chunk<T, kShareBeta>(), XR = 2 * CF + 5;
+  static constexpr int NC = kShareBeta ? CF + 1 : 1;
   T ring[5][XR][32];
-  T srec[2][5][NC][32];
+  T srec[kShareBeta ? 2 : 1][5][NC][32];
 };
-template <class T, int NV>
-__device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X23Shared<T>& sm) {
-  constexpr int CF = X23Shared<T>::CF;
-  constexpr int NC = X23Shared<T>::NC;
-  constexpr int XR = X23Shared<T>::XR;
+template <class T, int NV, bool kShareBeta>
+__device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X23Shared<T, kShareBeta>& sm) {
+  constexpr int CF = X23Shared<T, kShareBeta>::CF;
+  constexpr int NC = X23Shared<T, kShareBeta>::NC;
+  constexpr int XR = X23Shared<T, kShareBeta>::XR;
   auto& ring = sm.ring;
   auto& srec = sm.srec;
   const int N = v.N, L = v.L;
-  const unsigned nit = (unsigned)((L + 31) / 32);
+  const X23Split sp = v.x23;
   unsigned r = blk;
-  const int itile = (int)(r % nit);
-  r /= nit;
-  const int a = (int)(r % (unsigned)N);
-  r /= (unsigned)N;
+  const unsigned group = r % sp.groups;
+  r /= sp.groups;
+  const unsigned seg = r % sp.segments;
+  r /= sp.segments;
   const int p = (int)(r % 6u);
   const int dir = (int)(r / 6u) + 1;
   const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
   constexpr int NW = X23_THREADS / 32;
-  const int il = itile * 32 + lane;
-  const bool active = il < L;
-  const int i = v.is + (active ? il : 0);
+  // this lane's line: place a across (k - ks for x2 faces, j - js for x3) and
+  // radial index; lanes past the last line repeat it and store nothing
+  const unsigned line = min(group * 32u + (unsigned)lane, (unsigned)(N * L) - 1u);
+  const bool active = group * 32u + (unsigned)lane < (unsigned)(N * L);
+  const int a = (int)v.div_L(line);
+  const int i = v.is + (int)(line - (unsigned)a * (unsigned)L);
   const size_t vs = v.cells;
   const size_t s = dir == 1 ? (size_t)v.nc1 : (size_t)v.nc1 * v.nc2;
   // the first face's place in the state and flux arrays
   const size_t base = dir == 1 ? idx(v, p, 0, v.ks + a, v.js, i) : idx(v, p, 0, v.ks, v.js + a, i);
   const T* const W = prim_array<T>(v) + base - 3 * s;  // cell 0
   T* const F = flux_array<T>(v, dir) + base;           // face 0
-  const int nch = (N + 1 + CF - 1) / CF;
+  const int q0 = (int)(seg * sp.chunks);
+  const int q1 = min((N + CF) / CF, q0 + (int)sp.chunks);
   const int rsolver = v.rsolver;
   const double gamma = v.gamma;
   // copies of the cells [m0, m0 + n), the first of them in slot slot0
@@ -1403,7 +1228,7 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X2
       const int m = m0 + c;
       int slot = slot0 + c;
       slot -= (slot >= XR) ? XR : 0;
-      const bool ok = active && m < N + 6;
+      const bool ok = m < N + 6;
       const T* src = W + (size_t)(ok ? m : 3) * s;
       T* dst = &ring[0][slot][lane];
 #pragma unroll
@@ -1414,58 +1239,69 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X2
     }
     cp_async_commit();
   };
-  issue(0, CF + 5, 0);
+  issue(q0 * CF, CF + 5, 0);
   int islot = CF + 5, rslot = 0;  // slots of the next cell to copy and of cell q CF
-  for (int q = 0; q < nch; ++q) {
-    if (q + 1 < nch) {
+#pragma unroll 1
+  for (int q = q0; q < q1; ++q) {
+    cp_async_wait_all();
+    __syncthreads();
+    if (q + 1 < q1) {
       issue(q * CF + CF + 5, CF, islot);
       islot += CF;
       islot -= (islot >= XR) ? XR : 0;
-      cp_async_wait_one();
-    } else {
-      cp_async_wait_all();
     }
-    __syncthreads();
-    // 1. both face values of the cells below and above the chunk's faces
+    if constexpr (kShareBeta) {
+      // both face values of the cells below and above the chunk's faces
 #pragma unroll 1
-    for (int mc = warp; mc < NC; mc += NW) {
-      const T* st[5];  // the cell's stencil
+      for (int mc = warp; mc < NC; mc += NW) {
+        const T* st[5];  // the cell's stencil
 #pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        int sl = rslot + mc + m;
-        sl -= (sl >= XR) ? XR : 0;
-        st[m] = &ring[0][sl][lane];
-      }
-      T* const rec = &srec[0][0][mc][lane];
+        for (int m = 0; m < 5; ++m) {
+          int sl = rslot + mc + m;
+          sl -= (sl >= XR) ? XR : 0;
+          st[m] = &ring[0][sl][lane];
+        }
+        T* const rec = &srec[0][0][mc][lane];
 #pragma unroll
-      for (int n = 0; n < NV; ++n) {
-        const T q0 = st[0][n * (XR * 32)], q1 = st[1][n * (XR * 32)], q2 = st[2][n * (XR * 32)];
-        const T q3 = st[3][n * (XR * 32)], q4 = st[4][n * (XR * 32)];
-#if EXO_X23_SHARED_BETA
-        const WenoCell<T> wc = weno_cell<T>(q0, q1, q2, q3, q4);
-        rec[n * (NC * 32)] = weno_right<T>(wc, q0, q1, q2, q3, q4);
-        rec[(5 + n) * (NC * 32)] = weno_left<T>(wc, q0, q1, q2, q3, q4);
-#else
-        rec[n * (NC * 32)] = weno5<T>(q4, q3, q2, q1, q0);
-        rec[(5 + n) * (NC * 32)] = weno5<T>(q0, q1, q2, q3, q4);
-#endif
+        for (int n = 0; n < NV; ++n) {
+          const T c0 = st[0][n * (XR * 32)], c1 = st[1][n * (XR * 32)], c2 = st[2][n * (XR * 32)];
+          const T c3 = st[3][n * (XR * 32)], c4 = st[4][n * (XR * 32)];
+          const WenoCell<T> wc = weno_cell<T>(c0, c1, c2, c3, c4);
+          rec[n * (NC * 32)] = weno_right<T>(wc, c0, c1, c2, c3, c4);
+          rec[(5 + n) * (NC * 32)] = weno_left<T>(wc, c0, c1, c2, c3, c4);
+        }
       }
+      __syncthreads();
     }
-    rslot += CF;
-    rslot -= (rslot >= XR) ? XR : 0;
-    __syncthreads();
-    if (!active) continue;
-    // 2. the faces q CF .. q CF + CF - 1 (up to N)
+    // the faces q CF .. q CF + CF - 1 (up to N)
 #pragma unroll 1
     for (int mf = warp; mf < CF; mf += NW) {
       const int f = q * CF + mf;
-      if (f > N) break;
+      if (f > N || !active) break;
       T wl[5], wr[5], fx[5] = {T(0.), T(0.), T(0.), T(0.), T(0.)};
-      const T* const rec = &srec[0][0][mf][lane];
+      if constexpr (kShareBeta) {
+        const T* const rec = &srec[0][0][mf][lane];
 #pragma unroll
-      for (int n = 0; n < NV; ++n) {
-        wl[n] = rec[n * (NC * 32)];
-        wr[n] = rec[(5 + n) * (NC * 32) + 32];
+        for (int n = 0; n < NV; ++n) {
+          wl[n] = rec[n * (NC * 32)];
+          wr[n] = rec[(5 + n) * (NC * 32) + 32];
+        }
+      } else {
+        const T* st[6];  // the three cells below the face and the three above
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          int sl = rslot + mf + m;
+          sl -= (sl >= XR) ? XR : 0;
+          st[m] = &ring[0][sl][lane];
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          T c[6];
+#pragma unroll
+          for (int m = 0; m < 6; ++m) c[m] = st[m][n * (XR * 32)];
+          wl[n] = weno5<T>(c[4], c[3], c[2], c[1], c[0]);
+          wr[n] = weno5<T>(c[1], c[2], c[3], c[4], c[5]);
+        }
       }
       if (dir == 1) {
         if (f == 0) edge_outer_state<T>(v, p, UP, a, i, wl);
@@ -1489,20 +1325,29 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X2
         out += vs;
       }
     }
+    rslot += CF;
+    rslot -= (rslot >= XR) ? XR : 0;
   }
 }
 
 template <class T>
 __device__ __forceinline__ void flux_x23_block(const DevView& v, unsigned blk) {
-  if constexpr (EXO_X23_TILES) {
-    __shared__ __align__(16) X23Shared<T> sm;
-    if (!x23_uses_lines(v.L)) flux_x23_faces<T>(v, blk);
-    else if (v.nv == 5) flux_x23_pipe<T, 5>(v, blk, sm);
-    else flux_x23_pipe<T, 4>(v, blk, sm);
-  } else if constexpr (EXO_X23_LINES) {
-    flux_x23_lines<T>(v, blk);
+  if constexpr (EXO_MIXED) {
+    __shared__ union {
+      __align__(16) X23Shared<T, true> cells;
+      __align__(16) X23Shared<T, false> faces;
+    } sm;
+    if (x23_shares_beta(v.L)) {
+      if (v.nv == 5) flux_x23_pipe<T, 5, true>(v, blk, sm.cells);
+      else flux_x23_pipe<T, 4, true>(v, blk, sm.cells);
+    } else {
+      if (v.nv == 5) flux_x23_pipe<T, 5, false>(v, blk, sm.faces);
+      else flux_x23_pipe<T, 4, false>(v, blk, sm.faces);
+    }
   } else {
-    flux_x23_faces<T>(v, blk);
+    __shared__ __align__(16) X23Shared<T, false> sm;
+    if (v.nv == 5) flux_x23_pipe<T, 5, false>(v, blk, sm);
+    else flux_x23_pipe<T, 4, false>(v, blk, sm);
   }
 }
 
@@ -3180,26 +3025,16 @@ __global__ void EXO_X1_BOUNDS kb_flux_x1(Batch bt) {
   flux_x1_block<T>(sv, b);
 }
 
-// the mixed build's sliding-window kernel: 168 registers (3 blocks of 128
-// threads per SM) measured 16 % faster than its natural 208 at 6x192^2x96;
-// the FP64 per-face kernel needs fewer
-#if !defined(EXO_X23_MAXNREG) && EXO_MIXED && !EXO_X23_TILES
-#define EXO_X23_MAXNREG 168
-#endif
-// the pipelined line kernel of the mixed build at 128 registers (4 blocks of
-// 128 threads per SM): 1.64 ms per launch at 6x192^2x96 against 1.75 at its
-// natural 148 and 1.91 for one block per chunk
-#if EXO_X23_TILES && EXO_MIXED && !defined(EXO_X23_MINB)
+// the mixed build at 128 registers (4 blocks of 128 threads per SM): 1.64 ms
+// per launch at 6x192^2x96 against 1.75 at its natural 148 (line form with
+// recomputed addresses)
+#if EXO_MIXED && !defined(EXO_X23_MINB)
 #define EXO_X23_MINB 4
 #endif
-#if EXO_X23_TILES && defined(EXO_X23_MINB)
+#if defined(EXO_X23_MINB)
 #define EXO_X23_BOUNDS __launch_bounds__(X23_THREADS, EXO_X23_MINB)
-#elif EXO_X23_TILES
-#define EXO_X23_BOUNDS __launch_bounds__(X23_THREADS)
-#elif defined(EXO_X23_MAXNREG)
-#define EXO_X23_BOUNDS __maxnreg__(EXO_X23_MAXNREG)
 #else
-#define EXO_X23_BOUNDS
+#define EXO_X23_BOUNDS __launch_bounds__(X23_THREADS)
 #endif
 template <class T>
 __global__ void EXO_X23_BOUNDS kb_flux_x23(Batch bt) {
@@ -3344,9 +3179,6 @@ inline void launch_kb_implicit(int precision, unsigned blocks, int threads, int 
 // alone executes exactly the code it executes inside an ensemble.
 inline Batch one(const DevView& v, int kind) { return Batch{v.self, v.starts + 2 * kind, 1}; }
 
-// threads per block of the x2/x3 kernel: the tiled form is fixed at X23_THREADS
-inline int x23_threads(int tile) { return EXO_X23_TILES ? X23_THREADS : tile; }
-
 inline unsigned member_block_count(const DevView& v, int kind) {
   unsigned b[BK_COUNT];
   member_blocks(v, v.tiles, b);
@@ -3365,12 +3197,28 @@ int launch_reciprocal(int n, const double* x, double* out, void* stream) {
   return check_launch();
 }
 
-unsigned x23_blocks(const DevView& v, int tile) {
-  const bool lines = EXO_X23_TILES ? x23_uses_lines(v.L) : (bool)EXO_X23_LINES;
-  if (EXO_X23_TILES && lines) return x23_tile_blocks(v.N, v.L);
-  if (EXO_X23_TILES) tile = X23_THREADS;  // the per-face form of the tiled build
-  const size_t n = lines ? (size_t)2 * 6 * v.N * v.L : (size_t)2 * 6 * v.N * (v.N + 1) * v.L;
-  return (unsigned)((n + tile - 1) / tile);
+// Lines are cut into segments where one segment per line would fill the last
+// wave of blocks badly: the count of segments whose waves x length is least,
+// a segment's length being its chunks and half a chunk for the first cells'
+// way in.  (FP64, N = 40, 40 levels, 600 lines' blocks for 444 places: one
+// segment 135 us, two 116; N = 48, 3 levels, 60 blocks: seven segments.)
+X23Split x23_split(int N, int L) {
+  using T = EXO_FLUX_T;
+  const unsigned CF = x23_shares_beta(L) ? x23_chunk<T, true>() : x23_chunk<T, false>();
+  const unsigned groups = (unsigned)(((size_t)N * (size_t)L + 31) / 32);
+  const unsigned nch = ((unsigned)N + CF) / CF, places = 148u * X23_RESIDENT;
+  X23Split best{groups, nch, 1};
+  size_t least = 0;
+  for (unsigned n = 1; n <= nch; ++n) {
+    const unsigned per = (nch + n - 1) / n, segments = (nch + per - 1) / per;
+    const size_t waves = ((size_t)12 * groups * segments + places - 1) / places;
+    const size_t cost = waves * (2 * per + 1);
+    if (n == 1 || cost < least) {
+      least = cost;
+      best = {groups, per, segments};
+    }
+  }
+  return best;
 }
 
 int prepare_kernels() {
@@ -3415,7 +3263,7 @@ int launch_flux_x1(const DevView& v, void* stream) {
 }
 
 int launch_flux_x23(const DevView& v, void* stream) {
-  kb_flux_x23<EXO_FLUX_T><<<member_block_count(v, BK_X23), x23_threads(v.tiles[BK_X23]), 0,
+  kb_flux_x23<EXO_FLUX_T><<<member_block_count(v, BK_X23), X23_THREADS, 0,
                             (cudaStream_t)stream>>>(
       one(v, BK_X23));
   return check_launch();
@@ -3486,7 +3334,7 @@ int launch_batched_step(const BatchPlan& pl, void* stream) {
       kb_flux_x1<EXO_FLUX_T><<<pl.total[BK_X1], pl.x1_threads, pl.x1_smem, st>>>(B(BK_X1));
       if ((rc = check_launch())) return rc;
     }
-    kb_flux_x23<EXO_FLUX_T><<<pl.total[BK_X23], x23_threads(pl.threads[BK_X23]), 0, st>>>(
+    kb_flux_x23<EXO_FLUX_T><<<pl.total[BK_X23], X23_THREADS, 0, st>>>(
         B(BK_X23));
     if ((rc = check_launch())) return rc;
     kb_update<EXO_FLUX_T><<<pl.total[BK_UPDATE], pl.threads[BK_UPDATE], 0, st>>>(B(BK_UPDATE), s);
