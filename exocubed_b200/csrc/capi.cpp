@@ -329,6 +329,7 @@ int view_allocate(const exo_config& cfg, const HostTables& t, DevView& v,
     v.hs[HS_CVM] = cp - cfg.Rd;
   }
   v.gamma = cfg.gamma;
+  v.gas = make_riemann_gas(v.gamma);
   v.Rd = cfg.Rd;
   v.grav = shallow ? 0. : cfg.grav;
   v.cfl = cfg.cfl;

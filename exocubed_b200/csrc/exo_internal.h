@@ -154,6 +154,29 @@ inline FastDiv make_fastdiv(unsigned d) {
   return f;
 }
 
+#ifdef __CUDACC__
+#define EXO_HD __host__ __device__
+#else
+#define EXO_HD
+#endif
+// What the ideal-gas Riemann solvers need of gamma (LMARS: kappa + 1 and the
+// sound speed's factor; HLLC: 1 + (gamma - 1), 1 / (gamma - 1) and the shock
+// speed's (gamma + 1) / (2 gamma)).
+template <class T>
+struct RiemannGas {
+  T gamma, kappa1, cfac, gam, igm1, qfac;
+};
+template <class T>
+EXO_HD inline RiemannGas<T> make_riemann_gas(T gamma) {
+  const T one = T(1.), kappa = one / (gamma - one);
+  return {gamma,
+          kappa + one,
+          one + (one / kappa + one / kappa) / T(2.),
+          one + (gamma - one),
+          kappa,
+          (gamma + one) / (T(2) * gamma)};
+}
+
 // How the x2/x3 fluxes are cut: groups of 32 lines per panel and direction,
 // chunks of faces per segment of a line, segments.
 struct X23Split {
@@ -169,6 +192,7 @@ struct alignas(16) DevView {
   int is, ie, js, je, ks, ke;
   int eqn, rsolver, implicit_flag, coriolis;
   int precision, forcing;
+  RiemannGas<double> gas;  // of gamma
   double gamma, Rd, grav, cfl;
   double hs[NHS];                  // Held-Suarez constants (forcing == EXO_FORCING_HS94)
   size_t cells;                    // nc3*nc2*nc1 (one variable of one panel)
@@ -228,11 +252,6 @@ constexpr int X1_MAX_COLUMNS = 8;
 // the x1 kernel's dynamic shared memory limit (the mixed build's 8 columns
 // of 250 levels take 212 KB)
 constexpr int X1_SMEM_MAX = 224 * 1024;
-#ifdef __CUDACC__
-#define EXO_HD __host__ __device__
-#else
-#define EXO_HD
-#endif
 // the precisions stepped by the mixed build (exo::mixed)
 EXO_HD inline bool mixed_build(int precision) {
   return precision == EXO_PREC_MIXED || precision == EXO_PREC_MIXED_F32_SOLVE;
@@ -248,21 +267,23 @@ inline int implicit_launches(int kinds, int precision) {
   return ((kinds & IMPL_FULL) ? (precision == EXO_PREC_MIXED ? 1 : 2) : 0) +
          ((kinds & IMPL_PARTIAL) ? 2 : 0);
 }
-// shared doubles of one x1 column: w [nv][nc1] and psf [nc1+1]; the mixed
-// build adds ln psf and the face densities [2][nc1+1] and the cells' two
-// WENO5 face values [2][nv][L+2] in FP32 (nv (L+2) doubles)
+// shared doubles of one x1 column: w [5][nc1] and psf [nc1+1]; in the mixed
+// build density and pressure [2][nc1], psf, ln psf and the face densities
+// [3][nc1+1], and in FP32 what is reconstructed [5][nc1] and the cells' two
+// WENO5 face values [2][5][L+2]
 EXO_HD inline int x1_column_doubles(const DevView& v) {
   int faces = v.nc1 + 1;
-  return v.nv * v.nc1 +
-         (mixed_build(v.precision) ? 3 * faces + v.nv * (v.L + 2) : faces);
+  return mixed_build(v.precision)
+             ? 2 * v.nc1 + 3 * faces + (5 * v.nc1 + 1) / 2 + 5 * (v.L + 2)
+             : 5 * v.nc1 + faces;
 }
 inline int x1_cols(const DevView& v) { return v.tiles[BK_X1] > 0 ? v.tiles[BK_X1] : 1; }
 inline size_t x1_smem_bytes(const DevView& v) {
   return (size_t)x1_cols(v) * x1_column_doubles(v) * sizeof(double);
 }
-// threads: the block's faces in whole warps, at most 1024
+// threads: the block's faces, ghosts included, in whole warps, at most 1024
 inline int x1_threads(const DevView& v) {
-  int t = ((x1_cols(v) * (v.L + 1) + 31) / 32) * 32;
+  int t = ((x1_cols(v) * (v.nc1 + 1) + 31) / 32) * 32;
   return t > 1024 ? 1024 : t;
 }
 // Columns per block of a member of a batch whose x1 blocks run `threads`
@@ -270,7 +291,7 @@ inline int x1_threads(const DevView& v) {
 // than the batch's deepest takes more columns per block rather than leave
 // threads idle), 1 to X1_MAX_COLUMNS, within the kernel's shared memory.
 inline int x1_member_columns(const DevView& v, int threads, size_t smem_max) {
-  int c = threads / (v.L + 1);
+  int c = threads / (v.nc1 + 1);
   c = c < 1 ? 1 : (c > X1_MAX_COLUMNS ? X1_MAX_COLUMNS : c);
   const size_t per = (size_t)x1_column_doubles(v) * sizeof(double);
   while (c > 1 && (size_t)c * per > smem_max) --c;

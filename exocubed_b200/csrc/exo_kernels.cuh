@@ -43,12 +43,6 @@
 #ifndef EXO_X1_FLUX64
 #define EXO_X1_FLUX64 EXO_MIXED
 #endif
-// 1: the x1 kernel, whose cells' face values go through shared memory,
-// computes each cell's WENO smoothness indicators once for both of its faces
-// (mixed build; the FP64 build keeps weno5's order)
-#ifndef EXO_X1_SHARED_BETA
-#define EXO_X1_SHARED_BETA EXO_MIXED
-#endif
 
 namespace exo {
 namespace EXO_KNS {
@@ -423,23 +417,26 @@ __device__ __forceinline__ void riemann_roe_shallow(int ivx, const FaceGeo<T>& f
   flx[ivy] = tz + ty * fg.cthp;
 }
 
+// The solvers' functions of gamma: in FP64 those of the view, which the host
+// computed (two divisions a face fewer); in FP32 computed where they are used.
+template <class T>
+__device__ __forceinline__ RiemannGas<T> riemann_gas(const RiemannGas<double>& gas) {
+  if constexpr (sizeof(T) == sizeof(double)) return gas;
+  else return make_riemann_gas<T>(T(gas.gamma));
+}
+
 // lmars.cpp:24-110 (NVAPOR = NCLOUD = 0), no projection
 template <class T>
-__device__ __forceinline__ void riemann_lmars(double gamma_d, int ivx, const T* wli, const T* wri, T* flx) {
+__device__ __forceinline__ void riemann_lmars(const RiemannGas<T>& gas, int ivx, const T* wli, const T* wri, T* flx) {
   const T h = T(0.5), one = T(1.);
-  T gamma = T(gamma_d);
   int ivy = IVX + ((ivx - IVX) + 1) % 3;
   int ivz = IVX + ((ivx - IVX) + 2) % 3;
-  T fsig = one, feps = one;
-  T kappal = one / (gamma - one) * fsig / feps;
-  T kappar = one / (gamma - one) * fsig / feps;
-  T hl = wli[IPR] / wli[IDN] * (kappal + one) +
+  T hl = wli[IPR] / wli[IDN] * gas.kappa1 +
          h * (sqr(wli[ivx]) + sqr(wli[ivy]) + sqr(wli[ivz]));
-  T hr = wri[IPR] / wri[IDN] * (kappar + one) +
+  T hr = wri[IPR] / wri[IDN] * gas.kappa1 +
          h * (sqr(wri[ivx]) + sqr(wri[ivy]) + sqr(wri[ivz]));
   T rhobar = h * (wli[IDN] + wri[IDN]);
-  T cbar = sqrt(h * (one + (one / kappar + one / kappal) / T(2.)) *
-                (wli[IPR] + wri[IPR]) / rhobar);
+  T cbar = sqrt(h * gas.cfac * (wli[IPR] + wri[IPR]) / rhobar);
   T pbar = h * (wli[IPR] + wri[IPR]) + h * (rhobar * cbar) * (wli[ivx] - wri[ivx]);
   T ubar = h * (wli[ivx] + wri[ivx]) + h / (rhobar * cbar) * (wli[IPR] - wri[IPR]);
   T rdl = one, rdr = one;
@@ -460,20 +457,17 @@ __device__ __forceinline__ void riemann_lmars(double gamma_d, int ivx, const T* 
 
 // hllc_transform.cpp:24-263
 template <class T>
-__device__ __forceinline__ void riemann_hllc(double gamma_d, int ivx, const FaceGeo<T>& fg, T* wl, T* wr, T* flx) {
+__device__ __forceinline__ void riemann_hllc(const RiemannGas<T>& gas, int ivx, const FaceGeo<T>& fg, T* wl, T* wr, T* flx) {
   const T h = T(.5), one = T(1.0), zero = T(0.0);
-  T gamma = T(gamma_d);
   int ivy = IVX + ((ivx - IVX) + 1) % 3;
   int ivz = IVX + ((ivx - IVX) + 2) % 3;
-  T gm1 = gamma - one, igm1 = one / gm1;
   prim_to_local(ivx, fg, wl);
   prim_to_local(ivx, fg, wr);
   T wli[5], wri[5], fl[5], fr[5];
   wli[IDN] = wl[IDN]; wli[IVX] = wl[ivx]; wli[IVY] = wl[ivy]; wli[IVZ] = wl[ivz]; wli[IPR] = wl[IPR];
   wri[IDN] = wr[IDN]; wri[IVX] = wr[ivx]; wri[IVY] = wr[ivy]; wri[IVZ] = wr[ivz]; wri[IPR] = wr[IPR];
-  T fsig = one, feps = one;
-  T cl = sqrt((one + (gamma - one) * feps / fsig) * wli[IPR] / wli[IDN]);
-  T cr = sqrt((one + (gamma - one) * feps / fsig) * wri[IPR] / wri[IDN]);
+  T cl = sqrt(gas.gam * wli[IPR] / wli[IDN]);
+  T cr = sqrt(gas.gam * wri[IPR] / wri[IDN]);
   T KE_l, KE_r;
   if (ivx == IVX) {
     T cth = fg.cthc, vy, vz;
@@ -487,15 +481,15 @@ __device__ __forceinline__ void riemann_hllc(double gamma_d, int ivx, const Face
     KE_l = h * wli[IDN] * (sqr(wli[IVX]) + sqr(wli[IVY]) + sqr(wli[IVZ]));
     KE_r = h * wri[IDN] * (sqr(wri[IVX]) + sqr(wri[IVY]) + sqr(wri[IVZ]));
   }
-  T el = wli[IPR] * igm1 + KE_l;
-  T er = wri[IPR] * igm1 + KE_r;
+  T el = wli[IPR] * gas.igm1 + KE_l;
+  T er = wri[IPR] * gas.igm1 + KE_r;
   T rhoa = h * (wli[IDN] + wri[IDN]);
   T ca = h * (cl + cr);
   T pmid = h * (wli[IPR] + wri[IPR] + (wli[IVX] - wri[IVX]) * rhoa * ca);
   T ql = (pmid <= wli[IPR]) ? one
-         : sqrt(one + (gamma + one) / (T(2) * gamma) * (pmid / wli[IPR] - one));
+         : sqrt(one + gas.qfac * (pmid / wli[IPR] - one));
   T qr = (pmid <= wri[IPR]) ? one
-         : sqrt(one + (gamma + one) / (T(2) * gamma) * (pmid / wri[IPR] - one));
+         : sqrt(one + gas.qfac * (pmid / wri[IPR] - one));
   T al = wli[IVX] - cl * ql;
   T ar = wri[IVX] + cr * qr;
   T bp = ar > zero ? ar : T(TINY_NUMBER);
@@ -571,12 +565,12 @@ __device__ __forceinline__ void riemann_lmars_shallow(int ivx, const FaceGeo<T>&
 }
 
 template <class T>
-__device__ __forceinline__ void riemann(int rsolver, double gamma, int ivx, const FaceGeo<T>& fg,
+__device__ __forceinline__ void riemann(int rsolver, const RiemannGas<double>& gas, int ivx, const FaceGeo<T>& fg,
                                         T* wl, T* wr, T* flx) {
   switch (rsolver) {
     case EXO_RS_ROE_SHALLOW: riemann_roe_shallow(ivx, fg, wl, wr, flx); break;
-    case EXO_RS_LMARS: riemann_lmars(gamma, ivx, wl, wr, flx); break;
-    case EXO_RS_HLLC: riemann_hllc(gamma, ivx, fg, wl, wr, flx); break;
+    case EXO_RS_LMARS: riemann_lmars(riemann_gas<T>(gas), ivx, wl, wr, flx); break;
+    case EXO_RS_HLLC: riemann_hllc(riemann_gas<T>(gas), ivx, fg, wl, wr, flx); break;
     default: riemann_lmars_shallow(ivx, fg, wl, wr, flx); break;
   }
 }
@@ -742,11 +736,19 @@ __device__ __forceinline__ void prim_ghost_block(const DevView& v, unsigned blk,
 }
 
 // ------------------------------------------------------------ k_flux_x1 ---
-// One CTA per interior radial column.
 // Several radial columns per block (the x1 tile): each column's faces,
 // cells and hydrostatic scan are spread over the block's threads, so the
 // block's lanes stay busy (one column of L+1 faces leaves most of a warp
-// idle) and the columns' serial scans run side by side.
+// idle) and the columns' scans run side by side.
+// What bounds it: instruction issue (mixed build, 96^2x64: 1,724 instructions
+// per 32 cells at 0.66 a cycle and scheduler; DRAM 13 %), a third of them FP32
+// WENO5, then the FP64 decomposition and the Riemann solve.  It was 2,074 with
+// a division for its place per pass and element, a thread's cells converted to
+// FP32 five times, the reciprocal of gamma and the solver's functions of it
+// per cell, and the series' coefficients as literals.  Per launch, before and
+// now: FP64 40^2x40 76 -> 69 us, 96^2x64 484 -> 420; mixed 24^2x32 19 -> 17,
+// 62^2x45 120 -> 111, 96^2x64 312 -> 261, 126^2x70 666 -> 548, 192^2x96 1705
+// -> 1460.
 __device__ __forceinline__ int x1_columns_per_block(const DevView& v) {
   return v.tiles[BK_X1] > 0 ? v.tiles[BK_X1] : 1;
 }
@@ -760,78 +762,132 @@ __device__ __forceinline__ void divmod_small(int t, int d, float inv_d, int& q, 
   else if (r >= d) { ++q; r -= d; }
 }
 
+#if EXO_MIXED
 // ln(sinh x / x) for |x| <= 0.25: its Taylor series sum_n c_n x^{2n} with
 // c_n = 2^{2n} B_{2n} / (2n (2n)!) (B the Bernoulli numbers), seven terms
-// (truncation error below 4e-19 there)
+// (truncation error below 4e-19 there).  The two series' coefficients are read
+// from the constant bank: as literals each takes two moves to registers.
+__constant__ double kSinhc[7] = {1. / 6,        -1. / 180,           1. / 2835,
+                                 -1. / 37800,   1. / 467775,         -691. / 3831077250.,
+                                 2. / 127702575.};
 __device__ __forceinline__ double ln_sinhc(double x) {
   const double z = x * x;
-  return z * (1. / 6 +
-              z * (-1. / 180 +
-                   z * (1. / 2835 +
-                        z * (-1. / 37800 +
-                             z * (1. / 467775 +
-                                  z * (-691. / 3831077250. + z * (2. / 127702575.)))))));
+  double s = kSinhc[6];
+#pragma unroll
+  for (int k = 5; k >= 0; --k) s = kSinhc[k] + z * s;
+  return z * s;
 }
 // e^y for |y| <= 0.25: its Taylor series to y^13 (truncation below 5e-20)
+__constant__ double kInvFact[14] = {1.,
+                                    1.,
+                                    1. / 2,
+                                    1. / 6,
+                                    1. / 24,
+                                    1. / 120,
+                                    1. / 720,
+                                    1. / 5040,
+                                    1. / 40320,
+                                    1. / 362880,
+                                    1. / 3628800,
+                                    1. / 39916800,
+                                    1. / 479001600,
+                                    1. / 6227020800.};
 __device__ __forceinline__ double exp_small(double y) {
-  constexpr double inv_fact[14] = {1.,
-                                   1.,
-                                   1. / 2,
-                                   1. / 6,
-                                   1. / 24,
-                                   1. / 120,
-                                   1. / 720,
-                                   1. / 5040,
-                                   1. / 40320,
-                                   1. / 362880,
-                                   1. / 3628800,
-                                   1. / 39916800,
-                                   1. / 479001600,
-                                   1. / 6227020800.};
-  double s = inv_fact[13];
+  double s = kInvFact[13];
 #pragma unroll
-  for (int k = 12; k >= 0; --k) s = s * y + inv_fact[k];
+  for (int k = 12; k >= 0; --k) s = s * y + kInvFact[k];
   return s;
 }
+#endif
 
 template <class T>
 __device__ __forceinline__ void flux_x1_block(const DevView& v, unsigned blk) {
+  constexpr int NV = 5;  // the ideal gas only
   extern __shared__ double sm[];
-  __shared__ double s_gam[X1_MAX_COLUMNS], s_expf[X1_MAX_COLUMNS];
+  __shared__ double s_igam[X1_MAX_COLUMNS], s_expf[X1_MAX_COLUMNS];
   __shared__ double s_cthp[X1_MAX_COLUMNS], s_cosc[X1_MAX_COLUMNS];
-  __shared__ long long s_base[X1_MAX_COLUMNS];  // idx(p, 0, k, j, 0) of each column
+  __shared__ size_t s_base[X1_MAX_COLUMNS];  // the column's first face in the flux array
   const int cpb = x1_columns_per_block(v);
   const int ncol_total = 6 * v.N * v.N;
   const int col0 = (int)blk * cpb;
   const int ncb = min(cpb, ncol_total - col0);  // columns of this block
-  const int nc1 = v.nc1, nv = v.nv, L = v.L;
-  const int cstride = x1_column_doubles(v);    // shared doubles per column
+  const int nc1 = v.nc1, L = v.L, is = v.is, ie = v.ie;
+  const int cstride = x1_column_doubles(v);  // shared doubles per column
   const size_t vs = v.cells;
-  // shared memory of column c: w [nv][nc1], psf [nc1+1] (mixed: ln psf, dsf)
-  auto WC = [&](int c) { return sm + (size_t)c * cstride; };
-  auto PSF = [&](int c) { return sm + (size_t)c * cstride + nv * nc1; };
-  if ((int)threadIdx.x < ncb) {
-    const int c = threadIdx.x, col = col0 + c;
-    const int j = v.js + col % v.N;
-    const int k = v.ks + (col / v.N) % v.N;
-    const int p = col / (v.N * v.N);
-    s_base[c] = (long long)idx(v, p, 0, k, j, 0);
-    s_cthp[c] = geo(v, GCTHP1, p, k, j);
-    s_cosc[c] = geo(v, GCOSC, p, k, j);
-  }
-  __syncthreads();
-  {
-    const int per = nv * nc1;
-    const float inv_per = 1.f / (float)per, inv_nc1 = 1.f / (float)nc1;
-    for (int t = threadIdx.x; t < ncb * per; t += blockDim.x) {
-      int c, r, n, i;
-      divmod_small(t, per, inv_per, c, r);
-      divmod_small(r, nc1, inv_nc1, n, i);
-      WC(c)[r] = v.w[(size_t)s_base[c] + n * vs + i];
+  const int tid = (int)threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nwarps = (int)blockDim.x >> 5;
+  // Every pass runs over (column c, index i) with i up to the nc1 + 1 faces,
+  // the widest of them, so that a thread's place is computed once (a block
+  // has a thread for each place unless that is more than 1024).
+  const int per = nc1 + 1;
+  const float inv_per = 1.f / (float)per;
+  int c0, i0;
+  divmod_small(tid, per, inv_per, c0, i0);
+  auto each = [&](auto&& body) {
+    int c = c0, i = i0;
+#pragma unroll 1
+    for (int t = tid; t < ncb * per;) {
+      body(c, i);
+      t += (int)blockDim.x;
+      if (t < ncb * per) divmod_small(t, per, inv_per, c, i);
     }
+  };
+  // the column's first place in the state array
+  auto base = [&](int c) {
+    const unsigned col = (unsigned)(col0 + c);
+    const unsigned r = v.div_N(col), p = v.div_N(r);
+    return idx(v, (int)p, 0, v.ks + (int)(r - p * (unsigned)v.N),
+               v.js + (int)(col - r * (unsigned)v.N), 0);
+  };
+  // Shared memory of column c.  FP64: w [5][nc1] and psf [nc1 + 1].  Mixed:
+  // density and pressure [2][nc1], psf, ln psf and the isentropic density at
+  // the faces [3][nc1 + 1], then in FP32 what is reconstructed [5][nc1] and
+  // both face values of the cells is - 1 .. ie + 1 [2][5][L + 2].
+  auto COL = [&](int c) { return sm + (unsigned)(c * cstride); };
+#if EXO_MIXED
+  const int ncell = L + 2;
+  auto WD = [&](int c) { return COL(c); };
+  auto WP = [&](int c) { return COL(c) + nc1; };
+  auto PSF = [&](int c) { return COL(c) + 2 * nc1; };
+  auto WF = [&](int c) { return reinterpret_cast<T*>(COL(c) + 2 * nc1 + 3 * per); };
+  auto REC = [&](int c) { return WF(c) + NV * nc1; };
+#else
+  auto WD = [&](int c) { return COL(c) + IDN * nc1; };
+  auto WP = [&](int c) { return COL(c) + IPR * nc1; };
+  auto PSF = [&](int c) { return COL(c) + NV * nc1; };
+#endif
+  if (tid < ncb) {
+    const unsigned col = (unsigned)(col0 + tid);
+    const unsigned r = v.div_N(col), p = v.div_N(r);
+    const int k = v.ks + (int)(r - p * (unsigned)v.N), j = v.js + (int)(col - r * (unsigned)v.N);
+    s_base[tid] = idx(v, (int)p, 0, k, j, is);
+    s_cthp[tid] = geo(v, GCTHP1, (int)p, k, j);
+    s_cosc[tid] = geo(v, GCOSC, (int)p, k, j);
   }
-  __syncthreads();
   const bool decomp = (v.grav != 0.);
+  each([&](int c, int i) {
+    if (i >= nc1) return;
+    const double* src = v.w + base(c) + i;
+#if EXO_MIXED
+    T* f = WF(c) + i;
+    const double d = src[0], p = src[IPR * vs];
+    WD(c)[i] = d;
+    WP(c)[i] = p;
+#pragma unroll
+    for (int n = IVX; n <= IVZ; ++n) f[n * nc1] = T(src[n * vs]);
+    if (!decomp) {
+      f[IDN * nc1] = T(d);
+      f[IPR * nc1] = T(p);
+    }
+#else
+    double* dst = COL(c) + i;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) dst[n * nc1] = src[n * vs];
+    // the weight of the layer, which the downward scan below adds up
+    if (decomp && i >= is && i <= ie) PSF(c)[i] = -v.grav * src[0] * v.dx1f[i];
+#endif
+  });
+  __syncthreads();
   if (decomp) {
     // Decomposition::ChangeToPerturbation (change_to_perturbation.cpp:39-157).
 #if EXO_MIXED
@@ -839,18 +895,15 @@ __device__ __forceinline__ void flux_x1_block(const DevView& v, unsigned blk) {
     // one warp per column: each lane sums a chunk of levels, the lanes'
     // sums are scanned with shuffles, then each lane fills its chunk (FP64
     // throughout; only the order of the additions differs from the serial
-    // scan of the FP64 build)
+    // scan of the FP64 build).  The column's two logarithms share one call
+    // (lanes 0 and 1), and its two exponentials another.
     {
-      const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-      const int nwarps = (int)blockDim.x >> 5;
-      const int is = v.is, ie = v.ie;
       const int chunk = (L + 31) >> 5;
       const double grav = -v.grav;
       for (int c = warp; c < ncb; c += nwarps) {
-        double* wc = WC(c);
         double* psf = PSF(c);
-        const double* wd = wc + IDN * nc1;
-        const double* wp = wc + IPR * nc1;
+        const double* wd = WD(c);
+        const double* wp = WP(c);
         const int m0 = is + lane * chunk, m1 = min(m0 + chunk, ie + 1);
         double part = 0.;
         for (int m = m0; m < m1; ++m) part += grav * wd[m] * v.dx1f[m];
@@ -863,11 +916,23 @@ __device__ __forceinline__ void flux_x1_block(const DevView& v, unsigned blk) {
         }
         above = __shfl_down_sync(0xffffffffu, above, 1);
         if (lane == 31) above = 0.;
+        double gammad = v.gamma, fsig = 1., feps = 1.;
+        double gam = 1. + (gammad - 1.) * feps / fsig;
+        double lg = 0., ex = 0.;
+        if (lane < 2) lg = log(lane == 0 ? wp[is] : wd[is]);
+        const double lgd = __shfl_sync(0xffffffffu, lg, 1);
+        lg = __shfl_sync(0xffffffffu, lg, 0);
+        double ent = lg - gam * lgd;
+        const double RdTv = wp[ie] / wd[ie];
+        if (lane < 2) ex = exp(lane == 0 ? -grav * v.dx1f[ie] / (2 * RdTv) : -ent / gam);
         double top = 0.;
         if (lane == 0) {
-          const double RdTv = wp[ie] / wd[ie];
-          top = wp[ie] * exp(-grav * v.dx1f[ie] / (2 * RdTv));
+          top = wp[ie] * ex;
           psf[ie + 1] = top;
+        }
+        if (lane == 1) {
+          s_igam[c] = 1. / gam;
+          s_expf[c] = ex;
         }
         top = __shfl_sync(0xffffffffu, top, 0);
         double run = top + above;
@@ -876,66 +941,57 @@ __device__ __forceinline__ void flux_x1_block(const DevView& v, unsigned blk) {
           psf[m] = run;
         }
         __syncwarp();
-        if (lane == 0) {
-          for (int i = 1; i <= G; ++i) psf[is - i] = psf[is + i];
-          for (int i = 1; i <= G; ++i) psf[ie + i + 1] = psf[ie + 1 - i];
-          double gammad = v.gamma, fsig = 1., feps = 1.;
-          double gam = 1. + (gammad - 1.) * feps / fsig;
-          double ent = log(wp[is]) - gam * log(wd[is]);
-          s_gam[c] = gam;
-          s_expf[c] = exp(-ent / gam);
-        }
+        if (lane < G) psf[is - 1 - lane] = psf[is + 1 + lane];
+        __syncwarp();
+        if (lane < G) psf[ie + 2 + lane] = psf[ie - lane];
       }
     }
 #else
-    // one thread per column for the downward scan
-    if ((int)threadIdx.x < ncb) {
-      const int c = threadIdx.x;
-      double* wc = WC(c);
-      double* psf = PSF(c);
+    // one thread per column for the downward scan over the layers' weights,
+    // another warp's for the isentrope of the lowest cell
+    if (warp == 0 && lane < ncb) {
+      double* psf = PSF(lane);
+      const double* wd = WD(lane);
+      const double* wp = WP(lane);
       double grav = -v.grav;
-      int is = v.is, ie = v.ie;
-      double* wd = wc + IDN * nc1;
-      double* wp = wc + IPR * nc1;
       double RdTv = wp[ie] / wd[ie];
-      psf[ie + 1] = wp[ie] * exp(-grav * v.dx1f[ie] / (2 * RdTv));
-      for (int i = ie; i >= is; --i) psf[i] = psf[i + 1] + grav * wd[i] * v.dx1f[i];
+      double run = wp[ie] * exp(-grav * v.dx1f[ie] / (2 * RdTv));
+      psf[ie + 1] = run;
+#pragma unroll 8
+      for (int i = ie; i >= is; --i) {
+        run = run + psf[i];
+        psf[i] = run;
+      }
       for (int i = 1; i <= G; ++i) psf[is - i] = psf[is + i];
       for (int i = 1; i <= G; ++i) psf[ie + i + 1] = psf[ie + 1 - i];
+    }
+    if (warp == (nwarps > 1 ? 1 : 0) && lane < ncb) {
       double gammad = v.gamma, fsig = 1., feps = 1.;
       double gam = 1. + (gammad - 1.) * feps / fsig;
-      double ent = log(wp[is]) - gam * log(wd[is]);
-      s_gam[c] = gam;
-      s_expf[c] = exp(-ent / gam);
+      double ent = log(WP(lane)[is]) - gam * log(WD(lane)[is]);
+      s_igam[lane] = 1. / gam;
+      s_expf[lane] = exp(-ent / gam);
     }
 #endif
     __syncthreads();
-    const float inv_nc1 = 1.f / (float)nc1;
 #if EXO_MIXED
     // FP64 still, with the powers as exp(log(x) / gamma) and one log per face
     // shared by its two cells: ln psf and the face density of the isentropic
     // reference go to shared memory for the cells and for the restore
-    const float inv_f = 1.f / (float)(nc1 + 1);
-    for (int t = threadIdx.x; t < ncb * (nc1 + 1); t += blockDim.x) {
-      int c, i;
-      divmod_small(t, nc1 + 1, inv_f, c, i);
-      double* psf = PSF(c);
-      const double l = log(psf[i]);
-      psf[nc1 + 1 + i] = l;
-      psf[2 * (nc1 + 1) + i] = exp(l * (1. / s_gam[c])) * s_expf[c];
-    }
+    each([&](int c, int i) {
+      double* psf = PSF(c) + i;
+      const double l = log(psf[0]);
+      psf[per] = l;
+      psf[2 * per] = exp(l * s_igam[c]) * s_expf[c];
+    });
     __syncthreads();
-    for (int t = threadIdx.x; t < ncb * nc1; t += blockDim.x) {
-      int c, i;
-      divmod_small(t, nc1, inv_nc1, c, i);
-      double* wc = WC(c);
-      const double* psf = PSF(c);
-      const double* lpsf = psf + nc1 + 1;
-      const double* dsf = psf + 2 * (nc1 + 1);
-      const double igam = 1. / s_gam[c];
+    each([&](int c, int i) {
+      if (i >= nc1) return;
+      const double* psf = PSF(c) + i;
+      const double igam = s_igam[c];
       double psv, dsv;
-      if (fabs(psf[i] - psf[i + 1]) < 1.E-6) {
-        psv = (psf[i] + psf[i + 1]) * 0.5;
+      if (fabs(psf[0] - psf[1]) < 1.E-6) {
+        psv = (psf[0] + psf[1]) * 0.5;
         dsv = exp(log(psv) * igam) * s_expf[c];
       } else {
         // psv, the log-mean of the face pressures, is psf[i+1] (e^d - 1) / d
@@ -944,106 +1000,89 @@ __device__ __forceinline__ void flux_x1_block(const DevView& v, unsigned blk) {
         // e^((x + ln(sinh x / x)) / gamma): the face density times two short
         // series instead of a log and an exp (layers thinner than 0.4 scale
         // heights; thicker ones take the log and the exp)
-        const double d = lpsf[i] - lpsf[i + 1];
-        psv = (psf[i] - psf[i + 1]) / d;
+        const double d = psf[per] - psf[per + 1];
+        psv = (psf[0] - psf[1]) / d;
         const double x = 0.5 * d;
-        if (fabs(x) <= 0.2) dsv = dsf[i + 1] * exp_small((x + ln_sinhc(x)) * igam);
+        if (fabs(x) <= 0.2) dsv = psf[2 * per + 1] * exp_small((x + ln_sinhc(x)) * igam);
         else dsv = exp(log(psv) * igam) * s_expf[c];
       }
-      wc[IPR * nc1 + i] -= psv;
-      wc[IDN * nc1 + i] -= dsv;
-    }
+      T* f = WF(c) + i;
+      f[IPR * nc1] = T(WP(c)[i] - psv);
+      f[IDN * nc1] = T(WD(c)[i] - dsv);
+    });
 #else
-    for (int t = threadIdx.x; t < ncb * nc1; t += blockDim.x) {
-      int c, i;
-      divmod_small(t, nc1, inv_nc1, c, i);
-      double* wc = WC(c);
-      const double* psf = PSF(c);
+    each([&](int c, int i) {
+      if (i >= nc1) return;
+      const double* psf = PSF(c) + i;
       double psv, dsv;
-      if (fabs(psf[i] - psf[i + 1]) < 1.E-6)
-        psv = (psf[i] + psf[i + 1]) / 2.;
+      if (fabs(psf[0] - psf[1]) < 1.E-6)
+        psv = (psf[0] + psf[1]) / 2.;
       else
-        psv = (psf[i] - psf[i + 1]) / log(psf[i] / psf[i + 1]);
-      dsv = pow(psv, 1. / s_gam[c]) * s_expf[c];
-      wc[IPR * nc1 + i] -= psv;
-      wc[IDN * nc1 + i] -= dsv;
-    }
+        psv = (psf[0] - psf[1]) / log(psf[0] / psf[1]);
+      dsv = pow(psv, s_igam[c]) * s_expf[c];
+      WP(c)[i] -= psv;
+      WD(c)[i] -= dsv;
+    });
 #endif
     __syncthreads();
   }
   using TF = X1Flux<T>;
   TF* F = flux_array<TF>(v, 0);
-#if EXO_X1_SHARED_BETA
+#if EXO_MIXED
   // both face values of every cell is-1 .. ie+1, the cell's WENO5
-  // smoothness indicators computed once for the two (as the x2/x3 kernel
-  // does): rec [2][nv][L+2] floats of each column, after its psf arrays
-  const int ncell = L + 2;
-  auto REC = [&](int c) {
-    return reinterpret_cast<T*>(sm + (size_t)c * cstride + nv * nc1 + 3 * (nc1 + 1));
-  };
-  {
-    const float inv_nc = 1.f / (float)ncell;
-    for (int t = threadIdx.x; t < ncb * ncell; t += blockDim.x) {
-      int c, m;
-      divmod_small(t, ncell, inv_nc, c, m);
-      const int cell = v.is - 1 + m;
-      const double* wc = WC(c);
-      T* rec = REC(c);
+  // smoothness indicators computed once for the two (as the x2/x3 kernel does)
+  each([&](int c, int i) {
+    if (i >= ncell) return;
+    const T* q = WF(c) + is - 3 + i;
+    T* rec = REC(c) + i;
 #pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        if (n >= nv) break;
-        const double* q = wc + n * nc1 + cell;
-        const T q0 = T(q[-2]), q1 = T(q[-1]), q2 = T(q[0]), q3 = T(q[1]), q4 = T(q[2]);
-        const WenoCell<T> wcl = weno_cell<T>(q0, q1, q2, q3, q4);
-        rec[n * ncell + m] = weno_right<T>(wcl, q0, q1, q2, q3, q4);
-        rec[(nv + n) * ncell + m] = weno_left<T>(wcl, q0, q1, q2, q3, q4);
-      }
+    for (int n = 0; n < NV; ++n) {
+      const T q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4];
+      const WenoCell<T> wcl = weno_cell<T>(q0, q1, q2, q3, q4);
+      rec[0] = weno_right<T>(wcl, q0, q1, q2, q3, q4);
+      rec[NV * ncell] = weno_left<T>(wcl, q0, q1, q2, q3, q4);
+      q += nc1;
+      rec += ncell;
     }
-  }
+  });
   __syncthreads();
 #endif
-  const float inv_faces = 1.f / (float)(L + 1);
-  for (int t = threadIdx.x; t < ncb * (L + 1); t += blockDim.x) {
-    int c, f;
-    divmod_small(t, L + 1, inv_faces, c, f);
-    const double* wc = WC(c);
-    const double* psf = PSF(c);
-    const int i = v.is + f;
+  each([&](int c, int f) {
+    if (f > L) return;
+    const double* psf = PSF(c) + is + f;
     FaceGeo<TF> fg{TF(0.), TF(1.), TF(s_cthp[c]), TF(s_cosc[c])};
     // perturbations are formed in FP64 above; WENO5 runs in T, the restore in
     // FP64 and the Riemann solve in TF
-    TF wl[5], wr[5], fx[5] = {TF(0.), TF(0.), TF(0.), TF(0.), TF(0.)};
-#if EXO_X1_SHARED_BETA
-    {
-      const T* rec = REC(c);
+    TF wl[5], wr[5], fx[5];
+#if EXO_MIXED
+    const T* rec = REC(c) + f;
 #pragma unroll
-      for (int n = 0; n < 5; ++n) {
-        if (n >= nv) break;
-        wl[n] = TF(rec[n * ncell + f]);             // the upper face of cell i-1
-        wr[n] = TF(rec[(nv + n) * ncell + f + 1]);  // the lower face of cell i
-      }
+    for (int n = 0; n < NV; ++n) {
+      wl[n] = TF(rec[0]);               // the upper face of cell i-1
+      wr[n] = TF(rec[NV * ncell + 1]);  // the lower face of cell i
+      rec += ncell;
     }
 #else
-    #pragma unroll
-    for (int n = 0; n < 5; ++n) {
-      if (n >= nv) break;
-      const double* q = wc + n * nc1;
-      wl[n] = TF(weno_r<T>(q, 1, i - 1));
-      wr[n] = TF(weno_l<T>(q, 1, i));
+    const double* q = COL(c) + is + f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      wl[n] = weno_r<T>(q, 1, -1);
+      wr[n] = weno_l<T>(q, 1, 0);
+      q += nc1;
     }
 #endif
     if (decomp) {
       // RestoreFromPerturbation (change_to_perturbation.cpp:159-222), in FP64
-      double ps = psf[i];
+      double ps = psf[0];
       double xr = wr[IPR], xl = wl[IPR];
       xr += ps;
       if (xr < 0.) xr = ps;
       xl += ps;
       if (xl < 0.) xl = ps;
 #if EXO_MIXED
-      const double dsf = psf[2 * (nc1 + 1) + i];
+      const double dsf = psf[2 * per];
 #else
-      double dsf = pow(ps, 1. / s_gam[c]) * s_expf[c];
+      double dsf = pow(ps, s_igam[c]) * s_expf[c];
 #endif
       double dr = wr[IDN], dl = wl[IDN];
       dr += dsf;
@@ -1056,15 +1095,15 @@ __device__ __forceinline__ void flux_x1_block(const DevView& v, unsigned blk) {
       wl[IDN] = TF(dl);
     }
     // x1 runs for the ideal gas only: LMARS or HLLC
-    if (v.rsolver == EXO_RS_HLLC) riemann_hllc<TF>(v.gamma, IVX, fg, wl, wr, fx);
-    else riemann_lmars<TF>(v.gamma, IVX, wl, wr, fx);
-    TF* Fc = F + (size_t)s_base[c] + i;
-    #pragma unroll
-    for (int n = 0; n < 5; ++n) {
-      if (n >= nv) break;
-      Fc[n * vs] = fx[n];
+    if (v.rsolver == EXO_RS_HLLC) riemann_hllc<TF>(riemann_gas<TF>(v.gas), IVX, fg, wl, wr, fx);
+    else riemann_lmars<TF>(riemann_gas<TF>(v.gas), IVX, wl, wr, fx);
+    TF* out = F + s_base[c] + f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      *out = fx[n];
+      out += vs;
     }
-  }
+  });
 }
 
 // ----------------------------------------------------------- k_flux_x23 --
@@ -1140,7 +1179,7 @@ __device__ __forceinline__ void cp_async_wait_one() {
 // the FP64 pipe (FP64 build, 62 % busy), not memory (16 % and 11 % of DRAM).
 // Per launch, before (32 radial indices of one line per block, or one thread
 // per face where those left lanes idle; FP64 also through shared memory) and
-// now: FP64 48^2x3 33.1 -> 23.1 us, 40^2x40 145 -> 116, 96^2x64 695 -> 616;
+// now: FP64 48^2x3 33.1 -> 23.1 us, 40^2x40 145 -> 105, 96^2x64 695 -> 575;
 // mixed 24^2x32 26 -> 19, 62^2x45 143 -> 96, 126^2x70 595 -> 447, 192^2x96
 // 1115 -> 1104.
 #ifndef EXO_X23_THREADS
@@ -1159,8 +1198,8 @@ template <class T, bool kShareBeta>
 __host__ __device__ constexpr int x23_chunk() {
   return kShareBeta ? 15 : sizeof(T) == 4 ? 16 : 8;
 }
-// resident blocks per SM (launch bounds, or the registers it keeps)
-constexpr unsigned X23_RESIDENT = EXO_MIXED ? 4 : 3;
+// resident blocks per SM (128 registers a thread)
+constexpr unsigned X23_RESIDENT = 4;
 
 // cp.async of 4 or 8 bytes, zero-filled when src_bytes is 0
 template <int B>
@@ -1220,7 +1259,6 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X2
   const int q0 = (int)(seg * sp.chunks);
   const int q1 = min((N + CF) / CF, q0 + (int)sp.chunks);
   const int rsolver = v.rsolver;
-  const double gamma = v.gamma;
   // copies of the cells [m0, m0 + n), the first of them in slot slot0
   auto issue = [&](int m0, int n, int slot0) {
 #pragma unroll 1
@@ -1309,14 +1347,14 @@ __device__ __forceinline__ void flux_x23_pipe(const DevView& v, unsigned blk, X2
         const int k = v.ks + a, j = v.js + f;
         FaceGeo<T> fg{T(geo(v, GCOSF2, p, k, j)), T(geo(v, GSINF2, p, k, j)),
                       T(geo(v, GCTHP2, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-        riemann<T>(rsolver, gamma, IVY, fg, wl, wr, fx);
+        riemann<T>(rsolver, v.gas, IVY, fg, wl, wr, fx);
       } else {
         if (f == 0) edge_outer_state<T>(v, p, LEFT, a, i, wl);
         else if (f == N) edge_outer_state<T>(v, p, RIGHT, a, i, wr);
         const int k = v.ks + f, j = v.js + a;
         FaceGeo<T> fg{T(geo(v, GCOSF3, p, k, j)), T(geo(v, GSINF3, p, k, j)),
                       T(geo(v, GCTHP3, p, k, j)), T(geo(v, GCOSC, p, k, j))};
-        riemann<T>(rsolver, gamma, IVZ, fg, wl, wr, fx);
+        riemann<T>(rsolver, v.gas, IVZ, fg, wl, wr, fx);
       }
       T* out = F + (size_t)f * s;
 #pragma unroll
@@ -3011,8 +3049,9 @@ __global__ void EXO_PRIM_BOUNDS kb_prim_ghost(Batch bt, int compute_dt) {
   prim_ghost_block(sv, b, compute_dt);
 }
 
-// The x1 kernel is latency bound (a thread per column walks the hydrostatic
-// scan while the others wait): occupancy beats registers, measured
+// 48 registers and 100 bytes of spill (mixed, 96^2x64: 261 us; 64 and 72
+// registers, a block fewer on each SM: 310; 40 gains 3 % there and loses 10 %
+// at 24^2x32)
 #ifndef EXO_X1_MAXNREG
 #define EXO_X1_MAXNREG 48
 #endif
@@ -3200,7 +3239,7 @@ int launch_reciprocal(int n, const double* x, double* out, void* stream) {
 // Lines are cut into segments where one segment per line would fill the last
 // wave of blocks badly: the count of segments whose waves x length is least,
 // a segment's length being its chunks and half a chunk for the first cells'
-// way in.  (FP64, N = 40, 40 levels, 600 lines' blocks for 444 places: one
+// way in.  (FP64, N = 40, 40 levels, 600 blocks of whole lines: one
 // segment 135 us, two 116; N = 48, 3 levels, 60 blocks: seven segments.)
 X23Split x23_split(int N, int L) {
   using T = EXO_FLUX_T;

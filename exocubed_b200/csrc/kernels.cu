@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(BWD_THREADS) k_implicit_columns_bwd(int ncol, 
   implicit_bwd_group<double, full ? 5 : 3, false>(g, bws);
 }
 
-__global__ void k_riemann_rows(int rsolver, int eqn, int ivx, int n, double gamma,
+__global__ void k_riemann_rows(int rsolver, int eqn, int ivx, int n, RiemannGas<double> gas,
                                const double* wl, const double* wr, double* flx,
                                const double* cosf, const double* sinf, const double* cthp,
                                const double* cthc) {
@@ -104,7 +104,7 @@ __global__ void k_riemann_rows(int rsolver, int eqn, int ivx, int n, double gamm
   double a[5] = {0, 0, 0, 0, 0}, b[5] = {0, 0, 0, 0, 0}, f[5] = {0, 0, 0, 0, 0};
   for (int q = 0; q < nv; ++q) { a[q] = wl[(size_t)q * n + m]; b[q] = wr[(size_t)q * n + m]; }
   FaceGeo<double> fg{cosf ? cosf[m] : 0., sinf ? sinf[m] : 1., cthp ? cthp[m] : 0., cthc ? cthc[m] : 0.};
-  riemann<double>(rsolver, gamma, ivx, fg, a, b, f);
+  riemann<double>(rsolver, gas, ivx, fg, a, b, f);
   for (int q = 0; q < nv; ++q) flx[(size_t)q * n + m] = f[q];
 }
 
@@ -499,7 +499,7 @@ int launch_riemann_rows(int rsolver, int eqn, int ivx, int n, double gamma, cons
                         const double* cthp, const double* cthc, void* stream) {
   if (n <= 0) return 0;
   fp64::k_riemann_rows<<<fp64::nblk(n, 128), 128, 0, (cudaStream_t)stream>>>(
-      rsolver, eqn, ivx, n, gamma, wl, wr, flx, cosf, sinf, cthp, cthc);
+      rsolver, eqn, ivx, n, make_riemann_gas(gamma), wl, wr, flx, cosf, sinf, cthp, cthc);
   return fp64::check_launch();
 }
 

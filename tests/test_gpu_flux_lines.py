@@ -1,7 +1,7 @@
-"""The x2/x3 fluxes at the sizes where their lines, chunks and segments can go
-wrong (lines that fill no group of 32, faces one past a chunk, one and several
-chunks per segment, four variables, both ways of the mixed reconstruction),
-and WENO5 where its divisions leave the unchecked path."""
+"""The fluxes at the sizes where their lines, chunks and segments can go
+wrong (x2/x3: lines that fill no group of 32, faces one past a chunk, one and several
+chunks per segment, four variables, both ways of the mixed reconstruction; x1: columns
+per block), and WENO5 where its divisions leave the unchecked path."""
 import numpy as np
 import pytest
 
@@ -26,7 +26,7 @@ def _faces(a, d, N, L):
 # a wrong cell's velocity of some m/s against c = 300 m/s is 5e-5.
 @pytest.mark.parametrize("setup,N,L", [
     ("dry", 6, 1), ("dry", 6, 9), ("dry", 6, 16), ("dry", 14, 33), ("dry", 16, 45),
-    ("dry", 30, 31), ("dry", 32, 40), ("dry", 16, 100), ("dry", 30, 96),
+    ("dry", 30, 31), ("dry", 32, 40), ("dry", 16, 100), ("dry", 30, 96), ("dry", 6, 250),
     ("shallow", 6, 5), ("shallow", 8, 32), ("shallow", 16, 3), ("shallow", 30, 70)])
 def test_horizontal_fluxes_match_the_oracle(oracle_mod, setup, N, L):
     if setup == "dry":
@@ -56,6 +56,28 @@ def test_horizontal_fluxes_match_the_oracle(oracle_mod, setup, N, L):
     for n in (0, 4) if setup == "dry" else (0,):
         err = np.abs(got[:, n] / want[:, n] - 1.).max()
         assert err < 1e-6, (n, err)
+
+
+# The decomposition's log, exp and pow are the device's: 1e-11 of the largest
+# flux, as for any FP64 x1 flux (columns that fill their block, that leave a
+# warp idle, and blocks of more places than threads).
+@pytest.mark.parametrize("rsolver", [nat.EXO_RS_LMARS, nat.EXO_RS_HLLC])
+@pytest.mark.parametrize("L,columns", [(3, 4), (25, 8), (25, 1), (57, 4), (250, 4), (250, 5),
+                                       (121, 8)])
+def test_vertical_fluxes_match_the_oracle(oracle_mod, rsolver, L, columns):
+    N = 6
+    cfg = W.dry_atmosphere_config(N=N, L=L, rsolver=rsolver)
+    o = oracle_mod.Oracle(cfg)
+    o.set_primitive(W.dry_atmosphere_state(cfg, seed=L))
+    o.calculate_fluxes()
+    want = o.flux(0)[:, :, G:G + N, G:G + N, G:G + L + 1]
+    with CubedSphereAtmosphere(cfg) as g:
+        g.set_tiles([columns, 0, 0, 0, 0, 0])
+        g.set_primitive(W.dry_atmosphere_state(cfg, seed=L))
+        g.calculate_fluxes()
+        got = g.flux(0)[:, :, G:G + N, G:G + N, G:G + L + 1]
+    scale = np.abs(want).max(axis=(0, 2, 3, 4), keepdims=True)
+    assert (np.abs(got - want) / scale).max() < 1e-11
 
 
 def test_weno5_outside_the_unchecked_divisions_bitwise(oracle_mod, native):
