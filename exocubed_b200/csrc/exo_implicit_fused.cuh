@@ -2,12 +2,17 @@
 // back substitution in the same kernel (textually part of exo_kernels.cuh).
 //
 // The same algorithm as implicit_column and kb_implicit_bwd, in the form it
-// had before those two were split and their loads moved to warp tiles.  The
-// split form is faster (6x96^2x64: 764 against 867 us a solve alone; with the
-// blocks kept by their structure 617), but compiled with fused
-// multiply-adds it does not round as this one does: the last bits of u it
-// changes reach the FP32 copy of the primitives, and a run differs by 1e-7
-// within some tens of steps.  FP32 blocks, the 3x3 blocks and the FP64 build,
+// had before those two were split.  The split form is a little faster
+// (6x96^2x64: 764 against 788 us a solve; with the blocks kept by their
+// structure 617), but compiled with fused multiply-adds it does not round as
+// this one does: the last bits of u it changes reach the FP32 copy of the
+// primitives, and a run differs by 1e-7 within some tens of steps.  (The
+// boundary terms as branches, 752 us, change the roundings too.)  Its forward
+// sweep's loads by warp tiles and the swaps' branches taken by the warp are
+// 867 -> 788 us there, 4112 -> 4088 at 6x192^2x96, where the scratch's traffic
+// (480 of 640 bytes a level and column, 2.1 ms at the copy rate) weighs more.
+// More warps do not help (200 registers, ten warps: the same; 168: twice the
+// time, the lines of L1 in flight being what limits them).  FP32 blocks, the 3x3 blocks and the FP64 build,
 // whose results the split form leaves to the bit, take the split form.
 
 // Solve with the LU factors of implicit_column's mixed build (rows taken in
@@ -53,25 +58,23 @@ __device__ __forceinline__ void lu_solve_swapped(const R (&t)[5][5], const R (&i
 // a column for one variable in one 32-byte run (the per-lane accesses of
 // one level are 816 bytes apart, a sector each), the next chunk's copies in
 // flight while a chunk is corrected.  The factors are read per lane, one
-// level ahead, as in implicit_backward_full (they are contiguous across the
-// warp).  io.live: the lanes of the warp with a column.  wtile: 2 x 5 x 32 x
-// (BWD_TL + 1) doubles of shared memory for the warp alone.
+// level ahead (they are contiguous across the warp).  io.live: the lanes of
+// the warp with a column.  wtile: 2 x 5 x 32 x (BWD_TL + 1) doubles of shared
+// memory for the warp alone.
 constexpr int BWD_TL = 4;
 // the two u tiles of a warp's back substitution (5 variables x 32 columns x
 // BWD_TL levels, padded)
 constexpr int WARP_TILE_DOUBLES = 2 * 5 * 32 * (BWD_TL + 1);
-// shared doubles per thread: two face matrices, w and du of the next level
-constexpr int IMPL_SM_STRIDE = 61;
-static_assert(32 * IMPL_SM_STRIDE >= WARP_TILE_DOUBLES,
-              "the tiled back substitution's buffers fit in the warp's slices");
-// NB = 5: the full correction (30 factors per level, delta on every
-// variable); NB = 3: the partial one (12 factors per level, delta on rho,
-// m1 and E, the explicit du on m2 and m3, read per lane one level ahead).
-template <int NB, class IO>
+// a warp's shared memory: the level tile, then two face matrices per lane
+// (entry e of lane l at [e * 32 + l])
+constexpr int FUSED_WARP_DOUBLES = LEVEL_TILE_DOUBLES + 50 * 32;
+static_assert(FUSED_WARP_DOUBLES >= WARP_TILE_DOUBLES,
+              "the tiled back substitution's buffers fit in the warp's memory");
+template <class IO>
 __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
                                                         typename IO::Real* dp, double* wtile) {
   static_assert(BWD_TL == 4, "the lane -> (column, level) split below assumes 4 levels");
-  static_assert(NB == 5 || NB == 3, "5x5 or 3x3 blocks");
+  constexpr int NB = 5;
   constexpr int NF = NB * NB + NB;  // factors per level: (A c)_i and delta_i
   constexpr int TS = BWD_TL + 1;
   constexpr int TW = 5 * 32 * TS;
@@ -84,7 +87,7 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
 #pragma unroll
   for (int m = 0; m < 4; ++m)
     ub[m] = reinterpret_cast<double*>(__shfl_sync(
-        live, reinterpret_cast<unsigned long long>(io.uc), ((lane >> 2) + 8 * m) & 31));
+        live, reinterpret_cast<unsigned long long>(io.xc), ((lane >> 2) + 8 * m) & 31));
   const int l = lane & 3;
   const int nch = (ie - is + BWD_TL) / BWD_TL;
   auto range = [&](int c, int& lo, int& hi) {
@@ -110,7 +113,7 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
 #pragma unroll
       for (int e = 0; e < 20; ++e) {
         const int ll = e & 3, n = e >> 2;
-        if (lo + ll <= hi) cp_async8(&t[(n * 32 + lane) * TS + ll], io.uc + n * io.vs + lo + ll);
+        if (lo + ll <= hi) cp_async8(&t[(n * 32 + lane) * TS + ll], io.xc + n * io.vs + lo + ll);
       }
     }
     cp_async_commit();
@@ -118,25 +121,11 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
   load(0);
   if (nch > 1) load(1);
   using R = typename IO::Real;
-  // the factors of the next level (cur_s) and, with 1 2, of the
-  // one after (ahd_s): their loads are in flight for two levels (the
-  // registers of the finished forward sweep are free)
-  R cur_s[NF], ahd_s[NF];
+  // the factors of the next level, in flight while a level is corrected
+  R cur_s[NF];
   if (ie > is) {
 #pragma unroll
     for (int e = 0; e < NF; ++e) cur_s[e] = io.scr(ie - 1 - is, e);
-  }
-  if constexpr (false) {
-    if (ie - 1 > is) {
-#pragma unroll
-      for (int e = 0; e < NF; ++e) ahd_s[e] = io.scr(ie - 2 - is, e);
-    }
-  }
-  // the partial correction's explicit du of m2 and m3, one level ahead
-  double cur_du[2] = {0., 0.};
-  if constexpr (NB == 3) {
-    cur_du[0] = *io.duptr(ie, IVY);
-    cur_du[1] = *io.duptr(ie, IVZ);
   }
   for (int c = 0; c < nch; ++c) {
     if (c + 1 < nch) cp_async_wait_one();
@@ -146,13 +135,6 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
     int lo, hi;
     range(c, lo, hi);
     for (int i = hi; i >= lo; --i) {
-      double nxt_du[2] = {0., 0.};
-      if constexpr (NB == 3) {
-        if (i > is) {
-          nxt_du[0] = *io.duptr(i - 1, IVY);
-          nxt_du[1] = *io.duptr(i - 1, IVZ);
-        }
-      }
       if (i < ie) {
         R nxt_s[NF];
         const int ahead = i - 1;  // the level whose factors load now
@@ -170,34 +152,13 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
         }
 #pragma unroll
         for (int r = 0; r < NB; ++r) dp[r] = dl[r];
-        if constexpr (false) {
 #pragma unroll
-          for (int e = 0; e < NF; ++e) {
-            cur_s[e] = ahd_s[e];
-            ahd_s[e] = nxt_s[e];
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < NF; ++e) cur_s[e] = nxt_s[e];
-        }
+        for (int e = 0; e < NF; ++e) cur_s[e] = nxt_s[e];
       }
       // the corrected update of every variable
-      double d[5];
-      if constexpr (NB == 5) {
-#pragma unroll
-        for (int n = 0; n < 5; ++n) d[n] = dp[n];
-      } else {
-        d[IDN] = dp[0];
-        d[IVX] = dp[1];
-        d[IVY] = cur_du[0];
-        d[IVZ] = cur_du[1];
-        d[IEN] = dp[2];
-        cur_du[0] = nxt_du[0];
-        cur_du[1] = nxt_du[1];
-      }
       double uu[5];
 #pragma unroll
-      for (int n = 0; n < 5; ++n) uu[n] = t[(n * 32 + lane) * TS + (i - lo)] + 1. * d[n];
+      for (int n = 0; n < 5; ++n) uu[n] = io.stage < 0 ? dp[n] : t[(n * 32 + lane) * TS + (i - lo)] + 1. * dp[n];
       if (io.stage == 2) airparcel_round_trip(uu, io.Rd, io.gamma);
 #pragma unroll
       for (int n = 0; n < 5; ++n) t[(n * 32 + lane) * TS + (i - lo)] = uu[n];
@@ -215,7 +176,7 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
 #pragma unroll
       for (int e = 0; e < 20; ++e) {
         const int ll = e & 3, n = e >> 2;
-        if (lo + ll <= hi) io.uc[n * io.vs + lo + ll] = t[(n * 32 + lane) * TS + ll];
+        if (lo + ll <= hi) io.xc[n * io.vs + lo + ll] = t[(n * 32 + lane) * TS + ll];
       }
     }
     __syncwarp(live);
@@ -223,95 +184,12 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
   }
 }
 
-// BackwardSubstitution of the full correction (forward_backward.hpp:90-126):
-// delta_i -= (A c)_i delta_{i+1} from level ie (delta_ie given in dp) down
-// to is, each corrected update stored through io.  kPipe: software-pipelined,
-// the next level's factors and state in flight while a level finishes (for
-// the few resident columns of the solve kernel); otherwise one level at a
-// time, leaving the latency to the many columns of the back-substitution
-// kernel.
-template <class IO, bool kPipe = true>
-__device__ __forceinline__ void implicit_backward_full(IO& io, int is, int ie,
-                                                       typename IO::Real* dp) {
-  using R = typename IO::Real;
-  auto store = [&](int i, const double* u) {
-    double d[5];
-#pragma unroll
-    for (int n = 0; n < 5; ++n) d[n] = dp[n];
-    io.ustore(i, u, d);
-  };
-  if constexpr (!kPipe) {
-    {
-      double u[5];
-      io.uload(ie, u);
-      store(ie, u);
-    }
-#pragma unroll 1
-    for (int i = ie - 1; i >= is; --i) {
-      R cs[30];
-      double u[5];
-#pragma unroll
-      for (int e = 0; e < 30; ++e) cs[e] = io.scr(i - is, e);
-      io.uload(i, u);
-      R dl[5];
-#pragma unroll
-      for (int r = 0; r < 5; ++r) {
-        R ad = cs[r * 5] * dp[0];
-#pragma unroll
-        for (int k = 1; k < 5; ++k) ad += cs[r * 5 + k] * dp[k];
-        dl[r] = cs[25 + r] - ad;
-      }
-#pragma unroll
-      for (int r = 0; r < 5; ++r) dp[r] = dl[r];
-      store(i, u);
-    }
-    return;
-  }
-  R cur_s[30];
-  double cur_u[5];
-  io.uload(ie, cur_u);
-  store(ie, cur_u);
-  if (ie > is) {
-#pragma unroll
-    for (int e = 0; e < 30; ++e) cur_s[e] = io.scr(ie - 1 - is, e);
-    io.uload(ie - 1, cur_u);
-  }
-#pragma unroll 1
-  for (int i = ie - 1; i >= is; --i) {
-    R nxt_s[30];
-    double nxt_u[5];
-    if (i > is) {
-#pragma unroll
-      for (int e = 0; e < 30; ++e) nxt_s[e] = io.scr(i - 1 - is, e);
-      io.uload(i - 1, nxt_u);
-    }
-    R dl[5];
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      R ad = cur_s[r * 5] * dp[0];
-#pragma unroll
-      for (int k = 1; k < 5; ++k) ad += cur_s[r * 5 + k] * dp[k];
-      dl[r] = cur_s[25 + r] - ad;
-    }
-#pragma unroll
-    for (int r = 0; r < 5; ++r) dp[r] = dl[r];
-    store(i, cur_u);
-    if (i > is) {
-#pragma unroll
-      for (int e = 0; e < 30; ++e) cur_s[e] = nxt_s[e];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) cur_u[n] = nxt_u[n];
-    }
-  }
-}
-
 template <class IO>
-__device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real* sa, double* sp, int ss,
+__device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real* sa, int ss, double* tile,
                                                 double cos_theta, double sin_theta, double d2,
                                                 double d3, const double* x1f, const double* x1v,
                                                 const double* dx1f, int is, int ie, double dt,
-                                                double gamma, double grav,
-                                                double* wt = nullptr) {
+                                                double gamma, double grav, double* wt) {
   using R = typename IO::Real;
   using ColCell = exo::EXO_KNS::ColCell<R>;
   const double s = sin_theta;
@@ -341,24 +219,31 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
   };
   auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 25 + r * 5 + q) * ss]; };
 
-  // prefetch slots: w(i+1) and du(i) of the next level, copied asynchronously
-  auto pw = [&](int n) -> double& { return sp[n * ss]; };
-  auto pdu = [&](int n) -> double& { return sp[(5 + n) * ss]; };
-  auto prefetch = [&](int iw, int idu) {
+  // w(i+1) and du(i), four levels at a time by the whole warp; the last warp
+  // of a member, where some lanes have no column, copies per lane
+  LevelTile<IO, 5> lt(io, tile, is, ie - is + 1);
+  auto ready = [&](int k0) {
+    if (io.live == 0xffffffffu) {
+      lt.ready(io, k0);
+    } else if ((k0 & 3) == 0) {
+      __syncwarp(io.live);
+      for (int k = k0; k < min(k0 + 4, ie - is + 1); ++k) {
 #pragma unroll
-    for (int n = 0; n < 5; ++n) cp_async8(&pw(n), io.wptr(iw, n));
-    if (idu >= 0) {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) cp_async8(&pdu(n), io.duptr(idu, n));
+        for (int n = 0; n < 5; ++n) {
+          cp_async8(lt.place(n, k), io.wptr(is + 1 + k, n));
+          cp_async8(lt.place(5 + n, k), io.duptr(is + k, n));
+        }
+      }
+      cp_async_commit();
+      cp_async_wait_all();
+      __syncwarp(io.live);
     }
-    cp_async_commit();
   };
   double raw[5];
   io.w(is - 1, raw);
   ColCell cm = cell(raw);
   io.w(is, raw);
   ColCell c0 = cell(raw);
-  prefetch(is + 1, is);
   {
     R A[5][5];
     abs_jacobian(cm, c0, gm1, gam, A);
@@ -371,15 +256,14 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
   R dp[5];  // delta_{i-1}
   int cur = 0;
   for (int i = is; i <= ie; ++i) {
-    cp_async_wait_all();
+    ready(i - is);
     double rhs[5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      raw[n] = pw(n);
-      rhs[n] = pdu(n);
+      raw[n] = lt.get(n, i - is);
+      rhs[n] = lt.get(5 + n, i - is);
     }
     ColCell cp = cell(raw);
-    prefetch(i + 2, i < ie ? i + 1 : -1);
     const int nxt = cur ^ 1;
     {
       R A[5][5];
@@ -473,9 +357,13 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
           const R m = abs_r(t[O[r]][k]);
           if (m > best) { best = m; piv = r; }
         }
-        if (dk < R(0.1) * best) {
+        const bool take = dk < R(0.1) * best;
+        if (!take) piv = k;
+        perm |= (unsigned)piv << (3 * k);
+        // the warp decides: as a lane's own branch the swaps become selects
+        // that every level pays for
+        if (__any_sync(io.live, take)) {
           swapped = true;
-          perm |= (unsigned)piv << (3 * k);
 #pragma unroll
           for (int r = k + 1; r < 5; ++r) {
             const bool sw = (piv == r);
@@ -486,8 +374,6 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
               t[O[r]][q] = sw ? a : b;
             }
           }
-        } else {
-          perm |= (unsigned)k << (3 * k);
         }
       }
       idg[k] = inv_r(t[O[k]][k]);
@@ -511,38 +397,27 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
     });
 #pragma unroll
     for (int r = 0; r < 5; ++r) dp[r] = x[r];
-    const int lev = i - is;
+    R* const sl = &io.scr(i - is, 0);
     if (!last) {
 #pragma unroll
       for (int r = 0; r < 5; ++r)
 #pragma unroll
-        for (int q = 0; q < 5; ++q) io.scr(lev, r * 5 + q) = Ap[r][q];
+        for (int q = 0; q < 5; ++q) sl[(r * 5 + q) * 32] = Ap[r][q];
 #pragma unroll
-      for (int r = 0; r < 5; ++r) io.scr(lev, 25 + r) = dp[r];
+      for (int r = 0; r < 5; ++r) sl[(25 + r) * 32] = dp[r];
     }
     cm = c0;
     c0 = cp;
     cur = nxt;
   }
-  // the last level's prefetch (unused) must land before the back substitution
-  // reuses this thread's slots of shared memory
-  cp_async_wait_all();
-  if constexpr (IO::kLoadsU && sizeof(R) == 8) {
-    if (io.stage >= 0) {
-      // the warp's tiles (FP64 blocks: its 32 shared slices, free once every
-      // lane has finished its forward sweep)
-      implicit_backward_tiled<5>(io, is, ie, dp, wt);
-      return;
-    }
-  }
-  implicit_backward_full(io, is, ie, dp);
+  // the warp's shared memory, free once every lane has finished its forward
+  // sweep, holds the back substitution's tiles
+  implicit_backward_tiled(io, is, ie, dp, wt);
 }
 
-// this thread's slices of the block's shared memory: each thread's doubles
-// contiguous, IMPL_SM_STRIDE doubles apart (odd, so that a half-warp's 8-byte
-// accesses fall on distinct banks), then the radial tables
+// shared memory: FUSED_WARP_DOUBLES for each warp, then the radial tables
 constexpr size_t fused_smem(int threads, int nc1) {
-  return ((size_t)IMPL_SM_STRIDE * threads + 3 * (size_t)(nc1 + 1)) * sizeof(double);
+  return ((size_t)FUSED_WARP_DOUBLES * (threads / 32) + 3 * (size_t)(nc1 + 1)) * sizeof(double);
 }
 
 // A column of the stepping context: primitives and update from the state
@@ -553,41 +428,23 @@ struct FusedColumnIO {
   using Real = R;
   const double* wc;
   const double* duc;
-  double* uc;
+  double* xc;      // what is corrected: u, or for stage < 0 du
   size_t vs;       // stride between variables
   R* scr0;         // scratch of this column: [level][entry][32 lanes] per warp of columns
-  int stage;            // < 0: write the corrected update into du, leave u alone
+  int stage;       // < 0: write the corrected update into du, leave u alone
   double Rd, gamma;
-  double* duw;          // du of this column, for stage < 0
   __device__ __forceinline__ void w(int i, double* out) const {
 #pragma unroll
     for (int n = 0; n < 5; ++n) out[n] = wc[n * vs + i];
   }
+  __device__ __forceinline__ size_t wstride() const { return vs; }
+  __device__ __forceinline__ size_t dstride() const { return vs; }
   __device__ __forceinline__ const double* wptr(int i, int n) const { return wc + n * vs + i; }
   __device__ __forceinline__ const double* duptr(int i, int n) const { return duc + n * vs + i; }
   __device__ __forceinline__ R& scr(int lev, int e) const {
     return scr0[(lev * 30 + e) * 32];
   }
-  static constexpr bool kLoadsU = true;
-  unsigned live = 0xffffffffu;  // the lanes of the warp with a column
-  __device__ __forceinline__ void uload(int i, double* u) const {
-    if (stage < 0) return;
-#pragma unroll
-    for (int n = 0; n < 5; ++n) u[n] = uc[n * vs + i];
-  }
-  __device__ __forceinline__ void ustore(int i, const double* u, const double* dl) const {
-    if (stage < 0) {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) duw[n * vs + i] = dl[n];
-      return;
-    }
-    double uu[5];
-#pragma unroll
-    for (int n = 0; n < 5; ++n) uu[n] = u[n] + 1. * dl[n];
-    if (stage == 2) airparcel_round_trip(uu, Rd, gamma);
-#pragma unroll
-    for (int n = 0; n < 5; ++n) uc[n * vs + i] = uu[n];
-  }
+  unsigned live;   // the lanes of the warp with a column
 };
 
 
@@ -602,7 +459,7 @@ __device__ __forceinline__ void implicit_fused_block(const DevView& v, unsigned 
   const double* x1f;
   const double* x1v;
   const double* dx1f;
-  stage_radial(ism + blockDim.x * IMPL_SM_STRIDE, v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
+  stage_radial(ism + (blockDim.x >> 5) * FUSED_WARP_DOUBLES, v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
   const unsigned live = __ballot_sync(0xffffffffu, col < ncol);
   if (col >= ncol) return;
   const int j = v.js + col % v.N;
@@ -613,11 +470,11 @@ __device__ __forceinline__ void implicit_fused_block(const DevView& v, unsigned 
   // scratch in blocks of 32 columns: a warp's 32 entries are 128 (FP32) or
   // 256 (FP64) contiguous bytes
   R* scr0 = reinterpret_cast<R*>(v.scratch) + (size_t)(col >> 5) * v.L * 30 * 32 + (col & 31);
-  FusedColumnIO<R> io{v.w + base, v.du + base, v.u + base, v.cells, scr0, stage, v.Rd, v.gamma,
-                     v.du + base};
-  io.live = live;
-  double* const sm = ism + threadIdx.x * IMPL_SM_STRIDE;
-  implicit_column_fused(io, sm, sm + 50, 1, geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j),
-                        geo(v, GDX2A, p, k, j), geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is, v.ie,
-                        dt, v.gamma, v.grav, ism + (threadIdx.x & ~31u) * IMPL_SM_STRIDE);
+  FusedColumnIO<R> io{v.w + base, v.du + base, (stage < 0 ? v.du : v.u) + base, v.cells, scr0,
+                      stage,       v.Rd,        v.gamma,                          live};
+  double* const wt = ism + (threadIdx.x >> 5) * FUSED_WARP_DOUBLES;
+  implicit_column_fused(io, wt + LEVEL_TILE_DOUBLES + (threadIdx.x & 31), 32, wt,
+                        geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j), geo(v, GDX2A, p, k, j),
+                        geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is, v.ie, dt, v.gamma, v.grav,
+                        wt);
 }

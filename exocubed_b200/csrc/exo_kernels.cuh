@@ -1925,10 +1925,12 @@ struct LevelTile {
     cp_async_wait_all();
     __syncwarp();
   }
-  __device__ __forceinline__ double get(int n, int k) const {
+  // value n of level k of this lane's column
+  __device__ __forceinline__ double* place(int n, int k) const {
     const int lane = (int)(threadIdx.x & 31);
-    return tile[n * 128 + lane * 4 + ((k + (lane >> 2)) & 3)];
+    return tile + n * 128 + lane * 4 + ((k + (lane >> 2)) & 3);
   }
+  __device__ __forceinline__ double get(int n, int k) const { return *place(n, k); }
 };
 
 // shared memory of a warp of the solve: the level tile, then NE values of R
