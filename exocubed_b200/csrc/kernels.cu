@@ -94,18 +94,29 @@ __global__ void __launch_bounds__(BWD_THREADS) k_implicit_columns_bwd(int ncol, 
   implicit_bwd_group<double, full ? 5 : 3, false>(g, bws);
 }
 
-__global__ void k_riemann_rows(int rsolver, int eqn, int ivx, int n, RiemannGas<double> gas,
-                               const double* wl, const double* wr, double* flx,
-                               const double* cosf, const double* sinf, const double* cthp,
-                               const double* cthc) {
+// Solver and direction are the instantiation's: with them at run time the
+// states were indexed in local memory (120 bytes of stack; HLLC on 3.6 million
+// faces 167 us, now 107; its bytes at the copy rate 83)
+template <int kSolver, int kIvx>
+__global__ void k_riemann_rows(int nv, int n, RiemannGas<double> gas, const double* wl,
+                               const double* wr, double* flx, const double* cosf,
+                               const double* sinf, const double* cthp, const double* cthc) {
   int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= n) return;
-  int nv = eqn == EXO_EQN_SHALLOW_YZ ? 4 : 5;
   double a[5] = {0, 0, 0, 0, 0}, b[5] = {0, 0, 0, 0, 0}, f[5] = {0, 0, 0, 0, 0};
-  for (int q = 0; q < nv; ++q) { a[q] = wl[(size_t)q * n + m]; b[q] = wr[(size_t)q * n + m]; }
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    if (q >= nv) break;
+    a[q] = wl[(size_t)q * n + m];
+    b[q] = wr[(size_t)q * n + m];
+  }
   FaceGeo<double> fg{cosf ? cosf[m] : 0., sinf ? sinf[m] : 1., cthp ? cthp[m] : 0., cthc ? cthc[m] : 0.};
-  riemann<double>(rsolver, gas, ivx, fg, a, b, f);
-  for (int q = 0; q < nv; ++q) flx[(size_t)q * n + m] = f[q];
+  riemann<double>(kSolver, gas, kIvx, fg, a, b, f);
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    if (q >= nv) break;
+    flx[(size_t)q * n + m] = f[q];
+  }
 }
 
 __global__ void k_weno5(int n, const double* a, const double* b, const double* c,
@@ -498,8 +509,21 @@ int launch_riemann_rows(int rsolver, int eqn, int ivx, int n, double gamma, cons
                         const double* wr, double* flx, const double* cosf, const double* sinf,
                         const double* cthp, const double* cthc, void* stream) {
   if (n <= 0) return 0;
-  fp64::k_riemann_rows<<<fp64::nblk(n, 128), 128, 0, (cudaStream_t)stream>>>(
-      rsolver, eqn, ivx, n, make_riemann_gas(gamma), wl, wr, flx, cosf, sinf, cthp, cthc);
+  const int nv = eqn == EXO_EQN_SHALLOW_YZ ? 4 : 5;
+  auto run = [&](auto solver, auto dir) {
+    fp64::k_riemann_rows<decltype(solver)::value, decltype(dir)::value>
+        <<<fp64::nblk(n, 128), 128, 0, (cudaStream_t)stream>>>(
+            nv, n, make_riemann_gas(gamma), wl, wr, flx, cosf, sinf, cthp, cthc);
+  };
+  auto along = [&](auto solver) {
+    if (ivx == IVX) run(solver, std::integral_constant<int, IVX>{});
+    else if (ivx == IVY) run(solver, std::integral_constant<int, IVY>{});
+    else run(solver, std::integral_constant<int, IVZ>{});
+  };
+  if (rsolver == EXO_RS_ROE_SHALLOW) along(std::integral_constant<int, EXO_RS_ROE_SHALLOW>{});
+  else if (rsolver == EXO_RS_LMARS) along(std::integral_constant<int, EXO_RS_LMARS>{});
+  else if (rsolver == EXO_RS_HLLC) along(std::integral_constant<int, EXO_RS_HLLC>{});
+  else along(std::integral_constant<int, EXO_RS_LMARS_SHALLOW>{});
   return fp64::check_launch();
 }
 
