@@ -254,8 +254,9 @@ __device__ __forceinline__ void cov_to_contra(double* a, double cth) {
   a[IVY] = (v - w * cth) * is2;
   a[IVZ] = (w - v * cth) * is2;
 #else
-  a[IVY] = v / sth2 - w * cth / sth2;
-  a[IVZ] = -v * cth / sth2 + w / sth2;
+  const SharedDiv by_s2(sth2);
+  a[IVY] = by_s2(v) - by_s2(w * cth);
+  a[IVZ] = by_s2(-v * cth) + by_s2(w);
 #endif
 }
 __device__ __forceinline__ void contra_to_cov(double* a, double cth) {
@@ -585,6 +586,14 @@ __device__ __forceinline__ void riemann(int rsolver, const RiemannGas<double>& g
 __device__ __forceinline__ void ghost_interp(const DevView& v, const GhostEntry& e,
                                              const double* src, int i, double* c) {
   const size_t vs = v.cells;
+#if EXO_MIXED
+  auto by_C = [&](double a) { return a / e.C; };
+  auto by_s = [&](double a) { return a / e.ss; };
+#else
+  // the same quotients from one reciprocal each (and cov_to_contra's: FP64
+  // 96^2x64 109 -> 100 us; the mixed build's results would change in the last bit)
+  const SharedDiv by_C(e.C), by_s(e.ss);
+#endif
   const double* s0 = src + (size_t)(unsigned)(e.k0 * v.nc2 + e.j0) * (unsigned)v.nc1 + i;
   const double* s1 = src + (size_t)(unsigned)(e.k1 * v.nc2 + e.j1) * (unsigned)v.nc1 + i;
   #pragma unroll
@@ -593,16 +602,16 @@ __device__ __forceinline__ void ghost_interp(const DevView& v, const GhostEntry&
     if (n == IVY || n == IVZ) continue;
     double v1 = s0[n * vs];
     double v2 = s1[n * vs];
-    c[n] = (e.A * v1 + e.B * v2) / e.C;
+    c[n] = by_C(e.A * v1 + e.B * v2);
   }
   double v1y = s0[IVY * vs], v1z = s0[IVZ * vs];
   double v2y = s1[IVY * vs], v2z = s1[IVZ * vs];
-  double vy = (e.A * v1y + e.B * v2y) / e.C;
-  double vz = (e.A * v1z + e.B * v2z) / e.C;
-  double sth = e.ss, cth = e.cs;
+  double vy = by_C(e.A * v1y + e.B * v2y);
+  double vz = by_C(e.A * v1z + e.B * v2z);
+  double cth = e.cs;
   double vyt = vy, vzt = vz;
-  vy = vyt / sth / sth - vzt * cth / sth / sth;
-  vz = vzt / sth / sth - vyt * cth / sth / sth;
+  vy = by_s(by_s(vyt)) - by_s(by_s(vzt * cth));
+  vz = by_s(by_s(vzt)) - by_s(by_s(vyt * cth));
   double U = e.r[0] * vy + e.r[1] * vz;
   double V = e.r[2] * vy + e.r[3] * vz;
   vy = e.q[0] * U + e.q[1] * V;
@@ -1461,9 +1470,13 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
   const double a3p = x1vi * dx2f3p * dx1fi;
   const double vol = dx1fi * d2 * d3 * x1vi * x1vi * s;
   // the mixed build multiplies by reciprocals of the volume and the radius
-  // (one division each instead of eight; the FP64 build divides as the
-  // reference does)
-  [[maybe_unused]] const double ivol = inv_r(vol), irad = inv_r(x1vi);
+  // (one division each instead of eight); the FP64 build's quotients are the
+  // reference's, from one reciprocal each
+#if EXO_MIXED
+  const double ivol = inv_r(vol), irad = inv_r(x1vi);
+#else
+  const SharedDiv by_vol(vol), by_radius(x1vi);
+#endif
   double du[5];
   // flux divergence in T (the x1 part in FP64 where its fluxes are); the
   // conserved state accumulates in FP64
@@ -1472,12 +1485,13 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
   for (int n = 0; n < 5; ++n) {
     if (n >= nv) break;
     double change;
-    if constexpr (sizeof(T) == sizeof(double)) {
-      T dflx = (A1p * f0r[n] - A1 * f0l[n]);
-      dflx += (A2p * f1r[n] - A2 * f1l[n]);
-      dflx += (A3p * f2r[n] - A3 * f2l[n]);
-      change = wght * dflx / vol;
-    } else if constexpr (sizeof(X1Flux<T>) == sizeof(double)) {
+#if !EXO_MIXED
+    T dflx = (A1p * f0r[n] - A1 * f0l[n]);
+    dflx += (A2p * f1r[n] - A2 * f1l[n]);
+    dflx += (A3p * f2r[n] - A3 * f2l[n]);
+    change = by_vol(wght * dflx);
+#else
+    if constexpr (sizeof(X1Flux<T>) == sizeof(double)) {
       T d23 = (A2p * f1r[n] - A2 * f1l[n]);
       d23 += (A3p * f2r[n] - A3 * f2l[n]);
       const double d1 = a1p * f0r[n] - a1 * f0l[n];
@@ -1488,6 +1502,7 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
       dflx += (A3p * f2r[n] - A3 * f2l[n]);
       change = wght * (double)(dflx / T(vol));
     }
+#endif
     if (shallow) {
       un[n] -= change;
     } else {
@@ -1506,13 +1521,12 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
     const double y_ov_rC = (x1vi * dx2f3 * dx1fi * G2(GSINF3, 0) -
                             x1vi * dx2f3p * dx1fi * G2(GSINF3, v.nc2)) * ivol;
 #else
-    const double x_ov_rD = (x1vi * dx3f2 * dx1fi * G2(GSINF2, 0) -
-                            x1vi * dx3f2p * dx1fi * G2(GSINF2, 1)) / vol;
-    const double y_ov_rC = (x1vi * dx2f3 * dx1fi * G2(GSINF3, 0) -
-                            x1vi * dx2f3p * dx1fi * G2(GSINF3, v.nc2)) / vol;
+    const double x_ov_rD = by_vol(x1vi * dx3f2 * dx1fi * G2(GSINF2, 0) -
+                                  x1vi * dx3f2p * dx1fi * G2(GSINF2, 1));
+    const double y_ov_rC = by_vol(x1vi * dx2f3 * dx1fi * G2(GSINF3, 0) -
+                                  x1vi * dx2f3p * dx1fi * G2(GSINF3, v.nc2));
 #endif
     const double rho = wv[IDN], v1 = wv[IVX], v2 = wv[IVY], v3 = wv[IVZ];
-    [[maybe_unused]] const double radius = x1vi;
     double pr;
     const double v_2 = v2 + v3 * cosine;
     const double v_3 = v3 + v2 * cosine;
@@ -1523,7 +1537,7 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
 #if EXO_MIXED
       double src1 = (2.0 * pr + rho * (v2 * v_2 + v3 * v_3)) * irad;
 #else
-      double src1 = (2.0 * pr + rho * (v2 * v_2 + v3 * v_3)) / radius;
+      double src1 = by_radius(2.0 * pr + rho * (v2 * v_2 + v3 * v_3));
 #endif
       out[IVX] += wght * src1;
     }
@@ -1532,9 +1546,9 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
     out[IVY] += wght * src2;
     double src3 = -y_ov_rC * (pr + rho * v2 * v2 * sine2) - rho * v1 * v_3 * irad;
 #else
-    double src2 = -x_ov_rD * (pr + rho * v3 * v3 * sine2) - rho * v1 * v_2 / radius;
+    double src2 = -x_ov_rD * (pr + rho * v3 * v3 * sine2) - by_radius(rho * v1 * v_2);
     out[IVY] += wght * src2;
-    double src3 = -y_ov_rC * (pr + rho * v2 * v2 * sine2) - rho * v1 * v_3 / radius;
+    double src3 = -y_ov_rC * (pr + rho * v2 * v2 * sine2) - by_radius(rho * v1 * v_3);
 #endif
     out[IVZ] += wght * src3;
     // constant gravity (patches/25.constant_acc.patch:35-53)
@@ -3084,13 +3098,13 @@ __global__ void EXO_X23_BOUNDS kb_flux_x23(Batch bt) {
   flux_x23_block<T>(sv, b);
 }
 
-#ifdef EXO_UPD_MAXNREG
-#define EXO_UPD_BOUNDS __maxnreg__(EXO_UPD_MAXNREG)
-#else
-#define EXO_UPD_BOUNDS
-#endif
+// The update waits for its loads (mixed, 96^2x64: 61 % of the copy rate on the
+// bytes it needs, 16 warps per SM).  FP64 at its natural 140 registers has 12:
+// 303 us there, at 128 registers 276, at 96 and 80, with the inputs no longer
+// all requested at once, 329 and 312 (mixed 246, 276 and 274).  Its quotients
+// by the volume and the radius from one reciprocal each: 329 -> 303.
 template <class T>
-__global__ void EXO_UPD_BOUNDS kb_update(Batch bt, int stage) {
+__global__ void __maxnreg__(128) kb_update(Batch bt, int stage) {
   __shared__ __align__(16) DevView sv;
   unsigned b = batch_enter(bt, sv);
   update_block<T>(sv, b, stage);
