@@ -238,13 +238,21 @@ size_t decomposition_refs_doubles(const DevView& v) {
   return nq * (v.nc1 + 1) + 2 * nq * v.nc1 + 2 * nq;
 }
 
-// the column kernel's shared memory grows with L (the radial tables); the
-// attribute lets a launch go past the 48 KB default
+namespace {
+std::mutex g_columns_mu;
+}  // namespace
+
+// The column hook's two launches.  The back substitution reads the factors the
+// forward sweep left in the scratch, so the two are issued under one lock:
+// threads that share a scratch on one stream are kept apart by the stream's
+// order, call by call.  The column kernel's shared memory grows with L (the
+// radial tables); the attribute lets a launch go past the 48 KB default.
 template <bool full>
 static cudaError_t column_kernel(int ncol, int L, const double* w, double* du,
                                  const double* colgeo, const double* x1f, const double* x1v,
                                  const double* dx1f, double dt, double gamma, double grav,
                                  double* scratch, void* stream) {
+  std::lock_guard<std::mutex> together(g_columns_mu);
   cudaError_t e = cudaFuncSetAttribute(fp64::k_implicit_columns<full>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        fp64::IMPL_SMEM_MAX);

@@ -289,7 +289,9 @@ int exo_riemann(int rsolver, int eqn, int ivx, int n, double gamma,
      du      [ncol][5][L]    explicit update in, corrected update out
      colgeo  [ncol][4]       cos and sin of the cell metric, dx2f_ang, dx3f_ang
      x1f [L+7], x1v [L+6], dx1f [L+6]  radial faces, centres and widths
-     scratch ncol*L*30 doubles of caller-owned device memory
+     scratch ncol*L*30 doubles of caller-owned device memory; two calls may
+             share one when their work is ordered on the GPU (one stream, from
+             any host threads)
    Reflecting radial boundaries at both ends; dt is the stage's beta*dt. */
 int exo_implicit_columns(int ncol, int L, const double* w, double* du,
                          const double* colgeo, const double* x1f, const double* x1v,
@@ -324,8 +326,8 @@ int exo_partial_correction_columns(int ncol, int L, const double* w, double* du,
    that device current); make that first call before any stream capture.
    All calls share the one array and nothing in it needs to start at zero
    (every word a column reads was written earlier in the same call), but
-   calls that overlap on the GPU -- other streams, other threads -- race on
-   it: issue them in order on one stream. */
+   calls that overlap on the GPU -- on other streams -- race on it: issue
+   them on one stream (from any host threads). */
 #define EXO_NOALLOC_SCRATCH_DOUBLES 1048576
 int exo_implicit_columns_noalloc(int ncol, int L, const double* w, double* du,
                                  const double* colgeo, const double* x1f,

@@ -1,0 +1,74 @@
+// What the library's host code asks of the GPU, on the stand-in runtime of
+// host_cuda.h.  One check per argument; exit status 0 when it holds.
+#include <chrono>
+#include <condition_variable>
+#include <cstdio>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "../../include/exo_b200.h"
+#include "host_cuda.h"
+
+static int fail(const char* what) {
+  std::printf("FAIL %s: %s\n", what, exo_last_error());
+  return 1;
+}
+static bool is(const HostLaunch& l, const char* name) {
+  return l.kernel.find(name) != std::string::npos;
+}
+static bool forward(const HostLaunch& l) {
+  return is(l, "k_implicit_columns") && !is(l, "_bwd");
+}
+
+enum Form { FULL, PARTIAL, NOALLOC };
+static int columns(Form form, int ncol, int L, double* scratch, double dt = 60.) {
+  static double any[64];  // never read: nothing runs
+  const double* a = any;
+  if (form == NOALLOC)
+    return exo_implicit_columns_noalloc(ncol, L, a, any, a, a, a, a, dt, 1.4, -9.8, nullptr);
+  return form == FULL ? exo_implicit_columns(ncol, L, a, any, a, a, a, a, dt, 1.4, -9.8, scratch,
+                                             nullptr)
+                      : exo_partial_correction_columns(ncol, L, a, any, a, a, a, a, dt, 1.4, -9.8,
+                                                       scratch, nullptr);
+}
+
+// Two host threads solve columns on one stream with one scratch: the two
+// launches of a call, which hand the factors over in the scratch, stand side
+// by side in the stream.  Each forward sweep gives the other thread's time to
+// get between.
+static int check_pairs(Form form) {
+  std::mutex m;
+  std::condition_variable cv;
+  int sweeps = 0;
+  host_launches_clear();
+  host_on_launch([&](const HostLaunch& l) {
+    if (!forward(l)) return;
+    std::unique_lock<std::mutex> lk(m);
+    const int mine = ++sweeps;
+    cv.notify_all();
+    cv.wait_for(lk, std::chrono::milliseconds(300), [&] { return sweeps > mine; });
+  });
+  double scratch[8];
+  int rc[2] = {1, 1};
+  std::thread a([&] { rc[0] = columns(form, 4, 8, scratch); });
+  std::thread b([&] { rc[1] = columns(form, 4, 8, scratch); });
+  a.join();
+  b.join();
+  host_on_launch(nullptr);
+  const std::vector<HostLaunch> all = host_launches();
+  if (rc[0] || rc[1] || all.size() != 4) return fail("two calls of two launches");
+  for (int c = 0; c < 4; c += 2)
+    if (!forward(all[c]) || !is(all[c + 1], "_bwd") || all[c].thread != all[c + 1].thread)
+      return fail("a call's sweep and back substitution side by side in the stream");
+  return 0;
+}
+
+int main(int argc, char** argv) {
+  const char* what = argc > 1 ? argv[1] : "";
+  int rc = 2;
+  if (!std::strcmp(what, "pairs")) rc = check_pairs(FULL) + check_pairs(PARTIAL) + check_pairs(NOALLOC);
+  if (rc == 0) std::printf("%s: ok\n", what);
+  return rc;
+}
