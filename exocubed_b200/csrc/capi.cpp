@@ -106,6 +106,8 @@ struct exo_ctx {
 };
 
 
+static const char* const kWaitGaveUp = "a kernel's bounded wait for its bulk copies gave up";
+
 // Run one launch, bracketed by events when profiling.  `nlaunch` is the
 // number of kernels the launcher issues.
 template <typename F>
@@ -880,7 +882,12 @@ int exo_solve_implicit_3d(exo_ctx* c, double* du_host, const double* w_host, dou
                  [&] { return STEP(launch_implicit_du, c->v, dt, c->stream); });
   if (rc) return fail(rc, "implicit launch failed");
   CK(cudaMemcpyAsync(du_host, c->v.du, bytes, cudaMemcpyDeviceToHost, c->stream));
+  // the back substitution's waits are bounded: where one gave up, columns of
+  // du are left uncorrected
+  DevScalars s;
+  CK(cudaMemcpyAsync(&s, c->v.sc, sizeof(s), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  if (s.timeout) return fail(EXO_ERR_TIMEOUT, kWaitGaveUp);
   return EXO_OK;
 }
 
@@ -967,7 +974,7 @@ int exo_check_state(exo_ctx* c, int* invalid) {
   int zero = 0;
   CK(cudaMemcpyAsync(&c->v.sc->invalid, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (s.timeout) return fail(EXO_ERR_TIMEOUT, "a kernel's bounded wait for its bulk copies gave up");
+  if (s.timeout) return fail(EXO_ERR_TIMEOUT, kWaitGaveUp);
   return EXO_OK;
 }
 

@@ -189,7 +189,9 @@ int exo_boundary(exo_ctx* ctx);
    interior used) is corrected in place from the primitives w_host (ghosts
    used at the x1 boundaries) with time step dt.  It works in the context's
    own primitive and update arrays: load a state (exo_set_primitive) before
-   stepping the context again. */
+   stepping the context again.  EXO_ERR_TIMEOUT when a bounded wait of the
+   solve (or of an earlier call on the context) gave up: du_host may then
+   hold uncorrected columns. */
 int exo_solve_implicit_3d(exo_ctx* ctx, double* du_host, const double* w_host, double dt);
 /* Decomposition::ChangeToPerturbation(w, ...) (change_to_perturbation.cpp:
    39-157) on every radial column: w_host (six AthenaArray(NHYDRO, nc3, nc2,
@@ -420,7 +422,8 @@ typedef struct exo_array_view {
 /* The whole-array entry points on six panel views (views[p] = panel p), the
    reference's one AthenaArray per MeshBlock: exo_set_primitive,
    exo_get_primitive, exo_get_conserved and exo_solve_implicit_3d (du in and
-   out, w in) with their arrays gathered from and scattered to the views. */
+   out, w in) with their arrays gathered from and scattered to the views
+   (nothing is scattered when the call fails). */
 int exo_set_primitive_views(exo_ctx* ctx, const exo_array_view* w);
 int exo_get_primitive_views(exo_ctx* ctx, const exo_array_view* w);
 int exo_get_conserved_views(exo_ctx* ctx, const exo_array_view* u);

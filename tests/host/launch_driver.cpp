@@ -8,6 +8,7 @@
 #include <thread>
 #include <vector>
 
+#include "../../exocubed_b200/csrc/exo_internal.h"
 #include "../../include/exo_b200.h"
 #include "host_cuda.h"
 
@@ -65,10 +66,56 @@ static int check_pairs(Form form) {
   return 0;
 }
 
+// A bounded wait that gives up inside the back substitution is an error of the
+// call that launched it, whole arrays and views alike.
+static int check_timeout(int precision, int implicit_flag) {
+  exo_config cfg;
+  exo_config_default(&cfg, EXO_EQN_IDEAL);
+  cfg.N = 6;
+  cfg.L = 4;
+  cfg.precision = precision;
+  cfg.implicit_flag = implicit_flag;
+  exo_ctx* c = nullptr;
+  if (exo_create(&cfg, &c)) return fail("exo_create");
+  const size_t n = (size_t)6 * 5 * 12 * 12 * 10;
+  std::vector<double> du(n, 1.), w(n, 1.);
+  if (exo_solve_implicit_3d(c, du.data(), w.data(), 60.)) return fail("a solve without a timeout");
+  // the kernel's first argument is the batch, whose first member is the view
+  host_on_launch([](const HostLaunch& l) {
+    if (!is(l, "kb_implicit_bwd")) return;
+    const exo::DevView* const* batch = (const exo::DevView* const*)l.args[0];
+    batch[0]->sc->timeout = 1;
+  });
+  const int rc = exo_solve_implicit_3d(c, du.data(), w.data(), 60.);
+  host_on_launch(nullptr);
+  if (rc != EXO_ERR_TIMEOUT) return fail("EXO_ERR_TIMEOUT from exo_solve_implicit_3d");
+  exo_array_view v[6];
+  for (int p = 0; p < 6; ++p) {
+    v[p] = exo_array_view{};
+    v[p].data = w.data() + p * (n / 6);
+    v[p].dtype = EXO_DTYPE_F64;
+    v[p].nx4 = 5;
+    v[p].nx3 = v[p].nx2 = 12;
+    v[p].nx1 = 10;
+    v[p].stride[0] = 1440;
+    v[p].stride[1] = 120;
+    v[p].stride[2] = 10;
+    v[p].stride[3] = 1;
+    v[p].device = -1;
+  }
+  if (exo_solve_implicit_3d_views(c, v, v, 60.) != EXO_ERR_TIMEOUT)
+    return fail("EXO_ERR_TIMEOUT from exo_solve_implicit_3d_views");
+  exo_destroy(c);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   int rc = 2;
   if (!std::strcmp(what, "pairs")) rc = check_pairs(FULL) + check_pairs(PARTIAL) + check_pairs(NOALLOC);
+  if (!std::strcmp(what, "timeout"))
+    rc = check_timeout(EXO_PREC_FP64, 9) + check_timeout(EXO_PREC_FP64, 1) +
+         check_timeout(EXO_PREC_MIXED, 1) + check_timeout(EXO_PREC_MIXED_F32_SOLVE, 9);
   if (rc == 0) std::printf("%s: ok\n", what);
   return rc;
 }

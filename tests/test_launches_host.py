@@ -35,3 +35,7 @@ def _check(driver, what):
 
 def test_launches_of_a_column_solve_stay_together(driver):
     _check(driver, "pairs")
+
+
+def test_a_wait_that_gave_up_is_the_implicit_call_s_error(driver):
+    _check(driver, "timeout")
