@@ -293,6 +293,10 @@ int view_allocate(const exo_config& cfg, const HostTables& t, DevView& v,
   cudaStream_t stream = (cudaStream_t)stream_v;
   cudaMemPool_t pool = (cudaMemPool_t)pool_v;
   bool shallow = cfg.eqn == EXO_EQN_SHALLOW_YZ;
+  if (!places_fit(t.nc3, t.nc2)) {
+    *err = "N is too large: the kernels index the metric in 32 bits";
+    return EXO_ERR_CAPACITY;
+  }
   std::memset(&v, 0, sizeof(v));
   v.N = cfg.N;
   v.L = cfg.L;

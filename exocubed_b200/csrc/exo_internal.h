@@ -177,6 +177,21 @@ EXO_HD inline RiemannGas<T> make_riemann_gas(T gamma) {
           (gamma + one) / (T(2) * gamma)};
 }
 
+// Places in 32 bits, unsigned from the first product on (the signed product
+// passes 2^31 from nc2 = 3455 on, where one layer of shallow water still fits
+// a GPU): of field f in the horizontal metric, and of a row of nc1 cells in a
+// state array.  A state has fewer rows than the metric has values.
+EXO_HD inline unsigned geo_place(int nc3, int nc2, int f, int p, int k, int j) {
+  return ((unsigned)(f * 6 + p) * (unsigned)nc3 + (unsigned)k) * (unsigned)nc2 + (unsigned)j;
+}
+EXO_HD inline unsigned row_place(int nv, int nc3, int nc2, int p, int n, int k, int j) {
+  return ((unsigned)(p * nv + n) * (unsigned)nc3 + (unsigned)k) * (unsigned)nc2 + (unsigned)j;
+}
+// whether they are enough: nc2 up to 4884, where one layer of shallow water takes 195 GB
+inline bool places_fit(int nc3, int nc2) {
+  return (size_t)NGEO2D * 6 * nc3 * nc2 <= ((size_t)1 << 32);
+}
+
 // How the x2/x3 fluxes are cut: groups of 32 lines per panel and direction,
 // chunks of faces per segment of a line, segments.
 struct X23Split {

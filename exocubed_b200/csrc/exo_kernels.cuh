@@ -97,13 +97,10 @@ __device__ __forceinline__ double rk_beta(int stage) {
 }
 
 __device__ __forceinline__ size_t idx(const DevView& v, int p, int n, int k, int j, int i) {
-  return (size_t)(unsigned)(((p * v.nv + n) * v.nc3 + k) * v.nc2 + j) * (unsigned)v.nc1 +
-         (unsigned)i;
+  return (size_t)row_place(v.nv, v.nc3, v.nc2, p, n, k, j) * (unsigned)v.nc1 + (unsigned)i;
 }
 __device__ __forceinline__ double geo(const DevView& v, int f, int p, int k, int j) {
-  // (fits 32 bits: NGEO2D * 6 * nc3 * nc2 passes 2^32 beyond nc2 = 4800,
-  // whose state does not fit a GPU)
-  return v.geo[(unsigned)(((f * 6 + p) * v.nc3 + k) * v.nc2 + j)];
+  return v.geo[geo_place(v.nc3, v.nc2, f, p, k, j)];
 }
 
 // face-flux and primitive arrays in the type the flux kernels work in

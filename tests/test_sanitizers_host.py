@@ -51,3 +51,8 @@ def test_fastdiv_exact_under_sanitizers(tmp_path):
 def test_shared_division_is_ieee_under_sanitizers(tmp_path):
     out = _build_and_run(tmp_path, "shareddiv", ["tests/sanitize/shareddiv_driver.cpp"])
     assert "shareddiv: ok" in out
+
+
+def test_places_in_32_bits_under_sanitizers(tmp_path):
+    out = _build_and_run(tmp_path, "places", ["tests/sanitize/places_driver.cpp"])
+    assert "places: ok" in out
