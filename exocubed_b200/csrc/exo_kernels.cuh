@@ -588,7 +588,7 @@ __device__ __forceinline__ void ghost_interp(const DevView& v, const GhostEntry&
   auto by_s = [&](double a) { return a / e.ss; };
 #else
   // the same quotients from one reciprocal each (and cov_to_contra's: FP64
-  // 96^2x64 109 -> 100 us; the mixed build's results would change in the last bit)
+  // 96^2x64 109 -> 102 us; the mixed build's results would change in the last bit)
   const SharedDiv by_C(e.C), by_s(e.ss);
 #endif
   const double* s0 = src + (size_t)(unsigned)(e.k0 * v.nc2 + e.j0) * (unsigned)v.nc1 + i;
@@ -1486,7 +1486,7 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
     T dflx = (A1p * f0r[n] - A1 * f0l[n]);
     dflx += (A2p * f1r[n] - A2 * f1l[n]);
     dflx += (A3p * f2r[n] - A3 * f2l[n]);
-    change = by_vol(wght * dflx);
+    change = by_vol.finite(wght * dflx);
 #else
     if constexpr (sizeof(X1Flux<T>) == sizeof(double)) {
       T d23 = (A2p * f1r[n] - A2 * f1l[n]);
@@ -1518,9 +1518,9 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
     const double y_ov_rC = (x1vi * dx2f3 * dx1fi * G2(GSINF3, 0) -
                             x1vi * dx2f3p * dx1fi * G2(GSINF3, v.nc2)) * ivol;
 #else
-    const double x_ov_rD = by_vol(x1vi * dx3f2 * dx1fi * G2(GSINF2, 0) -
+    const double x_ov_rD = by_vol.finite(x1vi * dx3f2 * dx1fi * G2(GSINF2, 0) -
                                   x1vi * dx3f2p * dx1fi * G2(GSINF2, 1));
-    const double y_ov_rC = by_vol(x1vi * dx2f3 * dx1fi * G2(GSINF3, 0) -
+    const double y_ov_rC = by_vol.finite(x1vi * dx2f3 * dx1fi * G2(GSINF3, 0) -
                                   x1vi * dx2f3p * dx1fi * G2(GSINF3, v.nc2));
 #endif
     const double rho = wv[IDN], v1 = wv[IVX], v2 = wv[IVY], v3 = wv[IVZ];
@@ -1534,7 +1534,7 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
 #if EXO_MIXED
       double src1 = (2.0 * pr + rho * (v2 * v_2 + v3 * v_3)) * irad;
 #else
-      double src1 = by_radius(2.0 * pr + rho * (v2 * v_2 + v3 * v_3));
+      double src1 = by_radius.finite(2.0 * pr + rho * (v2 * v_2 + v3 * v_3));
 #endif
       out[IVX] += wght * src1;
     }
@@ -1543,9 +1543,9 @@ __device__ __forceinline__ void update_block(const DevView& v, unsigned blk, int
     out[IVY] += wght * src2;
     double src3 = -y_ov_rC * (pr + rho * v2 * v2 * sine2) - rho * v1 * v_3 * irad;
 #else
-    double src2 = -x_ov_rD * (pr + rho * v3 * v3 * sine2) - by_radius(rho * v1 * v_2);
+    double src2 = -x_ov_rD * (pr + rho * v3 * v3 * sine2) - by_radius.finite(rho * v1 * v_2);
     out[IVY] += wght * src2;
-    double src3 = -y_ov_rC * (pr + rho * v2 * v2 * sine2) - by_radius(rho * v1 * v_3);
+    double src3 = -y_ov_rC * (pr + rho * v2 * v2 * sine2) - by_radius.finite(rho * v1 * v_3);
 #endif
     out[IVZ] += wght * src3;
     // constant gravity (patches/25.constant_acc.patch:35-53)
@@ -1665,10 +1665,10 @@ __device__ __forceinline__ void roe_average(double* prim, double gm1, const GasD
   prim[IVX] = (sqrtdl * wl[IVX] + sqrtdr * wr[IVX]) * isdlpdr;
   prim[IVY] = (sqrtdl * wl[IVY] + sqrtdr * wr[IVY]) * isdlpdr;
   prim[IVZ] = (sqrtdl * wl[IVZ] + sqrtdr * wr[IVZ]) * isdlpdr;
-  double el = gd.gm1(wl[IPR]) + 0.5 * wl[IDN] * (sqr(wl[IVX]) + sqr(wl[IVY]) + sqr(wl[IVZ]));
-  double er = gd.gm1(wr[IPR]) + 0.5 * wr[IDN] * (sqr(wr[IVX]) + sqr(wr[IVY]) + sqr(wr[IVZ]));
+  double el = gd.gm1.finite(wl[IPR]) + 0.5 * wl[IDN] * (sqr(wl[IVX]) + sqr(wl[IVY]) + sqr(wl[IVZ]));
+  double er = gd.gm1.finite(wr[IPR]) + 0.5 * wr[IDN] * (sqr(wr[IVX]) + sqr(wr[IVY]) + sqr(wr[IVZ]));
   double hbar = ((el + wl[IPR]) / sqrtdl + (er + wr[IPR]) / sqrtdr) * isdlpdr;
-  prim[IPR] = gd.gp1((hbar - 0.5 * (sqr(prim[IVX]) + sqr(prim[IVY]) + sqr(prim[IVZ]))) * gm1) *
+  prim[IPR] = gd.gp1.finite((hbar - 0.5 * (sqr(prim[IVX]) + sqr(prim[IVY]) + sqr(prim[IVZ]))) * gm1) *
               prim[IDN];
 }
 #endif
@@ -1828,9 +1828,9 @@ __device__ __forceinline__ void abs_jacobian(const ColCell<double>& L, const Col
   // divisions by a common denominator share its reciprocal (SharedDiv: the
   // IEEE quotient)
   const SharedDiv by_rr(rr);
-  double cs = sqrt(by_rr((1. + (gamma - 1) * feps / fsig) * p));
+  double cs = sqrt(by_rr.finite((1. + (gamma - 1) * feps / fsig) * p));
   double ke = 0.5 * (u * u + v * v + w * w);
-  double hp = by_rr((gm1 + 1.) / gm1 * p);
+  double hp = by_rr.finite((gm1 + 1.) / gm1 * p);
   double h = hp + ke;
   const double Rm[5][5] = {{1., 1., 1., 0., 0.},
                            {u - cs, u, u + cs, 0., 0.},
@@ -1838,11 +1838,11 @@ __device__ __forceinline__ void abs_jacobian(const ColCell<double>& L, const Col
                            {w, w, w, 0., 1.},
                            {h - u * cs, ke, h + u * cs, v, w}};
   const SharedDiv by_hp(hp), by_2hp(2. * hp), by_2cshp(2. * cs * hp);
-  double mv2 = by_2hp(-v), mw2 = by_2hp(-w), i2 = by_2hp.r;
+  double mv2 = by_2hp.finite(-v), mw2 = by_2hp.finite(-w), i2 = by_2hp.r;
   const double Ri[5][5] = {
-      {by_2cshp(cs * ke + u * hp), by_2cshp(-hp - cs * u), mv2, mw2, i2},
-      {by_hp(hp - ke), by_hp(u), by_hp(v), by_hp(w), -by_hp.r},
-      {by_2cshp(cs * ke - u * hp), by_2cshp(hp - cs * u), mv2, mw2, i2},
+      {by_2cshp.finite(cs * ke + u * hp), by_2cshp.finite(-hp - cs * u), mv2, mw2, i2},
+      {by_hp.finite(hp - ke), by_hp.finite(u), by_hp.finite(v), by_hp.finite(w), -by_hp.r},
+      {by_2cshp.finite(cs * ke - u * hp), by_2cshp.finite(hp - cs * u), mv2, mw2, i2},
       {-v, 0., 1., 0., 0.},
       {-w, 0., 0., 1., 0.}};
   const double lam[5] = {fabs(u - cs), fabs(u), fabs(u + cs), fabs(u), fabs(u)};
@@ -2108,17 +2108,17 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, i
 #else
         double num = am * aleft + ap * aright;
         if constexpr (fj_nz(r, q)) num = num + (aright - aleft) * fj_entry<r, q>(c0, gm1);
-        double a = by_2vol(num);
+        double a = by_2vol.finite(num);
         if constexpr (r == q) a = a + rdt;
         if constexpr ((r == IVX && q == IDN) || (r == IEN && q == IVX)) a = a - grav;
         double bm = am;
         if constexpr (fj_nz(r, q)) bm = am + fj_entry<r, q>(cm, gm1);
-        double b = by_2vol(-bm * aleft);
+        double b = by_2vol.finite(-bm * aleft);
         if (first) a = a + ((q == IVX) ? -b : b);
         if (last) {
           double cmv = ap;
           if constexpr (fj_nz(r, q)) cmv = ap - fj_entry<r, q>(cp, gm1);
-          double c = by_2vol(-cmv * aright);
+          double c = by_2vol.finite(-cmv * aright);
           a = a + ((q == IVX) ? -c : c);
         }
 #endif
@@ -2162,7 +2162,7 @@ __device__ __forceinline__ void implicit_column(IO& io, typename IO::Real* sa, i
         c[r] = -cmv * cr;
 #else
         if constexpr (fj_nz(r, q)) cmv = cmv - fj_entry<r, q>(cp, gm1);
-        c[r] = by_2vol(-cmv * aright);
+        c[r] = by_2vol.finite(-cmv * aright);
 #endif
       });
     };
@@ -2458,15 +2458,15 @@ __device__ __forceinline__ void implicit_column_partial(IO& io, typename IO::Rea
 #else
         double num = am * aleft + ap * aright;
         if constexpr (fj_nz(pr, pq)) num = num + (aright - aleft) * fj_entry<pr, pq>(c0, gm1);
-        double a = by_2vol(num);
+        double a = by_2vol.finite(num);
         if constexpr (r == q) a = a + rdt;
         if constexpr (phi) a = a - grav;
         double bm = am;
         if constexpr (fj_nz(pr, pq)) bm = am + fj_entry<pr, pq>(cm, gm1);
-        double b = by_2vol(-bm * aleft);
+        double b = by_2vol.finite(-bm * aleft);
         double cmv = ap;
         if constexpr (fj_nz(pr, pq)) cmv = ap - fj_entry<pr, pq>(cp, gm1);
-        double c = by_2vol(-cmv * aright);
+        double c = by_2vol.finite(-cmv * aright);
         if (first) a = a + ((q == 1) ? -b : b);
         if (last) a = a + ((q == 1) ? -c : c);
 #endif

@@ -56,3 +56,10 @@ def test_shared_division_is_ieee_under_sanitizers(tmp_path):
 def test_places_in_32_bits_under_sanitizers(tmp_path):
     out = _build_and_run(tmp_path, "places", ["tests/sanitize/places_driver.cpp"])
     assert "places: ok" in out
+
+
+def test_shared_division_at_its_limits_under_sanitizers(tmp_path):
+    # (division by zero is one of the checked cases)
+    out = _build_and_run(tmp_path, "shareddiv_limits", ["tests/sanitize/shareddiv_limits_driver.cpp"],
+                         extra=["-fno-sanitize=float-divide-by-zero"])
+    assert "shareddiv limits: ok" in out
