@@ -1069,6 +1069,7 @@ int exo_implicit_columns(int ncol, int L, const double* w, double* du, const dou
   if (!w || !du || !colgeo || !x1f || !x1v || !dx1f || !scratch)
     return fail(EXO_ERR_ARG, "NULL array");
   if (!(dt > 0.) || !(gamma > 1.)) return fail(EXO_ERR_ARG, "dt must be > 0 and gamma > 1");
+  if (L > exo::COLUMN_MAX_L) return fail(EXO_ERR_ARG, exo::column_too_deep(L));
   RK(exo::launch_implicit_columns(ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt, gamma, grav,
                                   scratch, stream, 1));
   return EXO_OK;
@@ -1083,6 +1084,7 @@ int exo_partial_correction_columns(int ncol, int L, const double* w, double* du,
   if (!w || !du || !colgeo || !x1f || !x1v || !dx1f || !scratch)
     return fail(EXO_ERR_ARG, "NULL array");
   if (!(dt > 0.) || !(gamma > 1.)) return fail(EXO_ERR_ARG, "dt must be > 0 and gamma > 1");
+  if (L > exo::COLUMN_MAX_L) return fail(EXO_ERR_ARG, exo::column_too_deep(L));
   RK(exo::launch_implicit_columns(ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt, gamma, grav,
                                   scratch, stream, 0));
   return EXO_OK;

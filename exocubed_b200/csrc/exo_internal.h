@@ -294,6 +294,12 @@ enum { IMPL_FULL = 1, IMPL_PARTIAL = 2 };
 EXO_HD inline int implicit_kind(const DevView& v) {
   return (v.implicit_flag & 8) ? IMPL_FULL : IMPL_PARTIAL;
 }
+// the deepest column of the column hooks: its radial tables
+// and a warp's memory share a block's shared memory
+constexpr int COLUMN_MAX_L = 5518;
+inline std::string column_too_deep(int L) {
+  return "L = " + std::to_string(L) + " exceeds " + std::to_string(COLUMN_MAX_L) + " levels";
+}
 // its launches: a forward sweep and a back substitution per block size (the
 // mixed build's 5x5 FP64 blocks do both in one)
 inline int implicit_launches(int kinds, int precision) {

@@ -257,8 +257,16 @@ static cudaError_t column_kernel(int ncol, int L, const double* w, double* du,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        fp64::IMPL_SMEM_MAX);
   if (e != cudaSuccess) return e;
-  fp64::k_implicit_columns<full><<<fp64::nblk(ncol, fp64::IMPL_THREADS), fp64::IMPL_THREADS,
-                                   fp64::impl_smem<double, full>(fp64::IMPL_THREADS, L + 2 * G),
+  // from 4900 levels on (full correction) only one warp's memory fits beside
+  // the radial tables
+  const bool fits = fp64::impl_smem<double, full>(fp64::IMPL_THREADS, L + 2 * G) <=
+                    (size_t)fp64::IMPL_SMEM_MAX;
+  const int threads = fits ? fp64::IMPL_THREADS : 32;
+  static_assert(fp64::impl_smem<double, full>(32, COLUMN_MAX_L + 2 * G) <=
+                    (size_t)fp64::IMPL_SMEM_MAX,
+                "a block of one warp takes the deepest column");
+  fp64::k_implicit_columns<full><<<fp64::nblk(ncol, threads), threads,
+                                   fp64::impl_smem<double, full>(threads, L + 2 * G),
                                    (cudaStream_t)stream>>>(ncol, L, w, du, colgeo, x1f, x1v, dx1f,
                                                            dt, gamma, grav, scratch);
   e = cudaGetLastError();
@@ -334,6 +342,10 @@ int launch_implicit_columns_noalloc(int ncol, int L, const double* w, double* du
     scratch = g_noalloc_addr[dev];
   }
   if (ncol <= 0) return 0;
+  if (L > COLUMN_MAX_L) {
+    *err = column_too_deep(L);
+    return EXO_ERR_ARG;
+  }
   e = column_kernel<true>(ncol, L, w, du, colgeo, x1f, x1v, dx1f, dt, gamma, grav, scratch, stream);
   if (e != cudaSuccess) {
     *err = std::string("k_implicit_columns: ") + cudaGetErrorString(e);

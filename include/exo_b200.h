@@ -294,7 +294,8 @@ int exo_riemann(int rsolver, int eqn, int ivx, int n, double gamma,
      scratch ncol*L*30 doubles of caller-owned device memory; two calls may
              share one when their work is ordered on the GPU (one stream, from
              any host threads)
-   Reflecting radial boundaries at both ends; dt is the stage's beta*dt. */
+   Reflecting radial boundaries at both ends; dt is the stage's beta*dt.  L
+   is at most 5518 here and in the two forms below (EXO_ERR_ARG). */
 int exo_implicit_columns(int ncol, int L, const double* w, double* du,
                          const double* colgeo, const double* x1f, const double* x1v,
                          const double* dx1f, double dt, double gamma, double grav,

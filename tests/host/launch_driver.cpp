@@ -66,6 +66,26 @@ static int check_pairs(Form form) {
   return 0;
 }
 
+// The deepest columns the hooks take (the radial tables of a block stand in its
+// shared memory beside the warps' own), and the first ones they refuse.
+static int check_levels() {
+  double scratch[8];
+  for (Form form : {FULL, PARTIAL, NOALLOC})
+    for (int L : {1, 250, 4899, 4900, 5518}) {
+      host_launches_clear();
+      if (columns(form, 3, L, scratch)) return fail("a column solve of this depth");
+      const std::vector<HostLaunch> all = host_launches();
+      if (all.size() != 2 || all[0].grid * all[0].block < 3) return fail("two launches over 3 columns");
+    }
+  for (Form form : {FULL, PARTIAL, NOALLOC}) {
+    host_launches_clear();
+    if (columns(form, 3, 5519, scratch) != EXO_ERR_ARG) return fail("EXO_ERR_ARG past the deepest column");
+    if (columns(form, 0, 5519, scratch)) return fail("no columns of any depth");
+    if (!host_launches().empty()) return fail("no launch for a refused call");
+  }
+  return 0;
+}
+
 // A bounded wait that gives up inside the back substitution is an error of the
 // call that launched it, whole arrays and views alike.
 static int check_timeout(int precision, int implicit_flag) {
@@ -113,6 +133,7 @@ int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   int rc = 2;
   if (!std::strcmp(what, "pairs")) rc = check_pairs(FULL) + check_pairs(PARTIAL) + check_pairs(NOALLOC);
+  if (!std::strcmp(what, "levels")) rc = check_levels();
   if (!std::strcmp(what, "timeout"))
     rc = check_timeout(EXO_PREC_FP64, 9) + check_timeout(EXO_PREC_FP64, 1) +
          check_timeout(EXO_PREC_MIXED, 1) + check_timeout(EXO_PREC_MIXED_F32_SOLVE, 9);

@@ -39,3 +39,7 @@ def test_launches_of_a_column_solve_stay_together(driver):
 
 def test_a_wait_that_gave_up_is_the_implicit_call_s_error(driver):
     _check(driver, "timeout")
+
+
+def test_column_hooks_take_the_deepest_columns(driver):
+    _check(driver, "levels")
