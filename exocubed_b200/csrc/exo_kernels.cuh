@@ -2736,7 +2736,8 @@ struct BwdLayout {
   static constexpr size_t fac_bytes = FRING * level_bytes;
   static constexpr size_t del_bytes = (size_t)2 * NB * 32 * DS * sizeof(double);
   static constexpr size_t bytes = fac_bytes + del_bytes;
-  static_assert(level_bytes % 16 == 0, "bulk copies move multiples of 16 bytes");
+  static_assert(level_bytes % 16 == 0 && NM * 32 * sizeof(R) % 16 == 0,
+                "bulk copies start on and move multiples of 16 bytes");
 };
 constexpr int BWD_THREADS = 96;
 
@@ -2767,21 +2768,24 @@ __device__ __forceinline__ void implicit_bwd_group(const BwdGroup<R>& g, unsigne
   const int nch = (L + CL - 1) / CL;
   auto var = [](int m) { return NB == 5 ? m : (m == 2 ? (int)IEN : m); };
   if (threadIdx.x < 32) {
-    // the j-th level from the top, into slot j
+    // the j-th level from the top, into slot j; of the top level only delta,
+    // its (A c) being neither formed nor read
     auto issue = [&](int j) {
-      const int l = L - 1 - j;
+      const int l = L - 1 - j, e0 = j == 0 ? NM : 0;
       R* dst = ring + (j & (FRING - 1)) * NFAC * 32;
       if constexpr (kBulk) {
         if (l >= 0 && lane == 0) {
-          mbar_expect_tx(&full[j & (FRING - 1)], (unsigned)LY::level_bytes);
-          bulk_g2s(dst, g.scr + (size_t)l * g.lstride, (unsigned)LY::level_bytes,
+          const unsigned bytes = (unsigned)((NFAC - e0) * 32 * sizeof(R));
+          mbar_expect_tx(&full[j & (FRING - 1)], bytes);
+          bulk_g2s(dst + e0 * 32, g.scr + (size_t)l * g.lstride + e0 * 32, bytes,
                    &full[j & (FRING - 1)]);
         }
       } else {
         if (l >= 0 && lane < g.ncols) {
           const R* src = g.scr + (size_t)l * g.lstride + lane;
 #pragma unroll
-          for (int e = 0; e < NFAC; ++e) cp_async_r(dst + e * 32 + lane, src + e * g.estride);
+          for (int e = 0; e < NFAC; ++e)
+            if (e >= e0) cp_async_r(dst + e * 32 + lane, src + e * g.estride);
         }
         cp_async_commit();
       }
@@ -2817,7 +2821,7 @@ __device__ __forceinline__ void implicit_bwd_group(const BwdGroup<R>& g, unsigne
             __syncwarp();
           }
           const R* f = ring + (j & (FRING - 1)) * NFAC * 32 + lane;
-          // delta of the top level is its own (its (A c) is not formed)
+          // delta of the top level is its own
           R dl[NB];
 #pragma unroll
           for (int r = 0; r < NB; ++r) {
