@@ -156,10 +156,12 @@ __device__ __forceinline__ T weno5(T phip2, T phip1, T phi, T phim1, T phim2) {
                       kWeno[7] * sqr(3. * phi - 4. * phip1 + phip2);
     const double d0 = (b0 + eps) * (b0 + eps), d1 = (b1 + eps) * (b1 + eps),
                  d2 = (b2 + eps) * (b2 + eps);
-    // every weight's denominator below 2^400 (they are above eps^2): the
+    // every weight's denominator below 2^400 (they are above eps^2), and so the
+    // five values within 2^105 of each other, and one of them below 2^400: the
     // divisions need no further checks.  NaN and infinity fail this.
     const unsigned top = max(max((unsigned)__double2hiint(d0), (unsigned)__double2hiint(d1)),
-                             (unsigned)__double2hiint(d2));
+                             max((unsigned)__double2hiint(d2),
+                                 (unsigned)__double2hiint(phi) & 0x7fffffffu));
     double a0, a1, a2;
     if (top < ((1023u + 400u) << 20)) {
       a0 = div_nr(kWeno[9], d0);
