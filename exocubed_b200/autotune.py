@@ -4,7 +4,9 @@ For one atmosphere configuration it times every kernel of a few real steps
 at each candidate tile (one candidate per kernel per trial, the kernels
 timed separately by the library's event profiler) on a throw-away context
 with a synthetic state of that configuration, and caches the per-launch
-times under the key (N, L, equation set, solver, implicit flag, precision).
+times under the key (N, L, equation set, solver, implicit flag, precision) and
+the build of the library they were measured on: another build's fastest tiles
+are others.
 
 A single atmosphere takes, per kernel, the fastest candidate.  A batch of
 uneven members runs each kernel as one launch, so it takes, per kernel, the
@@ -15,6 +17,8 @@ results do not depend on them (tests/test_gpu_tiles.py checks it bit for
 bit).  The cache is a JSON file ($EXO_TILE_CACHE, default
 ~/.cache/exocubed_b200/tiles.json).
 """
+import functools
+import hashlib
 import json
 import os
 import threading
@@ -45,6 +49,17 @@ def config_key(cfg):
     c = cfg if isinstance(cfg, dict) else cfg.as_dict()
     return (f"N{c['N']}_L{c['L']}_eqn{c['eqn']}_rs{c['rsolver']}_imp{c['implicit_flag']}"
             f"_prec{c['precision']}")
+
+
+@functools.lru_cache(maxsize=None)
+def build_id(path=nat.LIB_PATH):
+    """The library's build: the start of its file's SHA-256."""
+    with open(path, "rb") as f:
+        return hashlib.file_digest(f, "sha256").hexdigest()[:12]
+
+
+def table_key(cfg):
+    return f"{config_key(cfg)}_build{build_id()}"
 
 
 class TileCache:
@@ -109,7 +124,7 @@ def measure(cfg, steps=2):
 def table_for(cfg, cache=None):
     """The configuration's table, measured once and cached."""
     cache = cache if cache is not None else TileCache()
-    key = config_key(cfg)
+    key = table_key(cfg)
     with _lock:
         if key not in cache.tables:
             cache.tables[key] = measure(cfg)
