@@ -1,19 +1,21 @@
 // exo_implicit_fused.cuh -- the mixed build's 5x5 solve in FP64 blocks with its
 // back substitution in the same kernel (textually part of exo_kernels.cuh).
 //
-// The same algorithm as implicit_column and kb_implicit_bwd, in the form it
-// had before those two were split.  The split form is a little faster
-// (6x96^2x64: 764 against 788 us a solve; with the blocks kept by their
-// structure 617), but compiled with fused multiply-adds it does not round as
-// this one does: the last bits of u it changes reach the FP32 copy of the
-// primitives, and a run differs by 1e-7 within some tens of steps.  (The
-// boundary terms as branches, 752 us, change the roundings too.)  Its forward
-// sweep's loads by warp tiles and the swaps' branches taken by the warp are
-// 867 -> 788 us there, 4112 -> 4088 at 6x192^2x96, where the scratch's traffic
-// (480 of 640 bytes a level and column, 2.1 ms at the copy rate) weighs more.
+// The same algorithm as implicit_column and kb_implicit_bwd in one kernel.  The
+// split form measured 764 us a solve at 6x96^2x64 (with the blocks kept by
+// their structure 617), this one 780; but compiled with fused multiply-adds
+// the split form does not round as this one does: the last bits of u it
+// changes reach the FP32 copy of the primitives, and a run differs by 1e-7
+// within some tens of steps.  (The boundary terms as branches change the
+// roundings too.)  FP32 blocks, the 3x3 blocks and the FP64 build, whose
+// results the split form leaves to the bit, take the split form.
+//
+// What bounds it: dependent FP64 operations at eight to nine warps per SM, on
+// large grids the scratch's traffic (480 of 640 bytes a level and column,
+// 2.1 ms at the copy rate at 6x192^2x96), and the L1 beside the blocks' shared
+// memory, which the columns' strided loads live on (fused_tiles).
 // More warps do not help (200 registers, ten warps: the same; 168: twice the
-// time, the lines of L1 in flight being what limits them).  FP32 blocks, the 3x3 blocks and the FP64 build,
-// whose results the split form leaves to the bit, take the split form.
+// time, the lines of L1 in flight being what limits them).
 
 // Solve with the LU factors of implicit_column's mixed build (rows taken in
 // the order 1, 4, 2, 3, 0, threshold row swaps packed 3 bits per step): y
@@ -65,10 +67,17 @@ constexpr int BWD_TL = 4;
 // the two u tiles of a warp's back substitution (5 variables x 32 columns x
 // BWD_TL levels, padded)
 constexpr int WARP_TILE_DOUBLES = 2 * 5 * 32 * (BWD_TL + 1);
-// a warp's shared memory: the level tile, then two face matrices per lane
-// (entry e of lane l at [e * 32 + l])
-constexpr int FUSED_WARP_DOUBLES = LEVEL_TILE_DOUBLES + 50 * 32;
-static_assert(FUSED_WARP_DOUBLES >= WARP_TILE_DOUBLES,
+// a warp's shared memory: the inputs (a level tile, or w and du of the next
+// level), then two face matrices (entry e of lane l at [e * 32 + l])
+template <bool kTile>
+__host__ __device__ constexpr int fused_input_doubles() {
+  return kTile ? LEVEL_TILE_DOUBLES : 10 * 32;
+}
+template <bool kTile>
+__host__ __device__ constexpr int fused_warp_doubles() {
+  return fused_input_doubles<kTile>() + 50 * 32;
+}
+static_assert(fused_warp_doubles<false>() >= WARP_TILE_DOUBLES,
               "the tiled back substitution's buffers fit in the warp's memory");
 template <class IO>
 __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
@@ -184,8 +193,8 @@ __device__ __forceinline__ void implicit_backward_tiled(IO& io, int is, int ie,
   }
 }
 
-template <class IO>
-__device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real* sa, int ss, double* tile,
+template <bool kTile, class IO>
+__device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real* sa, int ss, double* in,
                                                 double cos_theta, double sin_theta, double d2,
                                                 double d3, const double* x1f, const double* x1v,
                                                 const double* dx1f, int is, int ie, double dt,
@@ -219,9 +228,10 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
   };
   auto AMs = [&](int slot, int r, int q) -> R& { return sa[(slot * 25 + r * 5 + q) * ss]; };
 
-  // w(i+1) and du(i), four levels at a time by the whole warp; the last warp
-  // of a member, where some lanes have no column, copies per lane
-  LevelTile<IO, 5> lt(io, tile, is, ie - is + 1);
+  // w(i+1) and du(i): with kTile four levels at a time by the whole warp (the
+  // last warp of a member, where some lanes have no column, copies per lane),
+  // else each lane its own, a level ahead
+  LevelTile<IO, 5> lt(io, in, is, ie - is + 1);
   auto ready = [&](int k0) {
     if (io.live == 0xffffffffu) {
       lt.ready(io, k0);
@@ -239,11 +249,22 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
       __syncwarp(io.live);
     }
   };
+  double* const next = in + (threadIdx.x & 31);
+  auto prefetch = [&](int iw, int idu) {
+#pragma unroll
+    for (int n = 0; n < 5; ++n) cp_async8(next + n * 32, io.wptr(iw, n));
+    if (idu >= 0) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) cp_async8(next + (5 + n) * 32, io.duptr(idu, n));
+    }
+    cp_async_commit();
+  };
   double raw[5];
   io.w(is - 1, raw);
   ColCell cm = cell(raw);
   io.w(is, raw);
   ColCell c0 = cell(raw);
+  if constexpr (!kTile) prefetch(is + 1, is);
   {
     R A[5][5];
     abs_jacobian(cm, c0, gm1, gam, A);
@@ -256,14 +277,16 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
   R dp[5];  // delta_{i-1}
   int cur = 0;
   for (int i = is; i <= ie; ++i) {
-    ready(i - is);
+    if constexpr (kTile) ready(i - is);
+    else cp_async_wait_all();
     double rhs[5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      raw[n] = lt.get(n, i - is);
-      rhs[n] = lt.get(5 + n, i - is);
+      raw[n] = kTile ? lt.get(n, i - is) : next[n * 32];
+      rhs[n] = kTile ? lt.get(5 + n, i - is) : next[(5 + n) * 32];
     }
     ColCell cp = cell(raw);
+    if constexpr (!kTile) prefetch(i + 2, i < ie ? i + 1 : -1);
     const int nxt = cur ^ 1;
     {
       R A[5][5];
@@ -411,13 +434,38 @@ __device__ __forceinline__ void implicit_column_fused(IO& io, typename IO::Real*
     cur = nxt;
   }
   // the warp's shared memory, free once every lane has finished its forward
-  // sweep, holds the back substitution's tiles
+  // sweep and its last copies (unused) have landed, holds the back
+  // substitution's tiles
+  if constexpr (!kTile) cp_async_wait_all();
   implicit_backward_tiled(io, is, ie, dp, wt);
 }
 
-// shared memory: FUSED_WARP_DOUBLES for each warp, then the radial tables
+// shared memory: fused_warp_doubles for each warp, then the radial tables
+template <bool kTile>
 constexpr size_t fused_smem(int threads, int nc1) {
-  return ((size_t)FUSED_WARP_DOUBLES * (threads / 32) + 3 * (size_t)(nc1 + 1)) * sizeof(double);
+  return ((size_t)fused_warp_doubles<kTile>() * (threads / 32) + 3 * (size_t)(nc1 + 1)) * sizeof(double);
+}
+// How the inputs come in.  A level tile reads each sector once but takes 23 KB
+// a warp; per lane (15 KB) a sector is read four times, three of them from
+// L1.  An SM's shared memory goes up in steps, and what is left of 256 KB is
+// L1: at the default 64 columns a block, four blocks with tiles leave 60 KB as
+// long as they stay within the step of 196 KB (99 levels), past it 28 KB, too
+// few lines for the copies in flight.  At 32 columns eight blocks with tiles
+// leave 28 KB, nine without 60; at 128 two without leave 124 KB.  us a solve,
+// tiles / per lane:
+//   64 columns:   6x96^2x64 785 / 800, 96 levels 1168 / 1180, 99 1199 / 1230,
+//                 100 1587 / 1235, 110 1720 / 1306, 6x192^2x96 4128 / 4055
+//   32 columns:   6x96^2x64 998 / 805, 6x192^2x96 5600 / 4055
+//   128 columns:  6x96^2x64 778 / 799, 6x192^2x96 4128 / 3838
+// With three contexts' steps in turn on the GPU the tiles, which do not need
+// their lines to stay in L1, gain 5 % of a step at 6x96^2x64 (4450 against
+// 4690 us) and 6x192^2x96 (25650 against 26880), at 64 and at 128 columns; 128
+// is no default but an autotuner's choice for steps by themselves.  Tiles of
+// two levels (18 KB a warp): 4416, 4004 and 3995 us a solve at 6x192^2x96 and
+// 32, 64 and 128 columns.
+constexpr bool fused_tiles(int threads, int nc1) {
+  const size_t block = (fused_smem<true>(threads, nc1) + sizeof(DevView) + 127) / 128 * 128 + 1024;
+  return threads == 64 && 4 * block <= 196 * 1024;
 }
 
 // A column of the stepping context: primitives and update from the state
@@ -448,7 +496,7 @@ struct FusedColumnIO {
 };
 
 
-template <class R>
+template <class R, bool kTile>
 __device__ __forceinline__ void implicit_fused_block(const DevView& v, unsigned blk, int stage,
                                                double dt_given = 0.) {
   extern __shared__ double ism[];
@@ -459,7 +507,7 @@ __device__ __forceinline__ void implicit_fused_block(const DevView& v, unsigned 
   const double* x1f;
   const double* x1v;
   const double* dx1f;
-  stage_radial(ism + (blockDim.x >> 5) * FUSED_WARP_DOUBLES, v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
+  stage_radial(ism + (blockDim.x >> 5) * fused_warp_doubles<kTile>(), v.nc1, v.x1f, v.x1v, v.dx1f, x1f, x1v, dx1f);
   const unsigned live = __ballot_sync(0xffffffffu, col < ncol);
   if (col >= ncol) return;
   const int j = v.js + col % v.N;
@@ -472,8 +520,8 @@ __device__ __forceinline__ void implicit_fused_block(const DevView& v, unsigned 
   R* scr0 = reinterpret_cast<R*>(v.scratch) + (size_t)(col >> 5) * v.L * 30 * 32 + (col & 31);
   FusedColumnIO<R> io{v.w + base, v.du + base, (stage < 0 ? v.du : v.u) + base, v.cells, scr0,
                       stage,       v.Rd,        v.gamma,                          live};
-  double* const wt = ism + (threadIdx.x >> 5) * FUSED_WARP_DOUBLES;
-  implicit_column_fused(io, wt + LEVEL_TILE_DOUBLES + (threadIdx.x & 31), 32, wt,
+  double* const wt = ism + (threadIdx.x >> 5) * fused_warp_doubles<kTile>();
+  implicit_column_fused<kTile>(io, wt + fused_input_doubles<kTile>() + (threadIdx.x & 31), 32, wt,
                         geo(v, GCOSC, p, k, j), geo(v, GSINC, p, k, j), geo(v, GDX2A, p, k, j),
                         geo(v, GDX3A, p, k, j), x1f, x1v, dx1f, v.is, v.ie, dt, v.gamma, v.grav,
                         wt);

@@ -3125,12 +3125,13 @@ __global__ void EXO_IMPL_BOUNDS kb_implicit(Batch bt, int stage, double dt_given
 }
 
 #if EXO_MIXED
+template <bool kTile>
 __global__ void __maxnreg__(204) kb_implicit_fused(Batch bt, int stage, double dt_given) {
   __shared__ __align__(16) DevView sv;
   unsigned b = batch_enter(bt, sv);
   if (sv.eqn == EXO_EQN_SHALLOW_YZ || !(sv.implicit_flag & 1)) return;
   if (!(sv.implicit_flag & 8)) return;
-  implicit_fused_block<double>(sv, b, stage, dt_given);
+  implicit_fused_block<double, kTile>(sv, b, stage, dt_given);
 }
 #endif
 
@@ -3201,7 +3202,12 @@ inline void launch_kb_implicit(unsigned blocks, int threads, int nc1, cudaStream
   if (kinds & IMPL_FULL) {
 #if EXO_MIXED
     if constexpr (sizeof(R) == 8) {
-      kb_implicit_fused<<<blocks, threads, fused_smem(threads, nc1), st>>>(b, stage, dt_given);
+      if (fused_tiles(threads, nc1))
+        kb_implicit_fused<true>
+            <<<blocks, threads, fused_smem<true>(threads, nc1), st>>>(b, stage, dt_given);
+      else
+        kb_implicit_fused<false>
+            <<<blocks, threads, fused_smem<false>(threads, nc1), st>>>(b, stage, dt_given);
     } else
 #endif
     {
@@ -3286,7 +3292,8 @@ int prepare_kernels() {
       e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   };
 #if EXO_MIXED
-  allow((const void*)kb_implicit_fused, IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit_fused<true>, IMPL_SMEM_MAX);
+  allow((const void*)kb_implicit_fused<false>, IMPL_SMEM_MAX);
 #else
   allow((const void*)kb_implicit<double, true>, IMPL_SMEM_MAX);
   allow((const void*)kb_implicit_bwd<double, true>, (int)BwdLayout<double, 5>::bytes);

@@ -129,11 +129,47 @@ static int check_timeout(int precision, int implicit_flag) {
   return 0;
 }
 
+// The mixed 5x5 solve's shared memory leaves its loads an L1: not more than 61
+// doubles a column beside the radial tables, or four blocks of 64 columns
+// within the 196 KB that leave 60 KB of L1.
+static int check_fused_smem() {
+  for (int L : {1, 32, 96, 99, 100, 250}) {
+    exo_config cfg;
+    exo_config_default(&cfg, EXO_EQN_IDEAL);
+    cfg.N = 8;
+    cfg.L = L;
+    cfg.precision = EXO_PREC_MIXED;
+    cfg.implicit_flag = 9;
+    exo_ctx* c = nullptr;
+    if (exo_create(&cfg, &c)) return fail("exo_create");
+    const int nc1 = L + 6;
+    std::vector<double> du((size_t)6 * 5 * 14 * 14 * nc1, 1.), w(du);
+    for (int tile : {32, 64, 128}) {
+      const int tiles[6] = {0, 0, 0, tile, 0, 0};
+      if (exo_set_tiles(c, tiles)) return fail("exo_set_tiles");
+      host_launches_clear();
+      if (exo_solve_implicit_3d(c, du.data(), w.data(), 60.)) return fail("a solve");
+      const std::vector<HostLaunch> all = host_launches();
+      if (all.size() != 1 || !is(all[0], "kb_implicit_fused") || all[0].block != (unsigned)tile)
+        return fail("one launch at the tile");
+      const size_t small = (size_t)(61 * tile + 3 * (nc1 + 1)) * sizeof(double);
+      const size_t block = (all[0].smem + sizeof(exo::DevView) + 127) / 128 * 128 + 1024;
+      if (all[0].smem > small && !(tile == 64 && 4 * block <= 196 * 1024)) {
+        std::printf("%d levels, tile %d: %zu bytes\n", L, tile, all[0].smem);
+        return fail("shared memory that leaves an L1");
+      }
+    }
+    exo_destroy(c);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   int rc = 2;
   if (!std::strcmp(what, "pairs")) rc = check_pairs(FULL) + check_pairs(PARTIAL) + check_pairs(NOALLOC);
   if (!std::strcmp(what, "levels")) rc = check_levels();
+  if (!std::strcmp(what, "fused_smem")) rc = check_fused_smem();
   if (!std::strcmp(what, "timeout"))
     rc = check_timeout(EXO_PREC_FP64, 9) + check_timeout(EXO_PREC_FP64, 1) +
          check_timeout(EXO_PREC_MIXED, 1) + check_timeout(EXO_PREC_MIXED_F32_SOLVE, 9);

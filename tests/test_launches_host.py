@@ -43,3 +43,7 @@ def test_a_wait_that_gave_up_is_the_implicit_call_s_error(driver):
 
 def test_column_hooks_take_the_deepest_columns(driver):
     _check(driver, "levels")
+
+
+def test_the_mixed_solve_leaves_its_l1(driver):
+    _check(driver, "fused_smem")
