@@ -2,12 +2,13 @@
 // back substitution in the same kernel (textually part of exo_kernels.cuh).
 //
 // The same algorithm as implicit_column and kb_implicit_bwd in one kernel.  The
-// split form measured 764 us a solve at 6x96^2x64 (with the blocks kept by
-// their structure 617), this one 780; but compiled with fused multiply-adds
-// the split form does not round as this one does: the last bits of u it
-// changes reach the FP32 copy of the primitives, and a run differs by 1e-7
-// within some tens of steps.  (The boundary terms as branches change the
-// roundings too.)  FP32 blocks, the 3x3 blocks and the FP64 build, whose
+// split form is faster (6x24^2x32 109 us a solve against 123, 6x96^2x64 761
+// against 785, 6x192^2x96 4017 against 4166, with 128 columns a block 4025
+// against 3861; with the blocks kept by their structure 617 at 6x96^2x64);
+// but compiled with fused multiply-adds it does not round as this one does:
+// the last bits of u it changes reach the FP32 copy of the primitives, and a
+// run differs by 1e-7 within some tens of steps.  (The boundary terms as
+// branches change the roundings too.)  FP32 blocks, the 3x3 blocks and the FP64 build, whose
 // results the split form leaves to the bit, take the split form.
 //
 // What bounds it: dependent FP64 operations at eight to nine warps per SM, on

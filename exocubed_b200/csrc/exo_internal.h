@@ -279,11 +279,10 @@ struct Tiles {
 Tiles default_tiles();
 bool valid_tiles(const int* t, std::string* err);
 // The x1 kernel takes tiles[BK_X1] radial columns per block (1..X1_MAX_COLUMNS).
-// Shared memory per column: the primitives and the face pressures, and in
-// the mixed build ln psf and the face densities.
+// Shared memory per column: x1_column_doubles.
 constexpr int X1_MAX_COLUMNS = 8;
 // the x1 kernel's dynamic shared memory limit (the mixed build's 8 columns
-// of 250 levels take 212 KB)
+// of 250 levels take 199 KB)
 constexpr int X1_SMEM_MAX = 224 * 1024;
 // the precisions stepped by the mixed build (exo::mixed)
 EXO_HD inline bool mixed_build(int precision) {

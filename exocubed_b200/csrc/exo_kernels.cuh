@@ -748,15 +748,15 @@ __device__ __forceinline__ void prim_ghost_block(const DevView& v, unsigned blk,
 // cells and hydrostatic scan are spread over the block's threads, so the
 // block's lanes stay busy (one column of L+1 faces leaves most of a warp
 // idle) and the columns' scans run side by side.
-// What bounds it: instruction issue (mixed build, 96^2x64: 1,724 instructions
-// per 32 cells at 0.66 a cycle and scheduler; DRAM 13 %), a third of them FP32
-// WENO5, then the FP64 decomposition and the Riemann solve.  It was 2,074 with
+// What bounds it: instruction issue (mixed build, 96^2x64: 1,692 instructions
+// per 32 cells at 0.65 a cycle and scheduler; DRAM 13 %), a third of them FP32
+// WENO5, then the FP64 decomposition and the Riemann solve.  It was 2,076 with
 // a division for its place per pass and element, a thread's cells converted to
 // FP32 five times, the reciprocal of gamma and the solver's functions of it
-// per cell, and the series' coefficients as literals.  Per launch, before and
-// now: FP64 40^2x40 76 -> 69 us, 96^2x64 484 -> 420; mixed 24^2x32 19 -> 17,
-// 62^2x45 120 -> 111, 96^2x64 312 -> 261, 126^2x70 666 -> 548, 192^2x96 1705
-// -> 1460.
+// per cell, and the series' coefficients as literals.  Per launch (4 columns a
+// block), before and now: FP64 40^2x40 84 -> 70 us, 96^2x64 536 -> 422; mixed
+// 24^2x32 19 -> 17, 62^2x45 121 -> 109, 96^2x64 312 -> 258, 126^2x70 667 ->
+// 542, 192^2x96 1712 -> 1448.
 __device__ __forceinline__ int x1_columns_per_block(const DevView& v) {
   return v.tiles[BK_X1] > 0 ? v.tiles[BK_X1] : 1;
 }
@@ -1184,12 +1184,12 @@ __device__ __forceinline__ void cp_async_wait_one() {
 // (one thread per cell, both of its face values from one set of smoothness
 // indicators, through shared memory) and solves per face after a barrier.
 // What bounds it: instruction issue (mixed build, IPC 0.66 a scheduler) and
-// the FP64 pipe (FP64 build, 62 % busy), not memory (16 % and 11 % of DRAM).
+// the FP64 pipe (FP64 build, 67 % busy), not memory (17 % and 14 % of DRAM).
 // Per launch, before (32 radial indices of one line per block, or one thread
-// per face where those left lanes idle; FP64 also through shared memory) and
-// now: FP64 48^2x3 33.1 -> 23.1 us, 40^2x40 145 -> 105, 96^2x64 695 -> 575;
-// mixed 24^2x32 26 -> 19, 62^2x45 143 -> 96, 126^2x70 595 -> 447, 192^2x96
-// 1115 -> 1104.
+// per face where those left lanes idle, places recomputed, divisions with
+// range checks) and now: FP64 48^2x3 39 -> 23 us, 40^2x40 179 -> 103, 96^2x64
+// 1029 -> 573; mixed 24^2x32 30 -> 19, 62^2x45 176 -> 97, 126^2x70 833 -> 454,
+// 192^2x96 1626 -> 1120.
 #ifndef EXO_X23_THREADS
 #define EXO_X23_THREADS 128
 #endif
@@ -1198,7 +1198,9 @@ constexpr int X23_THREADS = EXO_X23_THREADS;
 // two faces: a rule on the levels alone, since the two ways round
 // differently and a run's results have to depend on nothing but its
 // configuration.  (The line is where a block of 32 levels of one line used to
-// give way to one thread per face, which did not share them.)
+// give way to one thread per face, which did not share them.  Sharing at all
+// levels would be faster: 20 levels of 126^2 157 -> 135 us, 33 of 96^2 168 ->
+// 151, 41 of 62^2 96 -> 84.)
 __host__ __device__ constexpr bool x23_shares_beta(int L) {
   return EXO_MIXED && L * 100 >= 65 * 32 * ((L + 31) / 32);
 }
@@ -1206,7 +1208,8 @@ template <class T, bool kShareBeta>
 __host__ __device__ constexpr int x23_chunk() {
   return kShareBeta ? 15 : sizeof(T) == 4 ? 16 : 8;
 }
-// resident blocks per SM (128 registers a thread)
+// resident blocks per SM: at 128 registers a thread, which the mixed build is
+// held to (EXO_X23_MINB) and the FP64 build takes of itself
 constexpr unsigned X23_RESIDENT = 4;
 
 // cp.async of 4 or 8 bytes, zero-filled when src_bytes is 0
@@ -2624,7 +2627,8 @@ __device__ __forceinline__ double* impl_radial(double* ism) {
   return ism + (blockDim.x >> 5) * impl_warp_doubles<R, full>();
 }
 // the largest dynamic shared memory a launch may ask for
-constexpr int IMPL_SMEM_MAX = 160 * 1024;  // 128 threads, 250 levels
+// (a step's 128 columns of 250 levels take 96 KB, the column hooks up to this)
+constexpr int IMPL_SMEM_MAX = 160 * 1024;
 
 // copies the radial geometry of the member into shared memory (all threads
 // of the block take part; returns the shared copies)
@@ -2670,11 +2674,9 @@ struct StepColumnIO {
   __device__ __forceinline__ size_t scr_stride() const { return 32; }
 };
 
-// One radial column of the stepping context: solve, then u += du and, on
-// the last stage, the AirParcel round trip.
-// stage 0..2: a stage of the step (dt = beta_stage * the CFL step, u += du);
-// stage -1: ImplicitSolver::SolveImplicit3D alone (dt given, du corrected in
-// place)
+// The forward sweep of one radial column of the stepping context.
+// stage 0..2: a stage of the step (dt = beta_stage * the CFL step);
+// stage -1: ImplicitSolver::SolveImplicit3D alone (dt given)
 template <class R, bool full>
 __device__ __forceinline__ void implicit_block(const DevView& v, unsigned blk, int stage,
                                                double dt_given = 0.) {
@@ -3084,8 +3086,8 @@ __global__ void EXO_X1_BOUNDS kb_flux_x1(Batch bt) {
 }
 
 // the mixed build at 128 registers (4 blocks of 128 threads per SM): 1.64 ms
-// per launch at 6x192^2x96 against 1.75 at its natural 148 (line form with
-// recomputed addresses)
+// per launch at 6x192^2x96 against 1.75 at its natural 148 (measured with
+// addresses recomputed per row and face)
 #if EXO_MIXED && !defined(EXO_X23_MINB)
 #define EXO_X23_MINB 4
 #endif
@@ -3265,7 +3267,8 @@ int launch_reciprocal(int n, const double* x, double* out, void* stream) {
 // wave of blocks badly: the count of segments whose waves x length is least,
 // a segment's length being its chunks and half a chunk for the first cells'
 // way in.  (FP64, N = 40, 40 levels, 600 blocks of whole lines: one
-// segment 135 us, two 116; N = 48, 3 levels, 60 blocks: seven segments.)
+// segment 135 us, two 116; N = 48, 3 levels, 60 blocks: seven segments.)  A
+// member of a batch keeps the split it has alone; results do not depend on it.
 X23Split x23_split(int N, int L) {
   using T = EXO_FLUX_T;
   const unsigned CF = x23_shares_beta(L) ? x23_chunk<T, true>() : x23_chunk<T, false>();
