@@ -15,8 +15,8 @@ pytestmark = pytest.mark.gpu
 
 
 def _members(precision):
-    """Uneven members: sizes, levels (32 takes the x2/x3 line form, the
-    others the per-face form), solvers, gases and one shallow-water sphere
+    """Uneven members: sizes, levels (mixed x2/x3: 32 shares the
+    smoothness indicators, the others do not), solvers, gases and one shallow-water sphere
     (fp64 only: its own equation set and variable count)."""
     out = []
     for n, (N, L, rs) in enumerate([(8, 12, nat.EXO_RS_LMARS), (12, 8, nat.EXO_RS_HLLC),

@@ -1,6 +1,6 @@
 """The implicit solve at the sizes where its pipeline can go wrong: columns
-shorter than the builders' lead, ring and batch lengths (1 to 9 levels and
-the next ones), groups of one column, of 31, 32 and 33.  FP64 against the
+around the ring's and the level tile's lengths (1 to 9 levels and the next
+ones), groups of one column, of 31, 32 and 33.  FP64 against the
 oracle bit for bit; the mixed builds against the oracle's FP64 solve."""
 import numpy as np
 import pytest

@@ -24,7 +24,7 @@ def pressure(u, gamma):
     return (gamma - 1.0) * (u[:, 4] - ke)
 
 
-@pytest.mark.parametrize("L", [16, 32])   # the per-face and the line form of x2/x3
+@pytest.mark.parametrize("L", [16, 32])   # x2/x3: per face, and with shared indicators
 @pytest.mark.parametrize("precision", [nat.EXO_PREC_MIXED, nat.EXO_PREC_MIXED_F32_SOLVE])
 @pytest.mark.parametrize("rsolver", [1, 2])
 def test_mixed_dry_atmosphere_close_to_oracle(oracle_mod, rsolver, precision, L):

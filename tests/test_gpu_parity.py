@@ -113,7 +113,7 @@ def test_c1_config_100_steps_bitwise(oracle_mod, seed):
     assert np.array_equal(_noncorner(g.primitive()), _noncorner(o.primitive()))
 
 
-@pytest.mark.parametrize("L", [12, 32])   # the per-face and the line form of x2/x3
+@pytest.mark.parametrize("L", [12, 32])   # lines that straddle groups of 32, and that fill them
 @pytest.mark.parametrize("rsolver", [1, 2])
 def test_dry_atmosphere_fluxes(oracle_mod, rsolver, L):
     N = 8
