@@ -14,7 +14,7 @@
 // What bounds it: dependent FP64 operations at eight to nine warps per SM, on
 // large grids the scratch's traffic (480 of 640 bytes a level and column,
 // 2.1 ms at the copy rate at 6x192^2x96), and the L1 beside the blocks' shared
-// memory, which the columns' strided loads live on (fused_tiles).
+// memory, whose lines hold the columns' strided loads in flight (fused_tiles).
 // More warps do not help (200 registers, ten warps: the same; 168: twice the
 // time, the lines of L1 in flight being what limits them).
 
@@ -447,9 +447,9 @@ constexpr size_t fused_smem(int threads, int nc1) {
   return ((size_t)fused_warp_doubles<kTile>() * (threads / 32) + 3 * (size_t)(nc1 + 1)) * sizeof(double);
 }
 // How the inputs come in.  A level tile reads each sector once but takes 23 KB
-// a warp; per lane (15 KB) a sector is read four times, three of them from
-// L1.  An SM's shared memory goes up in steps, and what is left of 256 KB is
-// L1: at the default 64 columns a block, four blocks with tiles leave 60 KB as
+// a warp; per lane (15 KB) a sector is read four times, mostly from L2 (L1 hits
+// 3 %).  An SM's shared memory goes up in steps, and what is left of 256 KB is
+// L1, a line of which every load in flight holds: at the default 64 columns a block, four blocks with tiles leave 60 KB as
 // long as they stay within the step of 196 KB (99 levels), past it 28 KB, too
 // few lines for the copies in flight.  At 32 columns eight blocks with tiles
 // leave 28 KB, nine without 60; at 128 two without leave 124 KB.  us a solve,
@@ -458,15 +458,19 @@ constexpr size_t fused_smem(int threads, int nc1) {
 //                 100 1587 / 1235, 110 1720 / 1306, 6x192^2x96 4128 / 4055
 //   32 columns:   6x96^2x64 998 / 805, 6x192^2x96 5600 / 4055
 //   128 columns:  6x96^2x64 778 / 799, 6x192^2x96 4128 / 3838
-// With three contexts' steps in turn on the GPU the tiles, which do not need
-// their lines to stay in L1, gain 5 % of a step at 6x96^2x64 (4450 against
-// 4690 us) and 6x192^2x96 (25650 against 26880), at 64 and at 128 columns; 128
-// is no default but an autotuner's choice for steps by themselves.  Tiles of
+// With three contexts' steps in turn on the GPU the tiles, which ask less of L1
+// and L2, gain 5 % of a step at 6x96^2x64 (4450 against 4690 us) and 6x192^2x96
+// (25650 against 26880), at 64 and at 128 columns; 128 is no default but an
+// autotuner's choice for steps by themselves.  Grids of few blocks gain nothing
+// from tiles even so (us a step, alone and in turn, tiles / per lane: 24 blocks,
+// 6x16^2x90, 1173 / 1122 and 494 / 473; 54, 6x24^2x32, 496 / 468 and 266 / 264;
+// but 85, 6x30^2x60, 1063 / 1034 and 596 / 628; 384, 6x64^2x33, 1320 / 1301 and
+// 1169 / 1231): the line is a block for every second SM.  Tiles of
 // two levels (18 KB a warp): 4416, 4004 and 3995 us a solve at 6x192^2x96 and
 // 32, 64 and 128 columns.
-constexpr bool fused_tiles(int threads, int nc1) {
+constexpr bool fused_tiles(unsigned blocks, int threads, int nc1) {
   const size_t block = (fused_smem<true>(threads, nc1) + sizeof(DevView) + 127) / 128 * 128 + 1024;
-  return threads == 64 && 4 * block <= 196 * 1024;
+  return threads == 64 && blocks > 148 / 2 && 4 * block <= 196 * 1024;
 }
 
 // A column of the stepping context: primitives and update from the state

@@ -3204,7 +3204,7 @@ inline void launch_kb_implicit(unsigned blocks, int threads, int nc1, cudaStream
   if (kinds & IMPL_FULL) {
 #if EXO_MIXED
     if constexpr (sizeof(R) == 8) {
-      if (fused_tiles(threads, nc1))
+      if (fused_tiles(blocks, threads, nc1))
         kb_implicit_fused<true>
             <<<blocks, threads, fused_smem<true>(threads, nc1), st>>>(b, stage, dt_given);
       else

@@ -129,21 +129,22 @@ static int check_timeout(int precision, int implicit_flag) {
   return 0;
 }
 
-// The mixed 5x5 solve's shared memory leaves its loads an L1: not more than 61
+// The mixed 5x5 solve's shared memory leaves its loads enough of L1: not more than 61
 // doubles a column beside the radial tables, or four blocks of 64 columns
-// within the 196 KB that leave 60 KB of L1.
-static int check_fused_smem() {
+// within the 196 KB that leave 60 KB of L1 (6 x 8^2 columns, and 6 x 32^2,
+// which is more than a block for every second SM).
+static int check_fused_smem(int N) {
   for (int L : {1, 32, 96, 99, 100, 250}) {
     exo_config cfg;
     exo_config_default(&cfg, EXO_EQN_IDEAL);
-    cfg.N = 8;
+    cfg.N = N;
     cfg.L = L;
     cfg.precision = EXO_PREC_MIXED;
     cfg.implicit_flag = 9;
     exo_ctx* c = nullptr;
     if (exo_create(&cfg, &c)) return fail("exo_create");
     const int nc1 = L + 6;
-    std::vector<double> du((size_t)6 * 5 * 14 * 14 * nc1, 1.), w(du);
+    std::vector<double> du((size_t)6 * 5 * (N + 6) * (N + 6) * nc1, 1.), w(du);
     for (int tile : {32, 64, 128}) {
       const int tiles[6] = {0, 0, 0, tile, 0, 0};
       if (exo_set_tiles(c, tiles)) return fail("exo_set_tiles");
@@ -169,7 +170,7 @@ int main(int argc, char** argv) {
   int rc = 2;
   if (!std::strcmp(what, "pairs")) rc = check_pairs(FULL) + check_pairs(PARTIAL) + check_pairs(NOALLOC);
   if (!std::strcmp(what, "levels")) rc = check_levels();
-  if (!std::strcmp(what, "fused_smem")) rc = check_fused_smem();
+  if (!std::strcmp(what, "fused_smem")) rc = check_fused_smem(8) + check_fused_smem(32);
   if (!std::strcmp(what, "timeout"))
     rc = check_timeout(EXO_PREC_FP64, 9) + check_timeout(EXO_PREC_FP64, 1) +
          check_timeout(EXO_PREC_MIXED, 1) + check_timeout(EXO_PREC_MIXED_F32_SOLVE, 9);
